@@ -15,12 +15,14 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <complex>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "asg_generic.cuh"
 #include "asg_internal.h"
+#include "asg_lines.cuh"
 
 // ---------------------------------------------------------------------------
 // error reporting
@@ -140,6 +142,20 @@ static void roots(int n, std::vector<float2>& out) {
   }
 }
 
+// roots minus their FP32 rounding
+static void roots_lo(int n, std::vector<float2>& out) {
+  out.resize(n);
+  for (int k = 0; k < n; ++k) {
+    const double a = -2.0 * M_PI * (double)k / (double)n;
+    out[k] = make_float2((float)(cos(a) - (double)(float)cos(a)),
+                         (float)(sin(a) - (double)(float)sin(a)));
+  }
+}
+static float4 two_floats(double re, double im) {
+  const float x = (float)re, y = (float)im;
+  return make_float4(x, y, (float)(re - (double)x), (float)(im - (double)y));
+}
+
 static constexpr int L2_MAX_CLUSTERS = 64;
 
 // four-step slot order of a fast line of length n (n = n1*n2)
@@ -153,10 +169,94 @@ static void fast_factors(int n, int* n1, int* n2) {
     case 256: *n1 = 16; *n2 = 16; break;
     case 384: *n1 = 16; *n2 = 24; break;
     case 512: *n1 = 16; *n2 = 32; break;
+    case 576: *n1 = 24; *n2 = 24; break;
     case 768: *n1 = 24; *n2 = 32; break;
     case 1024: *n1 = 32; *n2 = 32; break;
+    case 1536: *n1 = 32; *n2 = 48; break;
+    case 2048: *n1 = 32; *n2 = 64; break;
+    case 4096: *n1 = 64; *n2 = 64; break;
     default: *n1 = 0; *n2 = 0; break;
   }
+}
+
+// FP64 DFT of 2^a 3^b values, exp(-2 pi i j k / n) (set-up of the chirp tables).
+static void host_fft(std::vector<std::complex<double>>& v) {
+  const size_t n = v.size();
+  if (n == 1) return;
+  const size_t r = n % 2 == 0 ? 2 : 3, m = n / r;
+  std::vector<std::complex<double>> sub[3];
+  for (size_t j = 0; j < r; ++j) {
+    sub[j].resize(m);
+    for (size_t k = 0; k < m; ++k) sub[j][k] = v[k * r + j];
+    host_fft(sub[j]);
+  }
+  for (size_t k = 0; k < n; ++k) {
+    std::complex<double> s = 0.0;
+    for (size_t j = 0; j < r; ++j)
+      s += sub[j][k % m] * std::polar(1.0, -2.0 * M_PI * (double)((j * k) % n) / (double)n);
+    v[k] = s;
+  }
+}
+
+static void free_axis(LineAxis& a) {
+  cudaFree(const_cast<float4*>(a.ch));
+  cudaFree(const_cast<float4*>(a.bt));
+  cudaFree(const_cast<float4*>(a.tw));
+  a = LineAxis{};
+}
+
+// Transform length and tables of a line of n samples (n <= 2048): direct for the
+// four-step sizes, else the shortest four-step length that holds the chirp
+// convolution without wrap-around.
+static int line_axis(int n, LineAxis* a, cudaStream_t st) {
+  static const int sizes[] = {32, 64, 96, 128, 192, 256, 384, 512, 576, 768, 1024, 1536, 2048, 4096};
+  a->n = n;
+  a->m = 0;
+  a->direct = 0;
+  for (int m : sizes) {
+    if (m == n && m <= 2048) {
+      a->m = m;
+      a->direct = 1;
+      break;
+    }
+    if (a->m == 0 && m >= 2 * n - 1) a->m = m;
+  }
+  if (a->m == 0) return fail(ASG_ERR_SHAPE, "line of %d samples too long", n);
+  const int m = a->m;
+  int n1, n2;
+  fast_factors(m, &n1, &n2);
+  std::vector<float4> tw(m);
+  for (int ka = 0; ka < n1; ++ka)
+    for (int b = 0; b < n2; ++b) {
+      const double ang = -2.0 * M_PI * (double)(ka * b) / (double)m;
+      tw[ka * n2 + b] = two_floats(cos(ang), sin(ang));
+    }
+  float4* d = nullptr;
+  CKS(dalloc(&d, m));
+  a->tw = d;
+  CKS(h2d(d, tw.data(), m, st));
+  if (!a->direct) {
+    std::vector<float4> ch(n), bt(m);
+    std::vector<std::complex<double>> h(m, 0.0);
+    for (int j = 0; j < n; ++j) {
+      const double ang = M_PI * (double)(((long long)j * j) % (2LL * n)) / (double)n;
+      ch[j] = two_floats(cos(ang), -sin(ang));
+      h[j] = std::complex<double>(cos(ang), sin(ang));
+      if (j > 0) h[m - j] = h[j];
+    }
+    host_fft(h);
+    for (int k = 0; k < m; ++k)
+      bt[k] = two_floats(h[k].real() / m, h[k].imag() / m);
+    CKS(dalloc(&d, n));
+    a->ch = d;
+    CKS(h2d(d, ch.data(), n, st));
+    CKS(dalloc(&d, m));
+    a->bt = d;
+    CKS(h2d(d, bt.data(), m, st));
+  }
+  // the host vectors go out of scope here
+  CK(cudaStreamSynchronize(st));
+  return ASG_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -248,7 +348,8 @@ struct asg_plan {
   float2* spec2 = nullptr;  // whole-plane output of the epilogue pass (DSMEM split path)
   float2* nyq_tmp = nullptr;  // one plane: epilogue of the Nyquist plane (L2 path)
   int nyq_plane = -1;         // plane holding bin nT/2, or -1
-  GenPlan gp_t, gp_x, gp_y;
+  GenPlan gp_x, gp_y;
+  LineAxis ax_t = {};         // any-length column transforms (not tfast)
   cudaStream_t st;
   cudaEvent_t ev0, ev1;
   float2* spec = nullptr;
@@ -386,6 +487,7 @@ extern "C" int asg_plan_destroy(asg_plan* p) {
                   p->d_screens, p->d_src, p->d_step, p->d_max_cur, p->d_max_next,
                   p->d_status, p->d_status_step, p->d_iprev, p->d_hist, p->d_clamp};
   for (void* q : ptrs) cudaFree(q);
+  free_axis(p->ax_t);
   free_outputs(p);
   cudaEventDestroy(p->ev0);
   cudaEventDestroy(p->ev1);
@@ -399,12 +501,15 @@ static bool g_roots_done[ASG_MAX_DEVICES] = {};
 static int upload_roots() {
   const int dev = asg_device_slot();
   if (g_roots_done[dev]) return ASG_OK;
-  std::vector<float2> w192, w64;
+  std::vector<float2> w192, w64, lo192, lo64;
   roots(192, w192);
   roots(64, w64);
+  roots_lo(192, lo192);
+  roots_lo(64, lo64);
   if (asg_roots_upload_t(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_xy(w192.data(), w64.data()) != 0 ||
-      asg_roots_upload_l2(w192.data(), w64.data()) != 0)
+      asg_roots_upload_l2(w192.data(), w64.data()) != 0 ||
+      asg_roots_upload_tp(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0)
     return fail(ASG_ERR_CUDA, "upload of the constant root tables failed");
   g_roots_done[dev] = true;
   return ASG_OK;
@@ -439,18 +544,17 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     if (asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM && X > 1024)
       return fail(ASG_ERR_SHAPE, "grid %dx%d: nX > 1024 without a fast plane transform", X, Y);
   }
-  if (!p->tfast && asg_t_generic_smem(T) > 200 * 1024)
-    return fail(ASG_ERR_SHAPE, "nT=%d too long for the generic column transform", T);
-  if (!p->tfast && (T + 31) / 32 > 64)
+  if (!p->tfast && T > ASG_T_MAX)
     return fail(ASG_ERR_SHAPE, "nT=%d too long for the generic column transform", T);
   if (Y > 1024) return fail(ASG_ERR_SHAPE, "nY=%d > 1024", Y);
-  p->gp_t = make_gen_plan(T);
   p->gp_x = make_gen_plan(X);
   p->gp_y = make_gen_plan(Y);
   CK(cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking));
   CK(cudaEventCreate(&p->ev0));
   CK(cudaEventCreate(&p->ev1));
   CKS(upload_roots());
+
+  if (!p->tfast) CKS(line_axis(T, &p->ax_t, p->st));
 
   // ---- planes ----
   p->h_f_of_plane.resize(p->F);
@@ -969,11 +1073,11 @@ static int t_slot(const TParams& t) {
 
 static int run_t(asg_plan* p, const TParams& t, int kind = ASG_K_OTHER) {
   KScope k(p, kind);
-  if (!p->tfast) return asg_launch_t(t, false, p->gp_t, p->st);
+  if (!p->tfast) return asg_launch_t_pairs(t, p->ax_t, p->st);
   TParams tt = t;
   tt.cols_per_block = p->t_cols[t_slot(t)];
   tt.prefetch = p->t_prefetch;
-  return asg_launch_t(tt, true, p->gp_t, p->st);
+  return asg_launch_t_fast(tt, p->st);
 }
 static int run_xy(asg_plan* p, const XYParams& x, int kind = ASG_K_OTHER) {
   KScope k(p, kind);
@@ -2031,19 +2135,16 @@ extern "C" int asg_flux_columns(const float* in, float* out, int ncols, int nT, 
                                 double cfl_target, int max_subcycles) {
   g_err.clear();
   if (!in || !out || ncols <= 0 || nT < 3) return fail(ASG_ERR_ARG, "bad argument");
-  if ((nT + 31) / 32 > 64 || asg_t_generic_smem(nT) > 200 * 1024)
-    return fail(ASG_ERR_SHAPE, "nT=%d too long", nT);
+  if (nT > ASG_T_MAX) return fail(ASG_ERR_SHAPE, "nT=%d too long", nT);
   if (flux < ASG_FLUX_RUSANOV || flux > ASG_FLUX_KT_MINMOD)
     return fail(ASG_ERR_ARG, "unknown flux %d", flux);
   CKS(upload_roots());
   float *d = nullptr, *dout = nullptr;
   unsigned* st = nullptr;
-  float2* tw = nullptr;
   const size_t n = (size_t)ncols * nT;
   CKS(dalloc(&d, n));
   CKS(dalloc(&dout, n));
   CKS(dalloc(&st, 4));  // status word, then the sub-cycle cap counters [2]
-  CKS(dalloc(&tw, nT));
   CK(cudaMemset(st, 0, 4 * sizeof(unsigned)));
   CK(cudaMemcpy(d, in, n * sizeof(float), cudaMemcpyHostToDevice));
   TParams t;
@@ -2054,7 +2155,6 @@ extern "C" int asg_flux_columns(const float* in, float* out, int ncols, int nT, 
   t.real_in = d;
   t.write_real = 1;
   t.real_out = dout;
-  t.tw = tw;
   t.status = st;
   t.op.flux = flux;
   t.op.dz = (float)dz;
@@ -2066,8 +2166,7 @@ extern "C" int asg_flux_columns(const float* in, float* out, int ncols, int nT, 
   t.op.cfl_target = (float)cfl_target;
   t.op.max_subcycles = max_subcycles > 0 ? max_subcycles : 1024;
   t.op.subcycle_clamp = st + 1;
-  GenPlan gp = make_gen_plan(nT);
-  int s = asg_launch_t(t, false, gp, 0);
+  int s = asg_launch_flux_columns(t, 0);
   cudaError_t e = cudaDeviceSynchronize();
   if (s == ASG_OK && e == cudaSuccess)
     e = cudaMemcpy(out, dout, n * sizeof(float), cudaMemcpyDeviceToHost);
@@ -2077,7 +2176,6 @@ extern "C" int asg_flux_columns(const float* in, float* out, int ncols, int nT, 
   cudaFree(d);
   cudaFree(dout);
   cudaFree(st);
-  cudaFree(tw);
   if (s != ASG_OK) return fail(s, "flux kernel launch failed");
   if (e != cudaSuccess) return fail(ASG_ERR_CUDA, "%s", cudaGetErrorString(e));
   return sc;
@@ -2171,8 +2269,7 @@ extern "C" int asg_flux_columns_device(const float* d_in, float* d_out, int ncol
   t.op.cfl_target = (float)cfl_target;
   t.op.max_subcycles = max_subcycles > 0 ? max_subcycles : 1024;
   t.op.subcycle_clamp = scr->clamp;
-  GenPlan gp = make_gen_plan(nT);
-  const int s = asg_launch_t(t, false, gp, st);
+  const int s = asg_launch_flux_columns(t, st);
   if (s != ASG_OK) {
     const cudaError_t e = cudaGetLastError();  // this call's own launch error
     return fail(s, "flux kernel launch failed: %s", cudaGetErrorString(e));

@@ -84,17 +84,6 @@ struct PlainColumn {
   static constexpr bool kVecRun = false;
   ASG_DEV float4* run4(int t0) const { return reinterpret_cast<float4*>(base + t0); }
 };
-// Skewed copy of a column for the chunked KT step (lane l owns samples
-// 32l .. 32l+31): one pad word per 32 samples puts the 32 lanes' i-th samples
-// in 32 different shared-memory banks.  Holds nT + nT/32 floats.
-struct SkewColumn {
-  float* base;
-  ASG_DEV int idx(int t) const { return t + (t >> 5); }
-  ASG_DEV float get(int t) const { return base[idx(t)]; }
-  ASG_DEV void set(int t, float v) const { base[idx(t)] = v; }
-};
-__host__ __device__ constexpr int skew_floats(int nT) { return nT + nT / 32 + 4; }
-
 // ---------------------------------------------------------------------------
 // flux primitives (float32, same formulas and order as the reference)
 // ---------------------------------------------------------------------------
@@ -112,25 +101,6 @@ ASG_DEV float rus_tvd_fh(float uL, float uR) {
 }
 ASG_DEV float tvd_phi(float r, float b) {
   return fmaxf(0.f, fminf(fminf(b * r, 1.f), fminf(r, b)));
-}
-ASG_DEV float minmod2(float a, float b) {
-  return (a * b > 0.f) ? sgnf(a) * fminf(fabsf(a), fabsf(b)) : 0.f;
-}
-ASG_DEV float minmod3(float a, float b, float c) {
-  bool ok = (a * b > 0.f) && (b * c > 0.f);
-  return ok ? sgnf(a) * fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)) : 0.f;
-}
-// limited slope at a cell given its left/right neighbours (MC or minmod).
-// MC: minmod3(2 dm, (dm + dp)/2, 2 dp) = sign(dm) 2 min(|dm|, |dm + dp|/4, |dp|)
-// when dm dp > 0 (then all three arguments share the sign), else 0; the
-// power-of-two scalings are exact, so this is the same number with fewer
-// operations.
-template <bool MC>
-ASG_DEV float kt_slope(float um1, float u0, float up1) {
-  const float dm = u0 - um1, dp = up1 - u0;
-  const float m = MC ? 2.f * fminf(fminf(fabsf(dm), fabsf(dp)), 0.25f * fabsf(dm + dp))
-                     : fminf(fabsf(dm), fabsf(dp));
-  return (dm * dp > 0.f) ? copysignf(m, dm) : 0.f;
 }
 // KT interface flux from the reconstructed states (:772-793), for Burgers'
 // flux f(u) = -u^2/2, whose speeds are a = -u.  With aL = -um, aR = -up the
@@ -151,10 +121,11 @@ ASG_DEV float kt_fh(float um, float up) {
   const float mixed = (um < 0.f) ? fmaf(-0.5f, m2 + p2, -q15) : q15;
   return (q >= 0.f) ? same : mixed;
 }
-// Half the limited slope: every KT reconstruction uses u +/- slope/2.  The
-// MC slope is 2 min(...) and the halving undoes the doubling exactly (power
-// of two scalings are exact), so u + kt_half_slope() equals u + 0.5f * kt_slope()
-// bit for bit, with one multiplication less.
+// Half the limited slope at a cell given its left/right neighbours (MC or
+// minmod): every KT reconstruction uses u +/- slope/2.  The MC slope
+// minmod3(2 dm, (dm + dp)/2, 2 dp) is sign(dm) 2 min(|dm|, |dm + dp|/4, |dp|) when
+// dm dp > 0 (then all three arguments share the sign), else 0, and half of it
+// drops the doubling (power of two scalings are exact).
 template <bool MC>
 ASG_DEV float kt_half_slope(float um1, float u0, float up1) {
   const float dm = u0 - um1, dp = up1 - u0;
@@ -199,183 +170,6 @@ ASG_DEV void rusanov_column(const Col& col, int nT, float coef, bool tvd, float 
     carry = __shfl_sync(mask, u, 31);
     __syncwarp(mask);
     if (t < nT) col.set(t, out);
-  }
-  __syncwarp(mask);
-}
-
-// rhs of the KT scheme (MUSCL slopes, KT interface fluxes) at t = t0+lane,
-// reading src; fh_carry holds the flux at t0-1/2 from the previous block.
-template <bool MC, class Col>
-ASG_DEV float kt_rhs_lane(const Col& src, int t, int nT, float ndt, float& fh_carry,
-                          float& u_out, unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  const float u0 = (t < nT) ? src.get(t) : 0.f;
-  float um1 = __shfl_up_sync(mask, u0, 1);
-  float up1 = __shfl_down_sync(mask, u0, 1);
-  if (lane == 0) um1 = (t >= 1) ? src.get(t - 1) : 0.f;
-  if (lane == 31) up1 = (t + 1 < nT) ? src.get(t + 1) : 0.f;
-  const float sg = (t >= 1 && t < nT - 1) ? kt_slope<MC>(um1, u0, up1) : 0.f;
-  float sn = __shfl_down_sync(mask, sg, 1);
-  if (lane == 31) {
-    const float up2 = (t + 2 < nT) ? src.get(t + 2) : 0.f;
-    sn = (t + 1 >= 1 && t + 1 < nT - 1) ? kt_slope<MC>(u0, up1, up2) : 0.f;
-  }
-  // interface t+1/2
-  const float fh = kt_fh(u0 + 0.5f * sg, up1 - 0.5f * sn);
-  float fp = __shfl_up_sync(mask, fh, 1);
-  if (lane == 0) fp = fh_carry;
-  fh_carry = __shfl_sync(mask, fh, 31);
-  u_out = u0;
-  return (t >= 1 && t < nT - 1) ? (-ndt * (fh - fp)) : 0.f;
-}
-
-// one SSP-RK2 KT step of size dz; stage-1 values go to `stg`
-template <bool MC, class Col>
-ASG_DEV void kt_column_step(const Col& col, const Col& stg, int nT, float ndt, float dz,
-                            unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  float carry = 0.f;
-  for (int t0 = 0; t0 < nT; t0 += 32) {
-    const int t = t0 + lane;
-    float u;
-    const float r = kt_rhs_lane<MC>(col, t, nT, ndt, carry, u, mask);
-    if (t < nT) stg.set(t, u + dz * r);
-  }
-  __syncwarp(mask);
-  carry = 0.f;
-  for (int t0 = 0; t0 < nT; t0 += 32) {
-    const int t = t0 + lane;
-    float s1;
-    const float r = kt_rhs_lane<MC>(stg, t, nT, ndt, carry, s1, mask);
-    if (t < nT) col.set(t, 0.5f * col.get(t) + 0.5f * (s1 + dz * r));
-  }
-  __syncwarp(mask);
-}
-
-// Chunked variant of the KT step: lane l owns samples [l*CH, (l+1)*CH) and keeps
-// its window, stage-1 values and right-hand sides in registers (faster when
-// CH <= 32; the shuffle variant above is used for longer columns).
-// rhs of the KT scheme at the lane's CH points from a window of CH+4 values
-template <int CH, bool MC>
-ASG_DEV void kt_rhs_window(const float (&w)[CH + 4], int t0, int nT, float ndt, float (&rhs)[CH]) {
-  // slopes at window positions 1..CH+2  (t0-1 .. t0+CH); zero at the column ends
-  float s[CH + 2];
-#pragma unroll
-  for (int i = 0; i < CH + 2; ++i) {
-    int t = t0 - 1 + i;
-    s[i] = (t >= 1 && t < nT - 1) ? kt_slope<MC>(w[i], w[i + 1], w[i + 2]) : 0.f;
-  }
-  // interface fluxes at t+1/2 for t = t0-1 .. t0+CH-1
-  float fh[CH + 1];
-#pragma unroll
-  for (int i = 0; i < CH + 1; ++i) {
-    float um = w[i + 1] + 0.5f * s[i];
-    float up = w[i + 2] - 0.5f * s[i + 1];
-    fh[i] = kt_fh(um, up);
-  }
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    int t = t0 + i;
-    rhs[i] = (t >= 1 && t < nT - 1) ? (-ndt * (fh[i + 1] - fh[i])) : 0.f;
-  }
-}
-
-template <int CH, bool MC, class Col>
-ASG_DEV void load_window4(const Col& col, int t0, int nT, float (&w)[CH + 4]) {
-#pragma unroll
-  for (int i = 0; i < CH + 4; ++i) {
-    int t = t0 - 2 + i;
-    w[i] = (t >= 0 && t < nT) ? col.get(t) : 0.f;
-  }
-}
-
-// Column length exactly 32 CH: only the first lane's two leading and the last
-// lane's two trailing window values lie outside the column, and only their
-// slopes and end-sample rhs need zeroing, so the per-point range tests go.
-template <int CH, class Col>
-ASG_DEV void load_window4_exact(const Col& col, int t0, int lane, float (&w)[CH + 4]) {
-  const bool first = lane != 0, last = lane != 31;
-  w[0] = first ? col.get(t0 > 2 ? t0 - 2 : 0) : 0.f;
-  w[1] = first ? col.get(t0 > 1 ? t0 - 1 : 0) : 0.f;
-#pragma unroll
-  for (int i = 2; i < CH + 2; ++i) w[i] = col.get(t0 - 2 + i);
-  w[CH + 2] = last ? col.get(last ? t0 + CH : t0) : 0.f;
-  w[CH + 3] = last ? col.get(last ? t0 + CH + 1 : t0) : 0.f;
-}
-
-// One stage of the exact-length KT step, streamed along the lane's window:
-// slopes, interface fluxes and the update are formed point by point (only
-// the previous slope and flux stay live), and each updated value is written
-// as soon as it is known (every lane has its window in registers by then):
-//   stage 1: col[t] = u[t] + dz rhs(w)
-//   stage 2: col[t] = u[t]/2 + (w[t] + dz rhs(w))/2
-template <int CH, bool MC, bool STAGE2, class Col>
-ASG_DEV void kt_stage_exact(const Col& col, const float (&w)[CH + 4], const float (&u)[CH],
-                            int t0, int lane, float ndt, float dz) {
-  const bool first = lane != 0, last = lane != 31;
-  // slope at window position i+1 (t = t0 - 1 + i); zero at the column ends
-  auto slope = [&](int i) {
-    const float v = kt_slope<MC>(w[i], w[i + 1], w[i + 2]);
-    if (i <= 1) return first ? v : 0.f;
-    if (i >= CH) return last ? v : 0.f;
-    return v;
-  };
-  float sl = slope(0), sr = slope(1);
-  float fprev = kt_fh(w[1] + 0.5f * sl, w[2] - 0.5f * sr);  // interface t0 - 1/2
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    sl = sr;
-    sr = slope(i + 2);
-    const float f = kt_fh(w[i + 2] + 0.5f * sl, w[i + 3] - 0.5f * sr);  // t0 + i + 1/2
-    float rhs = -ndt * (f - fprev);
-    if (i == 0) rhs = first ? rhs : 0.f;
-    if (i == CH - 1) rhs = last ? rhs : 0.f;
-    fprev = f;
-    if (STAGE2) col.set(t0 + i, 0.5f * u[i] + 0.5f * (w[i + 2] + dz * rhs));
-    else col.set(t0 + i, u[i] + dz * rhs);
-  }
-}
-
-// one SSP-RK2 KT step of size dz on the column
-template <int CH, bool MC, class Col>
-ASG_DEV void kt_column_step_chunk(const Col& col, int nT, float ndt, float dz, unsigned mask) {
-  const int lane = threadIdx.x & 31;
-  const int t0 = lane * CH;
-  if (nT == 32 * CH && CH >= 2) {  // uniform across the warp
-    float w[CH + 4], u[CH];
-    load_window4_exact<CH>(col, t0, lane, w);
-#pragma unroll
-    for (int i = 0; i < CH; ++i) u[i] = w[i + 2];
-    __syncwarp(mask);  // every window is read before any lane writes
-    kt_stage_exact<CH, MC, false>(col, w, u, t0, lane, ndt, dz);
-    __syncwarp(mask);
-    load_window4_exact<CH>(col, t0, lane, w);
-    __syncwarp(mask);
-    kt_stage_exact<CH, MC, true>(col, w, u, t0, lane, ndt, dz);
-    __syncwarp(mask);
-    return;
-  }
-  float w[CH + 4];
-  load_window4<CH, MC>(col, t0, nT, w);
-  float u[CH], rhs[CH];
-#pragma unroll
-  for (int i = 0; i < CH; ++i) u[i] = w[i + 2];
-  kt_rhs_window<CH, MC>(w, t0, nT, ndt, rhs);
-  __syncwarp(mask);
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    int t = t0 + i;
-    if (t < nT) col.set(t, u[i] + dz * rhs[i]);  // stage1
-  }
-  __syncwarp(mask);
-  load_window4<CH, MC>(col, t0, nT, w);
-  kt_rhs_window<CH, MC>(w, t0, nT, ndt, rhs);
-  __syncwarp(mask);
-#pragma unroll
-  for (int i = 0; i < CH; ++i) {
-    int t = t0 + i;
-    float s1 = w[i + 2];
-    if (t < nT) col.set(t, 0.5f * u[i] + 0.5f * (s1 + dz * rhs[i]));
   }
   __syncwarp(mask);
 }
@@ -487,6 +281,63 @@ ASG_DEV void kt_step_stream(const Col& col, float ndt, float dz, unsigned mask) 
   __syncwarp(mask);
 }
 
+// The same single streaming pass for any column length nT: lane l owns the samples
+// [l L, (l + 1) L) with L = ceil(nT / 32) made odd (so that the lanes' scalar
+// accesses, L samples apart, spread over the shared-memory banks), the last
+// lanes' runs being short or empty.  Range tests replace the exact version's
+// first/last-lane rules; the four samples on either side of a run are read
+// before any lane writes.
+template <bool MC, class Col>
+ASG_DEV void kt_step_run(const Col& col, int nT, float ndt, float dz, unsigned mask) {
+  const int lane = threadIdx.x & 31;
+  const int L = ((nT + 31) / 32) | 1;
+  const int t0 = lane * L, t1 = min(t0 + L, nT), last = nT - 1;
+  const float c = -ndt * dz;
+  auto u = [&](int t) { return (t >= 0 && t < nT) ? col.get(t) : 0.f; };
+  // half slope at t, zero at the column ends and outside
+  auto sl = [&](float a, float b, float d, int t) {
+    const float v = kt_half_slope<MC>(a, b, d);
+    return (t >= 1 && t < last) ? v : 0.f;
+  };
+  const float hm4 = u(t0 - 4), hm3 = u(t0 - 3), hm2 = u(t0 - 2), hm1 = u(t0 - 1);
+  const float hp0 = u(t1), hp1 = u(t1 + 1), hp2 = u(t1 + 2), hp3 = u(t1 + 3);
+  float w0 = u(t0), w1 = u(t0 + 1), w2 = u(t0 + 2), w3 = u(t0 + 3);  // u[t .. t+3]
+  __syncwarp(mask);
+  if (t0 < nT) {
+    const float sm3 = sl(hm4, hm3, hm2, t0 - 3), sm2 = sl(hm3, hm2, hm1, t0 - 2);
+    const float sm1 = sl(hm2, hm1, w0, t0 - 1), s0 = sl(hm1, w0, w1, t0);
+    const float sA = sl(w0, w1, w2, t0 + 1);
+    float sB = sl(w1, w2, w3, t0 + 2);
+    const float fm25 = kt_fh(hm3 + sm3, hm2 - sm2);
+    const float fm15 = kt_fh(hm2 + sm2, hm1 - sm1);
+    const float fm05 = kt_fh(hm1 + sm1, w0 - s0);
+    const float fp05 = kt_fh(w0 + s0, w1 - sA);
+    float F = kt_fh(w1 + sA, w2 - sB);                               // flux at t+3/2
+    const float r_m2 = t0 >= 3 ? hm2 + c * (fm15 - fm25) : hm2;      // s1[t-2]
+    const float r_m1 = t0 >= 2 ? hm1 + c * (fm05 - fm15) : hm1;
+    float r0 = (t0 >= 1 && t0 < last) ? w0 + c * (fp05 - fm05) : w0;  // s1[t]
+    float r1 = t0 + 1 < last ? w1 + c * (F - fp05) : w1;             // s1[t+1]
+    const float qm1 = sl(r_m2, r_m1, r0, t0 - 1);
+    float q0 = sl(r_m1, r0, r1, t0);                                 // slope of s1 at t
+    float G = kt_fh(r_m1 + qm1, r0 - q0);                            // flux of s1 at t-1/2
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) {
+      const int k = t + 4 - t1;
+      const float u4 = k < 0 ? col.get(t + 4) : k == 0 ? hp0 : k == 1 ? hp1 : k == 2 ? hp2 : hp3;
+      const float sC = sl(w2, w3, u4, t + 3);
+      const float F2 = kt_fh(w2 + sB, w3 - sC);                      // flux at t+5/2
+      const float r2 = t + 2 < last ? w2 + c * (F2 - F) : w2;        // s1[t+2]
+      const float q1 = sl(r0, r1, r2, t + 1);
+      const float G1 = kt_fh(r0 + q0, r1 - q1);                      // flux of s1 at t+1/2
+      col.set(t, (t >= 1 && t < last) ? 0.5f * (w0 + (r0 + c * (G1 - G))) : w0);
+      w0 = w1; w1 = w2; w2 = w3; w3 = u4;
+      sB = sC; F = F2;
+      r0 = r1; r1 = r2; q0 = q1; G = G1;
+    }
+  }
+  __syncwarp(mask);
+}
+
 template <class Col>
 ASG_DEV float column_absmax(const Col& col, int nT) {
   const int lane = threadIdx.x & 31;
@@ -495,24 +346,37 @@ ASG_DEV float column_absmax(const Col& col, int nT) {
   return warp_max(m);
 }
 
+// f(t, i) for the lane's samples t = lane + 32 i of a column, unrolled when the
+// number CH = ceil(nT/32) of them is known (CH = 0: any nT)
+template <int CH, class Fn>
+ASG_DEV void for_samples(int lane, int nT, Fn f) {
+  if constexpr (CH > 0) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int t = lane + 32 * i;
+      if (t < nT) f(t, i);
+    }
+  } else {
+    int i = 0;
+#pragma unroll 4
+    for (int t = lane; t < nT; t += 32, ++i) f(t, i);
+  }
+}
+
 // ---------------------------------------------------------------------------
-// The whole column phase.  CH = ceil(nT/32) samples per lane.
+// The whole column phase.  CH = ceil(nT/32) samples per lane, or 0 (any nT).
 // ---------------------------------------------------------------------------
-// STREAM: the column holds exactly nT = 32 CH samples (CH >= 4) and the KT
-// sub-steps stream along it in place (kt_step_stream).
-template <int CH, bool STREAM = false, class Col>
-ASG_DEV float column_phase(const Col& col, const Col& stg, int c, int nT, const ColumnOps& op,
+// KT sub-steps stream along the column in place: kt_step_stream when the column
+// holds exactly nT = 32 CH samples (CH >= 4), kt_step_run for CH = 0.
+template <int CH, class Col>
+ASG_DEV float column_phase(const Col& col, int c, int nT, const ColumnOps& op,
                            bool write_stats) {
   const int lane = threadIdx.x & 31;
   const unsigned mask = 0xffffffffu;
   // 1) taper
   if (op.abl_xy != nullptr) {
     const float axy = op.abl_xy[c];
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      int t = lane + 32 * i;
-      if (t < nT) col.set(t, col.get(t) * (axy * op.abl_t[t]));
-    }
+    for_samples<CH>(lane, nT, [&](int t, int) { col.set(t, col.get(t) * (axy * op.abl_t[t])); });
     __syncwarp(mask);
   }
   // 2) Burgers
@@ -545,16 +409,13 @@ ASG_DEV float column_phase(const Col& col, const Col& stg, int c, int nT, const 
       }
       const float dzs = op.dz / (float)nsub;
       for (int k = 0; k < nsub; ++k) {
-        if constexpr (STREAM) {
+        if constexpr (CH > 0) {
           static_assert(CH >= 4 && CH <= 64, "streamed KT: 128 to 2048 samples");
           if (op.flux == FLUX_KT_MC) kt_step_stream<CH, true>(col, ndt, dzs, mask);
           else kt_step_stream<CH, false>(col, ndt, dzs, mask);
-        } else if constexpr (CH <= 32) {
-          if (op.flux == FLUX_KT_MC) kt_column_step_chunk<CH, true>(col, nT, ndt, dzs, mask);
-          else kt_column_step_chunk<CH, false>(col, nT, ndt, dzs, mask);
         } else {
-          if (op.flux == FLUX_KT_MC) kt_column_step<true>(col, stg, nT, ndt, dzs, mask);
-          else kt_column_step<false>(col, stg, nT, ndt, dzs, mask);
+          if (op.flux == FLUX_KT_MC) kt_step_run<true>(col, nT, ndt, dzs, mask);
+          else kt_step_run<false>(col, nT, ndt, dzs, mask);
         }
       }
     }
@@ -564,11 +425,7 @@ ASG_DEV float column_phase(const Col& col, const Col& stg, int c, int nT, const 
     int row = op.src[e].map[c];
     if (row >= 0) {
       const float* v = op.src[e].val + (size_t)row * nT;
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        int t = lane + 32 * i;
-        if (t < nT) col.set(t, col.get(t) + v[t]);
-      }
+      for_samples<CH>(lane, nT, [&](int t, int) { col.set(t, col.get(t) + v[t]); });
     }
     __syncwarp(mask);
   }
@@ -579,19 +436,15 @@ ASG_DEV float column_phase(const Col& col, const Col& stg, int c, int nT, const 
     float s = 0.f, mn = INFINITY, mx = -INFINITY;
     double sd = 0.0;
     bool bad = false;
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      int t = lane + 32 * i;
-      if (t < nT) {
-        float u = col.get(t);
-        s = fmaf(u, u, s);
-        mn = fminf(mn, u);
-        mx = fmaxf(mx, u);
-        am = fmaxf(am, fabsf(u));
-        bad |= !(fabsf(u) <= 3.402823466e38f);
-        if ((i & 7) == 7) { sd += (double)s; s = 0.f; }
-      }
-    }
+    for_samples<CH>(lane, nT, [&](int t, int i) {
+      float u = col.get(t);
+      s = fmaf(u, u, s);
+      mn = fminf(mn, u);
+      mx = fmaxf(mx, u);
+      am = fmaxf(am, fabsf(u));
+      bad |= !(fabsf(u) <= 3.402823466e38f);
+      if ((i & 7) == 7) { sd += (double)s; s = 0.f; }
+    });
     sd += (double)s;
     sd = warp_sum(sd);
     mn = warp_min(mn);
@@ -612,11 +465,7 @@ ASG_DEV float column_phase(const Col& col, const Col& stg, int c, int nT, const 
     }
     if (c == op.pax_col && !op.init_stats) {
       float* pa = op.pax + (size_t)(*op.step) * (size_t)nT;
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        int t = lane + 32 * i;
-        if (t < nT) pa[t] = col.get(t);
-      }
+      for_samples<CH>(lane, nT, [&](int t, int) { pa[t] = col.get(t); });
     }
   }
   return am;

@@ -1076,7 +1076,7 @@ extern "C" int asg_net_train_step(asg_net* n, const float* d_x, const float* d_t
 // ---------------------------------------------------------------------------
 // Learned KT step on columns.
 //
-// Gate (one warp per column, the column in a skewed shared-memory copy):
+// Gate (one warp per column, the column in shared memory):
 //   s      = max|u|,  steep = max_t |u[t+1] - u[t]|
 //   n_sub  = the per-column sub-cycle count of the plain KT step at cfl_target
 //   learned when n_sub >= min_sub and steep <= shock_ratio * s: one coarse KT
@@ -1109,7 +1109,6 @@ struct GateParams {
   unsigned* clamp;    // [2] fallback columns capped at max_sub, largest count needed
 };
 
-template <int CH>
 __global__ void __launch_bounds__(256) k_flux_gate(GateParams p) {
   extern __shared__ float sk_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1117,7 +1116,7 @@ __global__ void __launch_bounds__(256) k_flux_gate(GateParams p) {
   if (c >= p.ncols) return;
   const int nT = p.nT;
   const unsigned mask = 0xffffffffu;
-  SkewColumn col{sk_raw + warp * skew_floats(32 * CH)};
+  PlainColumn col{sk_raw + warp * nT};
   const float* src = p.in + (size_t)c * nT;
   float s = 0.f, steep = 0.f;
   for (int t = lane; t < nT; t += 32) {
@@ -1152,8 +1151,8 @@ __global__ void __launch_bounds__(256) k_flux_gate(GateParams p) {
   const int steps = learned ? 1 : nsub;
   const float dzs = p.dz / (float)steps;
   for (int k = 0; k < steps; ++k) {
-    if (p.mc) kt_column_step_chunk<CH, true>(col, nT, p.ndt, dzs, mask);
-    else kt_column_step_chunk<CH, false>(col, nT, p.ndt, dzs, mask);
+    if (p.mc) kt_step_run<true>(col, nT, p.ndt, dzs, mask);
+    else kt_step_run<false>(col, nT, p.ndt, dzs, mask);
   }
   float* dst = p.out + (size_t)c * nT;
   for (int t = lane; t < nT; t += 32) dst[t] = col.get(t);
@@ -1183,10 +1182,9 @@ __global__ void k_apply_correction(const float* __restrict__ y, const int* __res
     if (t >= 1 && t < nT - 1) out[(size_t)c * nT + t] += s * yr[t];
 }
 
-template <int CH>
 int launch_gate(const GateParams& p, cudaStream_t st) {
-  const size_t smem = (size_t)8 * skew_floats(32 * CH) * sizeof(float);
-  k_flux_gate<CH><<<(p.ncols + 7) / 8, 256, smem, st>>>(p);
+  const size_t smem = (size_t)8 * p.nT * sizeof(float);  // nT <= 1024
+  k_flux_gate<<<(p.ncols + 7) / 8, 256, smem, st>>>(p);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
 }
 
@@ -1240,10 +1238,7 @@ extern "C" int asg_flux_columns_learned(asg_net* n, const float* d_in, float* d_
   g.list_s = list_s;
   g.counter = counter;
   g.clamp = reinterpret_cast<unsigned*>(counter + 1);
-  const int ch = (nT + 31) / 32;
-  const int s = ch <= 2 ? launch_gate<2>(g, st) : ch <= 4 ? launch_gate<4>(g, st)
-              : ch <= 8 ? launch_gate<8>(g, st) : ch <= 16 ? launch_gate<16>(g, st)
-              : launch_gate<32>(g, st);
+  const int s = launch_gate(g, st);
   if (s != ASG_OK) return net_fail(s, "gate launch");
   int cnt[3] = {0, 0, 0};
   if (cudaMemcpyAsync(cnt, counter, sizeof(cnt), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -9,6 +9,7 @@
 
 struct SourceEvent;
 struct GenPlan;
+struct LineAxis;  // asg_lines.cuh
 
 // ---- t-column pass ---------------------------------------------------------
 #include "asg_column.cuh"
@@ -40,8 +41,11 @@ int asg_t_default_cols(int nT, int Y, int flux);
 bool asg_t_cols_supported(int nT, int Y, int flux, int cols);
 
 bool asg_t_fast_supported(int nT);
-size_t asg_t_generic_smem(int nT);
-int asg_launch_t(const TParams& p, bool fast, const GenPlan& pl, cudaStream_t st);
+int asg_launch_t_fast(const TParams& p, cudaStream_t st);
+// any nT up to ASG_T_MAX (asg_tpairs.cu), and the Burgers step alone on real columns
+constexpr int ASG_T_MAX = 2048;
+int asg_launch_t_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st);
+int asg_launch_flux_columns(const TParams& p, cudaStream_t st);
 
 // ---- xy-plane pass ---------------------------------------------------------
 struct ScreenDev {
@@ -162,6 +166,8 @@ int asg_launch_transpose(const float* in, float* out, int nz, int ncols, cudaStr
 int asg_roots_upload_t(const float2* w192, const float2* w64);
 int asg_roots_upload_xy(const float2* w192, const float2* w64);
 int asg_roots_upload_l2(const float2* w192, const float2* w64);
+int asg_roots_upload_tp(const float2* w192, const float2* w64, const float2* lo192,
+                        const float2* lo64);
 
 // One-time launcher set-up (shared-memory attributes, occupancy queries,
 // constant tables) is per device: what is set with one device current does not

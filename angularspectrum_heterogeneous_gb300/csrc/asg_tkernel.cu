@@ -3,10 +3,10 @@
 // real FFT along t, with the spectrum planes in HBM between passes.
 //
 // Spectrum layout in HBM: spec[plane][x*Y + y] (complex64).  One plane per
-// rfft bin; the fast kernels keep the planes in their permuted slot order
-// (plane = slot holding bin f, Nyquist bin in the last plane), the generic
-// kernels in natural order.  The xy kernels get the bin of each plane from
-// a host-built table.
+// rfft bin; these kernels keep the planes in their permuted slot order (plane =
+// slot holding bin f, Nyquist bin in the last plane), the any-length kernels
+// (asg_tpairs.cu) in natural order.  The xy kernels get the bin of each plane
+// from a host-built table.
 //
 // Reference semantics: rfft/irfft along t of angular_spectrum_solver.py
 // (:215, :272, :662-664, :679, :685), the analytic-signal step of :652-654
@@ -14,7 +14,6 @@
 // drops the imaginary part of the DC and Nyquist bins.
 #include "asg_internal.h"
 #include "asg_column.cuh"
-#include "asg_generic.cuh"
 
 ASG_DEFINE_ROOT_UPLOADER(asg_roots_upload_t)
 
@@ -199,8 +198,7 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
     ColumnOps op = p.op;
     if (MODE != TM_FLUX) op.flux = FLUX_NONE;
     op.abl_xy = nullptr;  // tapered at the end of phase 1
-    const float a =
-        column_phase<CH, MODE == TM_FLUX>(col, col, mycol, nT, op, MODE == TM_STATS);
+    const float a = column_phase<CH>(col, mycol, nT, op, MODE == TM_STATS);
     am = (a != a || am != am) ? __uint_as_float(0x7fc00000u) : fmaxf(am, a);
     if (p.write_real) {
       float2* dst = reinterpret_cast<float2*>(p.real_out + (size_t)mycol * nT);
@@ -309,99 +307,6 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
 }
 
 // ---------------------------------------------------------------------------
-// generic kernel: any nT, complex FFT of length nT on real data
-// ---------------------------------------------------------------------------
-template <int CH>
-__global__ void __launch_bounds__(128) tk_generic(TParams p, GenPlan pl) {
-  if (*p.status != 0) return;
-  constexpr int C = 4;
-  const int nT = p.nT;
-  const int F = nT / 2 + 1;
-  extern __shared__ float4 smraw[];
-  float2* A = reinterpret_cast<float2*>(smraw);
-  float2* B = A + C * nT;
-  float2* tw = B + C * nT;
-  float* stg_base = reinterpret_cast<float*>(tw + nT);  // KT stage-1 values [C][nT]
-  __shared__ float red_max[C];
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int c0 = blockIdx.x * C;
-  const int ncols = p.ncols;
-  for (int i = tid; i < nT; i += nthr) tw[i] = p.tw[i];
-  const int mycol = c0 + warp;
-  const bool active = mycol < ncols;
-
-  float* re;  // real samples, column cc at re + cc*nT
-  if (p.in_real) {
-    re = reinterpret_cast<float*>(B);
-    for (int it = tid; it < C * nT; it += nthr) {
-      const int cc = it / nT, t = it - (it / nT) * nT;
-      const int c = c0 + cc;
-      re[cc * nT + t] = (c < ncols) ? p.real_in[(size_t)c * nT + t] : 0.f;
-    }
-    __syncthreads();
-  } else {
-    for (int it = tid; it < C * F; it += nthr) {
-      const int cc = it % C, f = it / C;
-      const int c = c0 + cc;
-      float2 x = (c < ncols) ? p.spec[(size_t)f * ncols + c] : make_float2(0.f, 0.f);
-      float2* a = A + cc * nT;
-      if (f == 0 || (2 * f == nT)) {
-        a[f] = make_float2(x.x, 0.f);
-      } else {
-        a[f] = x;
-        a[nT - f] = cconj(x);
-      }
-    }
-    __syncthreads();
-    float2* res = gen_fft<true>(A, B, C, nT, 1, pl, tw);
-    float2* other = (res == A) ? B : A;
-    re = reinterpret_cast<float*>(other);
-    const float s = 1.0f / (float)nT;
-    for (int it = tid; it < C * nT; it += nthr) re[it] = res[it].x * s;
-    __syncthreads();
-  }
-
-  float am = 0.f;
-  if (active) {
-    PlainColumn col{re + warp * nT};
-    PlainColumn stg{stg_base + warp * nT};
-    am = column_phase<CH>(col, stg, mycol, nT, p.op, p.stats != 0);
-    if (p.write_real) {
-      for (int t = lane; t < nT; t += 32) p.real_out[(size_t)mycol * nT + t] = col.get(t);
-    }
-  }
-  if (p.stats) {
-    if (lane == 0) red_max[warp] = am;
-    __syncthreads();
-    if (tid == 0) {
-      float m = 0.f;
-      bool bad = false;
-      for (int w = 0; w < C; ++w) {
-        float v = red_max[w];
-        bad |= (v != v);
-        m = fmaxf(m, v);
-      }
-      if (bad) m = __uint_as_float(0x7fc00000u);
-      atomicMax(p.op.max_next, float_as_ordered(m));
-    }
-  }
-  if (!p.do_r2c) return;
-  __syncthreads();
-  // real -> complex in the buffer that does not hold `re`
-  float2* X = (reinterpret_cast<float2*>(re) == A) ? B : A;
-  float2* Y = (X == A) ? B : A;
-  for (int it = tid; it < C * nT; it += nthr) X[it] = make_float2(re[it], 0.f);
-  __syncthreads();
-  float2* res = gen_fft<false>(X, Y, C, nT, 1, pl, tw);
-  for (int it = tid; it < C * F; it += nthr) {
-    const int cc = it % C, f = it / C;
-    const int c = c0 + cc;
-    if (c < ncols) (p.spec_out ? p.spec_out : p.spec)[(size_t)f * ncols + c] = res[cc * nT + f];
-  }
-}
-
-// ---------------------------------------------------------------------------
 // host-side launchers
 // ---------------------------------------------------------------------------
 template <int M, int MODE, int C>
@@ -470,42 +375,17 @@ bool asg_t_fast_supported(int nT) {
   }
 }
 
-// generic: C = 4 columns of nT complex, ping-pong
-size_t asg_t_generic_smem(int nT) {
-  return (size_t)(2 * 4 * nT + nT) * sizeof(float2) + (size_t)4 * nT * sizeof(float);
-}
-
-template <int CH>
-static int launch_generic_t_ch(const TParams& p, const GenPlan& pl, cudaStream_t st) {
-  const size_t smem = asg_t_generic_smem(p.nT);
-  if (cudaFuncSetAttribute(tk_generic<CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return ASG_ERR_CUDA;
-  const int grid = (p.ncols + 3) / 4;
-  tk_generic<CH><<<grid, 128, smem, st>>>(p, pl);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
-}
-
-int asg_launch_t(const TParams& p, bool fast, const GenPlan& pl, cudaStream_t st) {
-  if (fast) {
-    switch (p.nT / 2) {
-      case 64: return launch_fast_t<64>(p, st);
-      case 96: return launch_fast_t<96>(p, st);
-      case 128: return launch_fast_t<128>(p, st);
-      case 192: return launch_fast_t<192>(p, st);
-      case 256: return launch_fast_t<256>(p, st);
-      case 384: return launch_fast_t<384>(p, st);
-      case 512: return launch_fast_t<512>(p, st);
-      case 768: return launch_fast_t<768>(p, st);
-      case 1024: return launch_fast_t<1024>(p, st);
-      default: return ASG_ERR_SHAPE;
-    }
+int asg_launch_t_fast(const TParams& p, cudaStream_t st) {
+  switch (p.nT / 2) {
+    case 64: return launch_fast_t<64>(p, st);
+    case 96: return launch_fast_t<96>(p, st);
+    case 128: return launch_fast_t<128>(p, st);
+    case 192: return launch_fast_t<192>(p, st);
+    case 256: return launch_fast_t<256>(p, st);
+    case 384: return launch_fast_t<384>(p, st);
+    case 512: return launch_fast_t<512>(p, st);
+    case 768: return launch_fast_t<768>(p, st);
+    case 1024: return launch_fast_t<1024>(p, st);
+    default: return ASG_ERR_SHAPE;
   }
-  const int ch = (p.nT + 31) / 32;
-  if (ch <= 4) return launch_generic_t_ch<4>(p, pl, st);
-  if (ch <= 8) return launch_generic_t_ch<8>(p, pl, st);
-  if (ch <= 16) return launch_generic_t_ch<16>(p, pl, st);
-  if (ch <= 32) return launch_generic_t_ch<32>(p, pl, st);
-  if (ch <= 64) return launch_generic_t_ch<64>(p, pl, st);
-  return ASG_ERR_SHAPE;
 }
