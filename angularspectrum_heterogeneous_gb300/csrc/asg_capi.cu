@@ -213,6 +213,8 @@ static int line_axis(int n, LineAxis* a, cudaStream_t st) {
   a->n = n;
   a->m = 0;
   a->direct = 0;
+  a->inv_hi = (float)(1.0 / n);
+  a->inv_lo = (float)(1.0 / n - (double)a->inv_hi);
   for (int m : sizes) {
     if (m == n && m <= 2048) {
       a->m = m;
@@ -350,6 +352,8 @@ struct asg_plan {
   int nyq_plane = -1;         // plane holding bin nT/2, or -1
   GenPlan gp_x, gp_y;
   LineAxis ax_t = {};         // any-length column transforms (not tfast)
+  bool lines = false;         // plane passes as any-length row and column passes
+  LineAxis ax_x = {}, ax_y = {};
   cudaStream_t st;
   cudaEvent_t ev0, ev1;
   float2* spec = nullptr;
@@ -488,6 +492,8 @@ extern "C" int asg_plan_destroy(asg_plan* p) {
                   p->d_status, p->d_status_step, p->d_iprev, p->d_hist, p->d_clamp};
   for (void* q : ptrs) cudaFree(q);
   free_axis(p->ax_t);
+  free_axis(p->ax_x);
+  free_axis(p->ax_y);
   free_outputs(p);
   cudaEventDestroy(p->ev0);
   cudaEventDestroy(p->ev1);
@@ -509,7 +515,8 @@ static int upload_roots() {
   if (asg_roots_upload_t(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_xy(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_l2(w192.data(), w64.data()) != 0 ||
-      asg_roots_upload_tp(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0)
+      asg_roots_upload_tp(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0 ||
+      asg_roots_upload_xylines(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0)
     return fail(ASG_ERR_CUDA, "upload of the constant root tables failed");
   g_roots_done[dev] = true;
   return ASG_OK;
@@ -539,9 +546,10 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   }
   if (!p->xyfast) {
     p->G = 1;
-    // planes larger than one CTA's shared memory take the generic row/column
-    // passes over HBM (their column pass holds whole columns: nX <= 1024)
-    if (asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM && X > 1024)
+    // the row and column passes take lines up to 1024; a plane with more rows
+    // runs in one CTA's shared memory if it fits
+    p->lines = X <= ASG_LINES_MAX;
+    if (!p->lines && asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM)
       return fail(ASG_ERR_SHAPE, "grid %dx%d: nX > 1024 without a fast plane transform", X, Y);
   }
   if (!p->tfast && T > ASG_T_MAX)
@@ -555,6 +563,10 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   CKS(upload_roots());
 
   if (!p->tfast) CKS(line_axis(T, &p->ax_t, p->st));
+  if (p->lines) {
+    CKS(line_axis(X, &p->ax_x, p->st));
+    CKS(line_axis(Y, &p->ax_y, p->st));
+  }
 
   // ---- planes ----
   p->h_f_of_plane.resize(p->F);
@@ -628,11 +640,10 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   // ---- device buffers ----
   const size_t nspec = (size_t)p->F * p->ncols;
   CKS(dalloc(&p->spec, nspec));
-  const bool big = !p->xyfast && asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM;
-  if ((p->split && !p->l2) || big) CKS(dalloc(&p->spec2, nspec));
+  if ((p->split && !p->l2) || (p->lines && cfg->nonlinear_obliquity)) CKS(dalloc(&p->spec2, nspec));
   for (int q = 0; q < p->F; ++q)
     if (2 * p->h_f_of_plane[q] == T) p->nyq_plane = q;
-  if (p->l2 && p->nyq_plane >= 0) CKS(dalloc(&p->nyq_tmp, (size_t)X * Y));
+  if ((p->l2 || p->lines) && p->nyq_plane >= 0) CKS(dalloc(&p->nyq_tmp, (size_t)X * Y));
   if (p->l2) {
     // scratch for up to L2_MAX_CLUSTERS clusters, two half-planes each
     const int Xs = X / 2;
@@ -1082,6 +1093,7 @@ static int run_t(asg_plan* p, const TParams& t, int kind = ASG_K_OTHER) {
 static int run_xy(asg_plan* p, const XYParams& x, int kind = ASG_K_OTHER) {
   KScope k(p, kind);
   if (p->l2 && x.epi == 0 && x.nscreens == 0) return asg_launch_xy_l2(x, p->st);
+  if (p->lines) return asg_launch_xy_lines(x, p->ax_x, p->ax_y, p->st);
   return asg_launch_xy(x, p->xyfast, p->gp_x, p->gp_y, p->st);
 }
 
@@ -1201,6 +1213,27 @@ static int status_to_error(asg_plan* p) {
   return fail(code, "device status %d at step %d", code, sstep);
 }
 
+// the epilogue of the Nyquist plane, which the kernels with a fused epilogue leave out
+static int nyquist_epilogue(asg_plan* p, int epi, int nscr) {
+  if (p->nyq_plane < 0) return ASG_OK;
+  const int pl = p->nyq_plane;
+  const size_t pe = (size_t)p->X * p->Y;
+  XYParams e = xyparams(p, nullptr, false);
+  e.epi = epi;
+  e.nscreens = nscr;
+  e.screens = p->d_screens;
+  e.nplanes = 1;
+  e.f_of_plane = p->f_of_plane + pl;
+  if (e.fw_exp) e.fw_exp += pl;
+  if (e.sa_coef) e.sa_coef += pl;
+  if (e.screen_fscale) e.screen_fscale += pl;
+  KScope k(p, ASG_K_OTHER);
+  CKS(asg_launch_epilogue_pass(e, p->spec + pl * pe, p->nyq_tmp, 0, p->st));
+  CK(cudaMemcpyAsync(p->spec + pl * pe, p->nyq_tmp, pe * sizeof(float2),
+                     cudaMemcpyDeviceToDevice, p->st));
+  return ASG_OK;
+}
+
 // one march step; `last` -> write the real field, no forward transform
 // closing plane pass + (x, y, omega) epilogue, then the column pass that
 // ends the step (or, for asg_apply_operator, just returns to real space)
@@ -1211,7 +1244,9 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
     x.epi = epi;
     x.nscreens = nscr;
     x.screens = p->d_screens;
+    if (p->lines) x.skip_plane = p->nyq_plane;
     CKS(run_xy(p, x, kind));
+    if (p->lines && (epi != 0 || nscr > 0)) CKS(nyquist_epilogue(p, epi, nscr));
     t_after.split_in = 0;
     return ASG_OK;
   }
@@ -1229,23 +1264,7 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
       KScope k(p, kind);
       CKS(asg_launch_xy_l2_closing(x, p->st));
     }
-    if (p->nyq_plane >= 0) {
-      const int pl = p->nyq_plane;
-      const size_t pe = (size_t)p->X * p->Y;
-      XYParams e = xyparams(p, nullptr, false);
-      e.epi = epi;
-      e.nscreens = nscr;
-      e.screens = p->d_screens;
-      e.nplanes = 1;
-      e.f_of_plane = p->f_of_plane + pl;
-      if (e.fw_exp) e.fw_exp += pl;
-      if (e.sa_coef) e.sa_coef += pl;
-      if (e.screen_fscale) e.screen_fscale += pl;
-      KScope k(p, ASG_K_OTHER);
-      CKS(asg_launch_epilogue_pass(e, p->spec + pl * pe, p->nyq_tmp, 0, p->st));
-      CK(cudaMemcpyAsync(p->spec + pl * pe, p->nyq_tmp, pe * sizeof(float2),
-                         cudaMemcpyDeviceToDevice, p->st));
-    }
+    CKS(nyquist_epilogue(p, epi, nscr));
     t_after.split_in = 0;
     return ASG_OK;
   }

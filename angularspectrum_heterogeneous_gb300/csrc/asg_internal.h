@@ -110,8 +110,8 @@ struct XYParams {
                            //    the second set is used by the pipelined flow)
   int pipe;                // 1 (with coop): split-phase barriers over two scratch halves
   unsigned grp_skew;       // added to every barrier target (test hook: 0 in normal runs)
-  float2* spec_tmp;        // [planes][X][Y] work spectrum of the large generic planes
-  int skip_plane;          // closing-stage kernel: plane left without epilogue (-1: none)
+  float2* spec_tmp;        // [planes][X][Y] work spectrum (power sums of the line passes)
+  int skip_plane;          // fused epilogues: plane left without one (-1: none)
   int bulk_rows;           // L2-exchange kernels' HBM row loads: 0 cp.async, 1 bulk copies in
                            // the diffraction kernel, 2 bulk copies in both kernels
   int rows8;               // 1: a cooperative launch of the diffraction kernel uses 8-row CTAs
@@ -129,9 +129,11 @@ bool asg_xy_split_supported(int X, int Y, int* G_out);
 int asg_launch_epilogue_pass(const XYParams& p, const float2* src, float2* dst, int split,
                              cudaStream_t st);
 size_t asg_xy_generic_smem(int X, int Y);
-// planes whose generic transform needs more shared memory than this run as
-// row and column passes over HBM through XYParams::spec_tmp (nX <= 1024)
 constexpr size_t ASG_XY_GENERIC_MAX_SMEM = 200 * 1024;
+// any nX, nY up to ASG_LINES_MAX as row and column passes (asg_xylines.cu)
+constexpr int ASG_LINES_MAX = 1024;
+int asg_launch_xy_lines(const XYParams& p, const LineAxis& axx, const LineAxis& axy,
+                        cudaStream_t st);
 int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPlan& ply,
                   cudaStream_t st);
 
@@ -168,6 +170,8 @@ int asg_roots_upload_xy(const float2* w192, const float2* w64);
 int asg_roots_upload_l2(const float2* w192, const float2* w64);
 int asg_roots_upload_tp(const float2* w192, const float2* w64, const float2* lo192,
                         const float2* lo64);
+int asg_roots_upload_xylines(const float2* w192, const float2* w64, const float2* lo192,
+                             const float2* lo64);
 
 // One-time launcher set-up (shared-memory attributes, occupancy queries,
 // constant tables) is per device: what is set with one device current does not

@@ -31,6 +31,7 @@ struct LineAxis {
   int n;              // line length
   int m;              // transform length: n when direct, else the convolution length
   int direct;
+  float inv_hi, inv_lo;  // 1/n as two floats (one would scale every inverse transform alike)
   // factors as (hi.re, hi.im, lo.re, lo.im)
   const float4* ch;   // [n] w_j (chirp axes)
   const float4* bt;   // [m] spectrum of conj(w), bins in natural order, 1/m folded in
@@ -42,6 +43,10 @@ ASG_DEV float2 mul_f4(float2 a, float4 w) {
 }
 ASG_DEV float2 mulc_f4(float2 a, float4 w) {
   return cmulc_hl(a, make_float2(w.x, w.y), make_float2(w.z, w.w));
+}
+
+ASG_DEV float2 scale_hl(float2 a, float hi, float lo) {
+  return make_float2(fmaf(a.x, hi, a.x * lo), fmaf(a.y, hi, a.y * lo));
 }
 
 // Forward DFT of N values whose upper half is zero (v[N/2..] need not be set).

@@ -106,7 +106,6 @@ __global__ void __launch_bounds__(128, pair_min_blocks<M, DIRECT>())
       }
     }
     __syncthreads();
-    const float inv = 1.0f / (float)n;
     if constexpr (!DIRECT) {
       for (int it = tid; it < P * N2; it += NT) {
         const int q = it & (P - 1), b = it >> lp;
@@ -133,7 +132,7 @@ __global__ void __launch_bounds__(128, pair_min_blocks<M, DIRECT>())
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
           const int t = b + N2 * a;
-          if (t < n) line[PL::pos(t)] = cscale(mulc_f4(v[a], __ldg(ax.ch + t)), inv);
+          if (t < n) line[PL::pos(t)] = scale_hl(mulc_f4(v[a], __ldg(ax.ch + t)), ax.inv_hi, ax.inv_lo);
         }
       }
     } else {
@@ -152,7 +151,7 @@ __global__ void __launch_bounds__(128, pair_min_blocks<M, DIRECT>())
         float2 v[N1];
         chirp_stepA_inv<PL>(line, b, v, ax.tw);
 #pragma unroll
-        for (int a = 0; a < N1; ++a) line[PL::pos(b + N2 * a)] = cscale(v[a], inv);
+        for (int a = 0; a < N1; ++a) line[PL::pos(b + N2 * a)] = scale_hl(v[a], ax.inv_hi, ax.inv_lo);
       }
     }
     __syncthreads();

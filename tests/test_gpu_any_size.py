@@ -23,6 +23,14 @@ def test_columns_of_any_length(nT):
     P.test_step_operators(None, (5, 4, nT))
 
 
+# the same along x and y (lines up to 1024), with an even and an odd nT (with and
+# without a Nyquist plane); the other axis and nT leave partial tiles and blocks
+@pytest.mark.parametrize("n", [n for n in LENGTHS if n <= 769] + [1000, 1023, 1024])
+def test_planes_of_any_size(n):
+    P.test_step_operators(None, (n, 5, 9))
+    P.test_step_operators(None, (6, n, 8))
+
+
 @pytest.mark.parametrize("nT", [4, 5, 31, 33, 64, 127, 129, 640, 1000, 1025, 2048])
 @pytest.mark.parametrize("flux", ["kt", "ktmm"])
 def test_kt_runs_of_any_length(nT, flux):
