@@ -156,6 +156,7 @@ struct TableParams {
   float2* out_pa;          // propagator x attenuation (or null)
   float2* out_p;           // propagator alone (or null)
   float2* out_a;           // attenuation alone (or null)
+  float2* out_sq;          // (propagator x attenuation)^2: both halves of a step (or null)
 };
 int asg_launch_table(const TableParams& p, cudaStream_t st);
 int asg_launch_obl_table(const TableParams& p, float* out, cudaStream_t st);

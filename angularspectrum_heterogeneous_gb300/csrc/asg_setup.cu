@@ -33,7 +33,7 @@ __device__ __forceinline__ void sincos_reduced(double ph, float* s, float* c) {
 
 // All multiplier tables of one step size in one pass: per mode the propagator
 // factor P and the attenuation/KK factor A are formed once and written as
-// out_pa = P A, out_p = P, out_a = A (any output may be null).  The phases,
+// out_pa = P A, out_p = P, out_a = A, out_sq = (P A)^2 (any output may be null).  The phases,
 // the wavenumbers and the exponents' arguments are FP64 (the propagator
 // phase in the cancellation-free form); exp and sin/cos of them are taken in
 // FP32 after an FP64 argument reduction; each entry is rounded to FP32 once
@@ -116,6 +116,10 @@ __global__ void k_build_table(TableParams p) {
       }
     }
     const double nrm = p.norm;
+    if (p.out_sq != nullptr) {
+      const double zr = pr * ar - pi * ai, zi = pr * ai + pi * ar;
+      p.out_sq[i] = make_float2((float)((zr * zr - zi * zi) * nrm), (float)(2.0 * zr * zi * nrm));
+    }
     if (p.out_pa != nullptr)
       p.out_pa[i] = make_float2((float)((pr * ar - pi * ai) * nrm), (float)((pr * ai + pi * ar) * nrm));
     if (p.out_p != nullptr) p.out_p[i] = make_float2((float)(pr * nrm), (float)(pi * nrm));
