@@ -142,15 +142,6 @@ static void roots(int n, std::vector<float2>& out) {
   }
 }
 
-// roots minus their FP32 rounding
-static void roots_lo(int n, std::vector<float2>& out) {
-  out.resize(n);
-  for (int k = 0; k < n; ++k) {
-    const double a = -2.0 * M_PI * (double)k / (double)n;
-    out[k] = make_float2((float)(cos(a) - (double)(float)cos(a)),
-                         (float)(sin(a) - (double)(float)sin(a)));
-  }
-}
 static float4 two_floats(double re, double im) {
   const float x = (float)re, y = (float)im;
   return make_float4(x, y, (float)(re - (double)x), (float)(im - (double)y));
@@ -169,22 +160,21 @@ static void fast_factors(int n, int* n1, int* n2) {
     case 256: *n1 = 16; *n2 = 16; break;
     case 384: *n1 = 16; *n2 = 24; break;
     case 512: *n1 = 16; *n2 = 32; break;
-    case 576: *n1 = 24; *n2 = 24; break;
     case 768: *n1 = 24; *n2 = 32; break;
     case 1024: *n1 = 32; *n2 = 32; break;
-    case 1536: *n1 = 32; *n2 = 48; break;
-    case 2048: *n1 = 32; *n2 = 64; break;
-    case 4096: *n1 = 64; *n2 = 64; break;
     default: *n1 = 0; *n2 = 0; break;
   }
 }
 
-// FP64 DFT of 2^a 3^b values, exp(-2 pi i j k / n) (set-up of the chirp tables).
+// FP64 DFT, exp(-2 pi i j k / n), by the smallest factors of n (set-up of the chirp
+// tables: products of radices up to 64).
 static void host_fft(std::vector<std::complex<double>>& v) {
   const size_t n = v.size();
   if (n == 1) return;
-  const size_t r = n % 2 == 0 ? 2 : 3, m = n / r;
-  std::vector<std::complex<double>> sub[3];
+  size_t r = 2;
+  while (n % r) ++r;
+  const size_t m = n / r;
+  std::vector<std::vector<std::complex<double>>> sub(r);
   for (size_t j = 0; j < r; ++j) {
     sub[j].resize(m);
     for (size_t k = 0; k < m; ++k) sub[j][k] = v[k * r + j];
@@ -205,38 +195,94 @@ static void free_axis(LineAxis& a) {
   a = LineAxis{};
 }
 
-// Transform length and tables of a line of n samples (n <= 2048): direct for the
-// four-step sizes, else the shortest four-step length that holds the chirp
-// convolution without wrap-around.
+// Operations per value of a register DFT of r points, roughly: a direct sum over a
+// prime, a radix-4 split as two stages of 2.
+static int radix_cost(int r) {
+  int c = 0;
+  while (r % 4 == 0) { c += 4; r /= 4; }
+  for (int q = 2; r > 1; ++q)
+    while (r % q == 0) { c += q; r /= q; }
+  return c;
+}
+
+// Factors (n1, n2) of a direct line among the radices of the kernel variants
+// (with_radix), the cheapest pair; false if there is none.
+static bool direct_factors(int n, int* n1, int* n2) {
+  auto ok32 = [](int r) {
+    return (r >= 1 && r <= 18) || r == 20 || r == 21 || r == 24 || r == 25 || r == 27 || r == 28 ||
+           r == 30 || r == 32;
+  };
+  auto ok64 = [](int r) {
+    return r == 27 || r == 28 || r == 30 || r == 32 || r == 36 || r == 40 || r == 48 || r == 64;
+  };
+  int best = 1 << 30;
+  for (int a = 1; a <= 64; ++a) {
+    if (n % a) continue;
+    const int b = n / a;
+    // the larger variants hold fewer warps per SM; an exchange costs about as much as a
+    // radix-4 stage
+    int c = radix_cost(a) + radix_cost(b) + (a > 1 ? 3 : 0) + abs(a - b) / 4;
+    if (n <= 1024 && ok32(a) && ok32(b)) c += a > 16 || b > 16 ? 4 : 0;
+    else if (n > 1024 && ok64(a) && ok64(b)) c += 8;
+    else continue;
+    if (c < best) {
+      best = c;
+      *n1 = a;
+      *n2 = b;
+    }
+  }
+  return best < (1 << 30);
+}
+
+// Factors of the convolution of a chirp line of n samples (n <= 2048): the shortest
+// length >= 2 n - 1 of the compiled ones.
+static bool chirp_factors(int n, int* n1, int* n2) {
+  static const int sizes[][2] = {
+#define F(a, b) {a, b},
+      ASG_CHIRP_SIZES(F) F(64, 64)
+#undef F
+  };
+  int best = 1 << 30;
+  for (const auto& f : sizes) {
+    const int m = f[0] * f[1];
+    if (m < 2 * n - 1 || m >= best) continue;
+    best = m;
+    *n1 = f[0];
+    *n2 = f[1];
+  }
+  return best < (1 << 30);
+}
+
+// Factors and tables of a line of n samples.
 static int line_axis(int n, LineAxis* a, cudaStream_t st) {
-  static const int sizes[] = {32, 64, 96, 128, 192, 256, 384, 512, 576, 768, 1024, 1536, 2048, 4096};
   a->n = n;
-  a->m = 0;
-  a->direct = 0;
   a->inv_hi = (float)(1.0 / n);
   a->inv_lo = (float)(1.0 / n - (double)a->inv_hi);
-  for (int m : sizes) {
-    if (m == n && m <= 2048) {
-      a->m = m;
-      a->direct = 1;
-      break;
-    }
-    if (a->m == 0 && m >= 2 * n - 1) a->m = m;
-  }
-  if (a->m == 0) return fail(ASG_ERR_SHAPE, "line of %d samples too long", n);
-  const int m = a->m;
-  int n1, n2;
-  fast_factors(m, &n1, &n2);
-  std::vector<float4> tw(m);
+  int n1 = 0, n2 = 0;
+  a->direct = direct_factors(n, &n1, &n2) ? 1 : 0;
+  if (!a->direct && !chirp_factors(n, &n1, &n2))
+    return fail(ASG_ERR_SHAPE, "line of %d samples too long", n);
+  const int m = n1 * n2;
+  a->m = m;
+  a->n1 = n1;
+  a->n2 = n2;
+  const int big = n1 > n2 ? n1 : n2;
+  // lengths above 1024 have their own direct radices
+  a->rm = n > 1024 ? 64 : big <= 16 ? 16 : big <= 24 ? 24 : 32;
+  const int tws = a->direct ? a->rm : n2;  // DirectPlan / ChirpPlan strides
+  a->s2 = tws + 2;
+  a->mg1 = ((1u << 20) + n1 - 1) / n1;
+  a->mg2 = ((1u << 20) + n2 - 1) / n2;
+  std::vector<float4> tw((size_t)n1 * tws, make_float4(0.f, 0.f, 0.f, 0.f));
   for (int ka = 0; ka < n1; ++ka)
     for (int b = 0; b < n2; ++b) {
       const double ang = -2.0 * M_PI * (double)(ka * b) / (double)m;
-      tw[ka * n2 + b] = two_floats(cos(ang), sin(ang));
+      tw[ka * tws + b] = two_floats(cos(ang), sin(ang));
     }
   float4* d = nullptr;
-  CKS(dalloc(&d, m));
+  CKS(dalloc(&d, tw.size()));
   a->tw = d;
-  CKS(h2d(d, tw.data(), m, st));
+  CKS(h2d(d, tw.data(), tw.size(), st));
   if (!a->direct) {
     std::vector<float4> ch(n), bt(m);
     std::vector<std::complex<double>> h(m, 0.0);
@@ -511,16 +557,18 @@ static bool g_roots_done[ASG_MAX_DEVICES] = {};
 static int upload_roots() {
   const int dev = asg_device_slot();
   if (g_roots_done[dev]) return ASG_OK;
-  std::vector<float2> w192, w64, lo192, lo64;
+  std::vector<float2> w192, w64;
   roots(192, w192);
   roots(64, w64);
-  roots_lo(192, lo192);
-  roots_lo(64, lo64);
+  std::vector<float4> lr(LINE_ROOTS);
+  for (int n = 1; n <= 64; ++n)
+    for (int j = 0; j < n; ++j)
+      lr[n * (n - 1) / 2 + j] = two_floats(cos(2.0 * M_PI * j / n), -sin(2.0 * M_PI * j / n));
   if (asg_roots_upload_t(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_xy(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_l2(w192.data(), w64.data()) != 0 ||
-      asg_roots_upload_tp(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0 ||
-      asg_roots_upload_xylines(w192.data(), w64.data(), lo192.data(), lo64.data()) != 0)
+      asg_roots_upload_tp(lr.data()) != 0 ||
+      asg_roots_upload_xyrows(lr.data()) != 0 || asg_roots_upload_xycols(lr.data()) != 0)
     return fail(ASG_ERR_CUDA, "upload of the constant root tables failed");
   g_roots_done[dev] = true;
   return ASG_OK;

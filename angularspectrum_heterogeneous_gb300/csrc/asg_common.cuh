@@ -57,20 +57,6 @@ ASG_DEV float2 mul_mi(float2 a) {
 // the per-unit uploader that ASG_DEFINE_ROOT_UPLOADER defines.
 static __constant__ float2 c_w192[192];
 static __constant__ float2 c_w64[64];
-// what FP32 rounding took off the entries (the any-length transforms add it back)
-static __constant__ float2 c_w192lo[192];
-static __constant__ float2 c_w64lo[64];
-
-#define ASG_DEFINE_ROOT_UPLOADER_HL(name)                                           \
-  int name(const float2* w192, const float2* w64, const float2* lo192,              \
-           const float2* lo64) {                                                    \
-    if (cudaMemcpyToSymbol(c_w192, w192, sizeof(float2) * 192) != cudaSuccess ||   \
-        cudaMemcpyToSymbol(c_w64, w64, sizeof(float2) * 64) != cudaSuccess ||      \
-        cudaMemcpyToSymbol(c_w192lo, lo192, sizeof(float2) * 192) != cudaSuccess || \
-        cudaMemcpyToSymbol(c_w64lo, lo64, sizeof(float2) * 64) != cudaSuccess)     \
-      return -1;                                                                    \
-    return 0;                                                                       \
-  }
 
 #define ASG_DEFINE_ROOT_UPLOADER(name)                                              \
   int name(const float2* w192, const float2* w64) {                                 \
@@ -95,33 +81,13 @@ ASG_DEV float2 twiddle_const(int j) {
   return INV ? cconj(w) : w;
 }
 
-// a * (hi + lo), and a * conj(hi + lo): a factor known to FP64 as the sum of two
-// floats, the product rounded to FP32
-ASG_DEV float2 cmul_hl(float2 a, float2 hi, float2 lo) {
-  const float tx = fmaf(a.x, lo.x, -a.y * lo.y), ty = fmaf(a.x, lo.y, a.y * lo.x);
-  return make_float2(fmaf(a.x, hi.x, fmaf(-a.y, hi.y, tx)), fmaf(a.x, hi.y, fmaf(a.y, hi.x, ty)));
-}
-ASG_DEV float2 cmulc_hl(float2 a, float2 hi, float2 lo) {
-  return cmul_hl(a, make_float2(hi.x, -hi.y), make_float2(lo.x, -lo.y));
-}
-
 template <int N, bool INV>
-ASG_DEV float2 twiddle_const_lo(int j) {
-  float2 w;
-  if constexpr (192 % N == 0) w = c_w192lo[((j % N) * (192 / N)) % 192];
-  else w = c_w64lo[((j % N) * (64 / N)) % 64];
-  return INV ? cconj(w) : w;
-}
-
-// HL: with the low parts of the constants
-template <int N, bool INV, bool HL = false>
 ASG_DEV float2 twiddle_mul(float2 v, int j) {
   const int e = ((j % N) + N) % N;
   if (e == 0) return v;
   if (4 * e == N) return mul_mi<INV>(v);            // W^(N/4) = -i
   if (2 * e == N) return make_float2(-v.x, -v.y);   // W^(N/2) = -1
   if (4 * e == 3 * N) return mul_mi<!INV>(v);       // W^(3N/4) = +i
-  if constexpr (HL) return cmul_hl(v, twiddle_const<N, INV>(e), twiddle_const_lo<N, INV>(e));
   return cmul(v, twiddle_const<N, INV>(e));
 }
 
@@ -137,7 +103,7 @@ struct DftSplit {
   static constexpr int Q = N / P;
 };
 
-template <int N, bool INV, bool HL = false>
+template <int N, bool INV>
 ASG_DEV void dft(float2 (&v)[N]) {
   if constexpr (N == 1) {
     return;
@@ -155,11 +121,6 @@ ASG_DEV void dft(float2 (&v)[N]) {
     float2 m = make_float2(a.x - 0.5f * t.x, a.y - 0.5f * t.y);
     // (b - c) * i * s3
     float2 r = make_float2(-s3 * d.y, s3 * d.x);
-    if constexpr (HL) {
-      constexpr float s3lo = (float)(0.86602540378443864676 - (double)0.86602540378443864676f);
-      const float l = INV ? s3lo : -s3lo;
-      r = make_float2(fmaf(-s3, d.y, -l * d.y), fmaf(s3, d.x, l * d.x));
-    }
     v[1] = cadd(m, r);
     v[2] = csub(m, r);
   } else if constexpr (N == 4) {
@@ -182,9 +143,9 @@ ASG_DEV void dft(float2 (&v)[N]) {
       float2 t[P];
 #pragma unroll
       for (int p = 0; p < P; ++p) t[p] = v[Q * p + q];
-      dft<P, INV, HL>(t);
+      dft<P, INV>(t);
 #pragma unroll
-      for (int ka = 0; ka < P; ++ka) v[Q * ka + q] = twiddle_mul<N, INV, HL>(t[ka], q * ka);
+      for (int ka = 0; ka < P; ++ka) v[Q * ka + q] = twiddle_mul<N, INV>(t[ka], q * ka);
     }
     float2 o[N];
 #pragma unroll
@@ -192,7 +153,7 @@ ASG_DEV void dft(float2 (&v)[N]) {
       float2 t[Q];
 #pragma unroll
       for (int q = 0; q < Q; ++q) t[q] = v[Q * ka + q];
-      dft<Q, INV, HL>(t);
+      dft<Q, INV>(t);
 #pragma unroll
       for (int kb = 0; kb < Q; ++kb) o[ka + P * kb] = t[kb];
     }
@@ -237,11 +198,6 @@ template <> struct FastPlan<384> : LinePlan<16, 24> {};
 template <> struct FastPlan<512> : LinePlan<16, 32> {};
 template <> struct FastPlan<768> : LinePlan<24, 32> {};
 template <> struct FastPlan<1024> : LinePlan<32, 32> {};
-// lengths of the any-size line transforms only (asg_lines.cuh)
-template <> struct FastPlan<576> : LinePlan<24, 24> {};
-template <> struct FastPlan<1536> : LinePlan<32, 48> {};
-template <> struct FastPlan<2048> : LinePlan<32, 64> {};
-template <> struct FastPlan<4096> : LinePlan<64, 64> {};
 
 // step A on one subline (column b) of a line starting at `line` (padded
 // layout); tw = W_N^j table (N entries, smem or global)

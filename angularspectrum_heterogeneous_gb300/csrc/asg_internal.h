@@ -130,10 +130,13 @@ int asg_launch_epilogue_pass(const XYParams& p, const float2* src, float2* dst, 
                              cudaStream_t st);
 size_t asg_xy_generic_smem(int X, int Y);
 constexpr size_t ASG_XY_GENERIC_MAX_SMEM = 200 * 1024;
-// any nX, nY up to ASG_LINES_MAX as row and column passes (asg_xylines.cu)
+// any nX, nY up to ASG_LINES_MAX as row and column passes (asg_xyrows.cu, asg_xycols.cu)
 constexpr int ASG_LINES_MAX = 1024;
 int asg_launch_xy_lines(const XYParams& p, const LineAxis& axx, const LineAxis& axy,
                         cudaStream_t st);
+int asg_launch_xy_rows(const XYParams& p, const LineAxis& ax, float2* dst, bool inverse,
+                       cudaStream_t st);
+int asg_launch_xy_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaStream_t st);
 int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPlan& ply,
                   cudaStream_t st);
 
@@ -169,10 +172,9 @@ int asg_launch_transpose(const float* in, float* out, int nz, int ncols, cudaStr
 int asg_roots_upload_t(const float2* w192, const float2* w64);
 int asg_roots_upload_xy(const float2* w192, const float2* w64);
 int asg_roots_upload_l2(const float2* w192, const float2* w64);
-int asg_roots_upload_tp(const float2* w192, const float2* w64, const float2* lo192,
-                        const float2* lo64);
-int asg_roots_upload_xylines(const float2* w192, const float2* w64, const float2* lo192,
-                             const float2* lo64);
+int asg_roots_upload_tp(const float4* line_roots);
+int asg_roots_upload_xyrows(const float4* line_roots);
+int asg_roots_upload_xycols(const float4* line_roots);
 
 // One-time launcher set-up (shared-memory attributes, occupancy queries,
 // constant tables) is per device: what is set with one device current does not

@@ -1,57 +1,177 @@
-// Line transforms of any length in shared memory.
+// Line transforms of any length in shared memory, n = n1 n2: step A takes a DFT of
+// n1 points in registers, step B one of n2.
 //
-// A length that the four-step plans cover (FastPlan: 2^a and 3 2^a sizes) is
-// transformed directly.  Every other length n, prime ones included, runs as a
-// chirp convolution (Bluestein): with w_j = exp(-i pi j^2 / n),
+// A length whose two factors are among the radices below (primes up to 17
+// included, as direct sums over the half-sized symmetric and antisymmetric parts)
+// is transformed directly (200 x 180 x 400 as 10 x 20, 12 x 15 and 20 x 20: 0.98 ms per
+// step against 2.2 ms as chirp convolutions).  Every other length runs as a chirp convolution
+// (Bluestein): with w_j = exp(-i pi j^2 / n),
 //   X[k] = w_k sum_j (x[j] w_j) conj(w_{k-j}),
-// a circular convolution of length M >= 2 n - 1 with M a four-step size.  The
-// convolution's forward transform, the product with the transformed chirp and
-// the inverse transform take two exchanges through shared memory:
-//   step A     DFT_N1 of the chirped inputs, twiddles            -> shared
-//   step B     DFT_N2, times the chirp's spectrum, inverse DFT_N2 -> shared
-//   step A^-1  twiddles, inverse DFT_N1, times w_k
-// n <= M/2, so the upper half of step A's inputs is zero and the upper half of
-// step A^-1's outputs is not needed; both DFT_N1 skip that half.
+// a circular convolution of length m >= 2 n - 1, m a product of two radices.
+// The convolution's forward transform, the product with the transformed chirp
+// and the inverse transform take two exchanges through shared memory:
+//   step A     DFT_n1 of the chirped inputs, twiddles            -> shared
+//   step B     DFT_n2, times the chirp's spectrum, inverse DFT_n2 -> shared
+//   step A^-1  twiddles, inverse DFT_n1, times w_k
+// n <= m/2, so the upper half of step A's inputs is zero and the upper half of
+// step A^-1's outputs is not needed; both DFT_n1 skip that half.
 // The inverse transform uses the conjugates of both tables (the chirp is even,
 // so the spectrum of its conjugate is the conjugate of its spectrum).
 //
-// Every factor (chirp, its spectrum, twiddles, the constants of the register DFTs) is
-// kept as two floats: rounded to one, the same relative errors of 3e-8 return at
-// every step of a march and add up, which the direct sums of this length never
-// did.  20 forward/inverse pairs of 101 samples: error 2.4e-6 with single
-// factors, 7.5e-7 with double ones, 1.6e-6 for the direct sum.
+// Every factor (chirp, its spectrum, twiddles, the constants of the register DFTs) is kept as two floats: rounded to one, the same relative errors
+// of 3e-8 return at every step of a march and add up.  20 forward/inverse pairs
+// of 101 samples: error 2.4e-6 with single factors, 7.5e-7 with double ones,
+// 1.6e-6 for the direct sum.
 //
-// Against the direct sum over a prime length this is O(log n) instead of O(n)
-// per sample: a column pass over 257 x 257 x 601 takes 0.89 ms instead of 27 ms.
+// Against Stockham lines with direct sums over a prime length this is O(log n)
+// instead of O(n) per sample: a column pass over 257 x 257 x 601 takes 0.9 ms
+// instead of 27 ms.
 #pragma once
 #include "asg_common.cuh"
 
+// Block of a kernel variant whose largest radix is BIG: threads at most, blocks per SM (so
+// 128, 168 or 255 registers, what the register DFTs need without spills).  Small
+// blocks: their load, exchange and barrier phases overlap each other's (224-thread
+// blocks, two per SM: 257 x 257 x 601 rows 20 % slower).
+template <int BIG>
+struct LineBlock {
+  static constexpr int NT = 128;
+  static constexpr int MB = BIG <= 24 ? 4 : BIG <= 48 ? 3 : 2;
+};
 // Device tables of one axis (built in FP64 on the host, see line_axis()).
 struct LineAxis {
   int n;              // line length
-  int m;              // transform length: n when direct, else the convolution length
+  int m;              // transform length n1 n2: n when direct, else the convolution length
   int direct;
+  int n1, n2;
+  int s2;             // shared-memory stride of a subline (plan constant, PL::S2)
+  int rm;             // direct variant: the larger of n1, n2 rounded up to 16, 24, 32 or 64
+  unsigned mg1, mg2;  // ceil(2^20 / n1), ceil(2^20 / n2): exact quotients below 16384
   float inv_hi, inv_lo;  // 1/n as two floats (one would scale every inverse transform alike)
   // factors as (hi.re, hi.im, lo.re, lo.im)
   const float4* ch;   // [n] w_j (chirp axes)
   const float4* bt;   // [m] spectrum of conj(w), bins in natural order, 1/m folded in
-  const float4* tw;   // [m] W_m^(b ka) at index ka N2 + b: lanes along b read it coalesced
+  const float4* tw;   // W_m^(b ka) at index ka PL::TWS + b: lanes along b read it coalesced
 };
+__host__ __device__ inline int div_magic(int i, unsigned mg) { return (int)(((unsigned)i * mg) >> 20); }
 
+// a * (hi + lo), and a * conj(hi + lo): a factor known to FP64 as the sum of two
+// floats, the product rounded to FP32
+ASG_DEV float2 cmul_hl(float2 a, float2 hi, float2 lo) {
+  const float tx = fmaf(a.x, lo.x, -a.y * lo.y), ty = fmaf(a.x, lo.y, a.y * lo.x);
+  return make_float2(fmaf(a.x, hi.x, fmaf(-a.y, hi.y, tx)), fmaf(a.x, hi.y, fmaf(a.y, hi.x, ty)));
+}
 ASG_DEV float2 mul_f4(float2 a, float4 w) {
   return cmul_hl(a, make_float2(w.x, w.y), make_float2(w.z, w.w));
 }
 ASG_DEV float2 mulc_f4(float2 a, float4 w) {
-  return cmulc_hl(a, make_float2(w.x, w.y), make_float2(w.z, w.w));
+  return cmul_hl(a, make_float2(w.x, -w.y), make_float2(w.z, -w.w));
 }
-
 ASG_DEV float2 scale_hl(float2 a, float hi, float lo) {
   return make_float2(fmaf(a.x, hi, a.x * lo), fmaf(a.y, hi, a.y * lo));
 }
 
-// Forward DFT of N values whose upper half is zero (v[N/2..] need not be set).
+// exp(-2 pi i j / N) for N <= 64 at index N (N - 1) / 2 + j, as two floats
+constexpr int LINE_ROOTS = 64 * 65 / 2;
+static __constant__ float4 c_roots[LINE_ROOTS];
+#define ASG_DEFINE_LINE_ROOT_UPLOADER(name)                                                   \
+  int name(const float4* r) {                                                                  \
+    return cudaMemcpyToSymbol(c_roots, r, sizeof(float4) * LINE_ROOTS) == cudaSuccess ? 0 : -1; \
+  }
+
+// v * W_N^j (forward) or W_N^-j
+template <int N, bool INV>
+ASG_DEV float2 root_mul(float2 v, int j) {
+  const int e = j % N;
+  if (e == 0) return v;
+  if (4 * e == N) return mul_mi<INV>(v);
+  if (2 * e == N) return make_float2(-v.x, -v.y);
+  if (4 * e == 3 * N) return mul_mi<!INV>(v);
+  const float4 w = c_roots[N * (N - 1) / 2 + e];
+  return INV ? mulc_f4(v, w) : mul_f4(v, w);
+}
+
+constexpr int radix_split(int n) {  // first factor of the register DFT's recursion
+  return n % 4 == 0 && n > 4 ? (n % 8 == 0 && n >= 64 ? 8 : 4)
+         : n % 2 == 0 ? 2 : n % 3 == 0 ? 3 : n % 5 == 0 ? 5 : n % 7 == 0 ? 7 : n;
+}
+
+// DFT of N values in registers, natural order in and out, unnormalised
+template <int N, bool INV>
+ASG_DEV void ldft(float2 (&v)[N]) {
+  if constexpr (N == 1) {
+    return;
+  } else if constexpr (N == 2) {
+    const float2 a = v[0], b = v[1];
+    v[0] = cadd(a, b);
+    v[1] = csub(a, b);
+  } else if constexpr (N == 4) {
+    const float2 a = v[0], b = v[1], c = v[2], d = v[3];
+    const float2 s0 = cadd(a, c), d0 = csub(a, c);
+    const float2 s1 = cadd(b, d), d1 = mul_mi<INV>(csub(b, d));
+    v[0] = cadd(s0, s1);
+    v[2] = csub(s0, s1);
+    v[1] = cadd(d0, d1);
+    v[3] = csub(d0, d1);
+  } else if constexpr (radix_split(N) == N) {
+    // odd prime: X[m], X[N-m] = (v0 + sum_k t_k cos) -/+ i sum_k d_k sin over the sums
+    // and differences t_k, d_k of v[k], v[N-k]
+    constexpr int H = (N - 1) / 2;
+    const float2 v0 = v[0];
+    float2 t[H], d[H], x0 = v0;
+#pragma unroll
+    for (int k = 1; k <= H; ++k) {
+      t[k - 1] = cadd(v[k], v[N - k]);
+      d[k - 1] = csub(v[k], v[N - k]);
+      x0 = cadd(x0, t[k - 1]);
+    }
+    v[0] = x0;
+#pragma unroll
+    for (int m = 1; m <= H; ++m) {
+      float2 r = v0, s = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 1; k <= H; ++k) {
+        const float4 w = c_roots[N * (N - 1) / 2 + (k * m) % N];  // cos, -sin
+        r = make_float2(fmaf(t[k - 1].x, w.z, r.x), fmaf(t[k - 1].y, w.z, r.y));
+        s = make_float2(fmaf(d[k - 1].x, w.w, s.x), fmaf(d[k - 1].y, w.w, s.y));
+        r = make_float2(fmaf(t[k - 1].x, w.x, r.x), fmaf(t[k - 1].y, w.x, r.y));
+        s = make_float2(fmaf(d[k - 1].x, w.y, s.x), fmaf(d[k - 1].y, w.y, s.y));
+      }
+      // forward: X[m] = r + i s (s carries -sin), X[N-m] = r - i s
+      const float2 is = make_float2(-s.y, s.x);
+      v[m] = INV ? csub(r, is) : cadd(r, is);
+      v[N - m] = INV ? cadd(r, is) : csub(r, is);
+    }
+  } else {
+    constexpr int P = radix_split(N), Q = N / P;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      float2 t[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) t[p] = v[Q * p + q];
+      ldft<P, INV>(t);
+#pragma unroll
+      for (int ka = 0; ka < P; ++ka) v[Q * ka + q] = root_mul<N, INV>(t[ka], q * ka);
+    }
+    float2 o[N];
+#pragma unroll
+    for (int ka = 0; ka < P; ++ka) {
+      float2 t[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) t[q] = v[Q * ka + q];
+      ldft<Q, INV>(t);
+#pragma unroll
+      for (int kb = 0; kb < Q; ++kb) o[ka + P * kb] = t[kb];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = o[i];
+  }
+}
+
+// Forward DFT of N values (a multiple of 4) whose upper half is zero (v[N/2..] need
+// not be set).
 template <int N>
-ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
+ASG_DEV void ldft_lo(float2 (&v)[N]) {
   if constexpr (N == 4) {
     const float2 a = v[0], b = v[1], c = mul_mi<false>(b);
     v[0] = cadd(a, b);
@@ -59,7 +179,7 @@ ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
     v[2] = csub(a, b);
     v[3] = csub(a, c);
   } else {
-    constexpr int P = DftSplit<N>::P, Q = DftSplit<N>::Q;
+    constexpr int P = radix_split(N), Q = N / P;
     static_assert(P == 4 || P == 8, "half-empty DFT");
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -76,10 +196,10 @@ ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           e[p] = v[Q * p + q];
-          o[p] = twiddle_mul<8, false, true>(e[p], p);
+          o[p] = root_mul<8, false>(e[p], p);
         }
-        dft<4, false, true>(e);
-        dft<4, false, true>(o);
+        ldft<4, false>(e);
+        ldft<4, false>(o);
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           t[2 * p] = e[p];
@@ -87,7 +207,7 @@ ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
         }
       }
 #pragma unroll
-      for (int ka = 0; ka < P; ++ka) v[Q * ka + q] = twiddle_mul<N, false, true>(t[ka], q * ka);
+      for (int ka = 0; ka < P; ++ka) v[Q * ka + q] = root_mul<N, false>(t[ka], q * ka);
     }
     float2 o[N];
 #pragma unroll
@@ -95,7 +215,7 @@ ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
       float2 t[Q];
 #pragma unroll
       for (int q = 0; q < Q; ++q) t[q] = v[Q * ka + q];
-      dft<Q, false, true>(t);
+      ldft<Q, false>(t);
 #pragma unroll
       for (int kb = 0; kb < Q; ++kb) o[ka + P * kb] = t[kb];
     }
@@ -104,91 +224,180 @@ ASG_DEV void dft_fwd_lo(float2 (&v)[N]) {
   }
 }
 
-// --- chirp convolution -------------------------------------------------------
-// step A of subline b: v[a] = input b + N2 a for a < N1/2 (chirped, zero past n)
-template <class PL>
-ASG_DEV void chirp_stepA(float2* line, int b, float2 (&v)[PL::N1], const float4* __restrict__ tw) {
-  dft_fwd_lo<PL::N1>(v);
-  line[PL::pos(b)] = v[0];
-#pragma unroll
-  for (int ka = 1; ka < PL::N1; ++ka)
-    line[PL::pos(b + PL::N2 * ka)] = mul_f4(v[ka], __ldg(tw + ka * PL::N2 + b));
-}
-
-template <class PL, bool INV>
-ASG_DEV void chirp_stepB(float2* line, int ka, const float4* __restrict__ bt) {
-  float2 v[PL::N2];
-  float4* p = reinterpret_cast<float4*>(line + ka * (PL::N2 + 2));
-#pragma unroll
-  for (int b = 0; b < PL::N2 / 2; ++b) {
-    const float4 q = p[b];
-    v[2 * b] = make_float2(q.x, q.y);
-    v[2 * b + 1] = make_float2(q.z, q.w);
-  }
-  dft<PL::N2, false, true>(v);
-#pragma unroll
-  for (int kb = 0; kb < PL::N2; ++kb) {
-    const float4 w = __ldg(bt + ka + PL::N1 * kb);
-    v[kb] = INV ? mulc_f4(v[kb], w) : mul_f4(v[kb], w);
-  }
-  dft<PL::N2, true, true>(v);
-#pragma unroll
-  for (int b = 0; b < PL::N2 / 2; ++b)
-    p[b] = make_float4(v[2 * b].x, v[2 * b].y, v[2 * b + 1].x, v[2 * b + 1].y);
-}
-
-// step A^-1 of subline b: v[a], a < N1/2, are the outputs b + N2 a before the
-// final chirp (the upper half is not formed: nothing reads it)
-template <class PL>
-ASG_DEV void chirp_stepA_inv(const float2* line, int b, float2 (&v)[PL::N1],
-                             const float4* __restrict__ tw) {
-  v[0] = line[PL::pos(b)];
-#pragma unroll
-  for (int ka = 1; ka < PL::N1; ++ka)
-    v[ka] = mulc_f4(line[PL::pos(b + PL::N2 * ka)], __ldg(tw + ka * PL::N2 + b));
-  dft<PL::N1, true, true>(v);
-}
-
-// --- direct four-step transforms with the axis' twiddle layout -----------------
-// forward: step A from registers (v[a] = input b + N2 a), then step B leaves
-// bin ka + N1 kb in v[kb] of task ka; inverse: step B^-1 from registers (bin
-// ka + N1 kb in v[kb]), then step A^-1 leaves output b + N2 a in v[a].
-template <class PL>
-ASG_DEV void direct_stepA(float2* line, int b, float2 (&v)[PL::N1], const float4* __restrict__ tw) {
-  dft<PL::N1, false, true>(v);
-  line[PL::pos(b)] = v[0];
-#pragma unroll
-  for (int ka = 1; ka < PL::N1; ++ka)
-    line[PL::pos(b + PL::N2 * ka)] = mul_f4(v[ka], __ldg(tw + ka * PL::N2 + b));
-}
-template <class PL>
-ASG_DEV void run_load(const float2* line, int ka, float2 (&v)[PL::N2]) {
-  const float4* p = reinterpret_cast<const float4*>(line + ka * (PL::N2 + 2));
-#pragma unroll
-  for (int b = 0; b < PL::N2 / 2; ++b) {
-    const float4 q = p[b];
-    v[2 * b] = make_float2(q.x, q.y);
-    v[2 * b + 1] = make_float2(q.z, q.w);
-  }
-}
-template <class PL>
-ASG_DEV void run_store(float2* line, int ka, const float2 (&v)[PL::N2]) {
-  float4* p = reinterpret_cast<float4*>(line + ka * (PL::N2 + 2));
-#pragma unroll
-  for (int b = 0; b < PL::N2 / 2; ++b)
-    p[b] = make_float4(v[2 * b].x, v[2 * b].y, v[2 * b + 1].x, v[2 * b + 1].y);
-}
-
-// Padded line stride (complex) for lanes running over CL lines first: lines
-// start 16 / CL complex apart modulo the 16 of one 128-byte wavefront, so 16
-// lanes over CL lines and 16 / CL neighbouring slots meet no bank twice.  Even
-// (float4 runs): CL <= 8.
-template <class PL, int CL>
-struct LineStride {
-  static constexpr int R = CL >= 16 ? 2 : 16 / CL;
-  static constexpr int value = PL::PADDED + ((R - PL::PADDED % 16) % 16 + 16) % 16;
+// ---------------------------------------------------------------------------
+// Plans.  Sublines are S2 complex apart in shared memory, even with S2 / 2 odd: a
+// step's strided 8-byte accesses and the 16-byte accesses of a run meet no bank
+// twice, and with S2 and the twiddle stride TWS known to the compiler every
+// access of a step is an immediate offset from one address (run-time strides
+// cost an integer multiply each: the chirp passes of 257 x 257 x 601 took 1.3-1.5 times as long).
+//
+// ChirpPlan: the convolution length's factors, compile-time.
+// DirectPlan: any n1, n2 among the radices of a variant, the code of a radix picked
+// by a switch that is uniform over the block: f(Radix<R>).
+// The host's plan picks from the same lists (line_axis()).
+// ---------------------------------------------------------------------------
+template <int R>
+struct Radix {
+  static constexpr int v = R;
 };
-inline int line_stride(int padded, int cl) {
-  const int r = cl >= 8 ? 2 : 16 / cl;
-  return padded + ((r - padded % 16) % 16 + 16) % 16;
+
+template <int N1, int N2>
+struct ChirpPlan {
+  static constexpr bool DIRECT = false;
+  static constexpr int BIG = N1 > N2 ? N1 : N2, S2 = N2 + 2, TWS = N2;
+  static_assert(N1 % 4 == 0 && N2 % 4 == 0 && (S2 / 2) % 2 == 1, "chirp radices");
+  ASG_DEV static constexpr int n1(const LineAxis&) { return N1; }
+  ASG_DEV static constexpr int n2(const LineAxis&) { return N2; }
+  ASG_DEV static int div1(const LineAxis&, int i) { return i / N1; }
+  ASG_DEV static int div2(const LineAxis&, int i) { return i / N2; }
+  template <class F>
+  ASG_DEV static void with_n1(const LineAxis&, F f) { f(Radix<N1>{}); }
+  template <class F>
+  ASG_DEV static void with_n2(const LineAxis&, F f) { f(Radix<N2>{}); }
+};
+
+#define ASG_RADIX(R) \
+  case R: f(Radix<R>{}); break;
+template <int RM>
+struct DirectPlan {
+  static constexpr bool DIRECT = true;
+  static constexpr int BIG = RM, S2 = RM + 2, TWS = RM;
+  ASG_DEV static int n1(const LineAxis& ax) { return ax.n1; }
+  ASG_DEV static int n2(const LineAxis& ax) { return ax.n2; }
+  ASG_DEV static int div1(const LineAxis& ax, int i) { return div_magic(i, ax.mg1); }
+  ASG_DEV static int div2(const LineAxis& ax, int i) { return div_magic(i, ax.mg2); }
+  // radices: all up to 18, the 7-smooth ones up to 32; for lengths above 1024 some
+  // up to 64
+  template <class F>
+  ASG_DEV static void with_radix(int r, F f) {
+    if constexpr (RM == 16) {
+      switch (r) {
+        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
+        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
+        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) default: break;
+      }
+    } else if constexpr (RM == 24) {
+      switch (r) {
+        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
+        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
+        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) ASG_RADIX(17) ASG_RADIX(18)
+        ASG_RADIX(20) ASG_RADIX(21) ASG_RADIX(24) default: break;
+      }
+    } else if constexpr (RM == 32) {
+      switch (r) {
+        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
+        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
+        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) ASG_RADIX(17) ASG_RADIX(18)
+        ASG_RADIX(20) ASG_RADIX(21) ASG_RADIX(24) ASG_RADIX(25) ASG_RADIX(27) ASG_RADIX(28)
+        ASG_RADIX(30) ASG_RADIX(32) default: break;
+      }
+    } else {
+      switch (r) {
+        ASG_RADIX(27) ASG_RADIX(28) ASG_RADIX(30) ASG_RADIX(32) ASG_RADIX(36) ASG_RADIX(40)
+        ASG_RADIX(48) ASG_RADIX(64) default: break;
+      }
+    }
+  }
+  template <class F>
+  ASG_DEV static void with_n1(const LineAxis& ax, F f) { with_radix(ax.n1, f); }
+  template <class F>
+  ASG_DEV static void with_n2(const LineAxis& ax, F f) { with_radix(ax.n2, f); }
+};
+
+// position of natural index j in a line
+template <class PL>
+ASG_DEV int line_pos(const LineAxis& ax, int j) {
+  return j + PL::div2(ax, j) * (PL::S2 - PL::n2(ax));
 }
+
+// --- the steps on one subline -------------------------------------------------
+// step A: v[a] = input b + n2 a (a < n1/2 in the chirp form) -> twiddled bins
+template <class PL, int N1>
+ASG_DEV void line_stepA(float2* line, int b, float2 (&v)[N1], const LineAxis& ax) {
+  if constexpr (PL::DIRECT) ldft<N1, false>(v);
+  else ldft_lo<N1>(v);
+  line[b] = v[0];
+  const float4* tw = ax.tw + b;
+#pragma unroll
+  for (int ka = 1; ka < N1; ++ka)
+    line[b + PL::S2 * ka] = mul_f4(v[ka], __ldg(tw + ka * PL::TWS));
+}
+// step A^-1: v[a] = output b + n2 a (of the chirp form the lower half is used)
+template <class PL, int N1>
+ASG_DEV void line_stepA_inv(const float2* line, int b, float2 (&v)[N1], const LineAxis& ax) {
+  v[0] = line[b];
+  const float4* tw = ax.tw + b;
+#pragma unroll
+  for (int ka = 1; ka < N1; ++ka)
+    v[ka] = mulc_f4(line[b + PL::S2 * ka], __ldg(tw + ka * PL::TWS));
+  ldft<N1, true>(v);
+}
+// a run of N2 values of one subline (16-byte accesses)
+template <int N2>
+ASG_DEV void run_load(const float2* run, float2 (&v)[N2]) {
+#pragma unroll
+  for (int b = 0; b + 1 < N2; b += 2) {
+    const float4 q = *reinterpret_cast<const float4*>(run + b);
+    v[b] = make_float2(q.x, q.y);
+    v[b + 1] = make_float2(q.z, q.w);
+  }
+  if constexpr (N2 % 2 == 1) v[N2 - 1] = run[N2 - 1];
+}
+template <int N2>
+ASG_DEV void run_store(float2* run, const float2 (&v)[N2]) {
+#pragma unroll
+  for (int b = 0; b + 1 < N2; b += 2)
+    *reinterpret_cast<float4*>(run + b) = make_float4(v[b].x, v[b].y, v[b + 1].x, v[b + 1].y);
+  if constexpr (N2 % 2 == 1) run[N2 - 1] = v[N2 - 1];
+}
+// step B of the chirp form: DFT_n2, the chirp's spectrum (conj: of the inverse
+// transform), inverse DFT_n2, in place
+template <class PL, int N2>
+ASG_DEV void chirp_stepB(float2* run, int ka, const LineAxis& ax, bool conj) {
+  float2 v[N2];
+  run_load<N2>(run, v);
+  ldft<N2, false>(v);
+  const float4* bt = ax.bt + ka;
+  const float sg = conj ? -1.f : 1.f;
+#pragma unroll
+  for (int kb = 0; kb < N2; ++kb) {
+    float4 w = __ldg(bt + PL::n1(ax) * kb);
+    w.y *= sg;
+    w.w *= sg;
+    v[kb] = mul_f4(v[kb], w);
+  }
+  ldft<N2, true>(v);
+  run_store<N2>(run, v);
+}
+// chirp factor at `ch`, conjugated for the inverse transform
+ASG_DEV float2 chirp_mul(float2 v, const float4* ch, bool conj) {
+  float4 w = __ldg(ch);
+  if (conj) {
+    w.y = -w.y;
+    w.w = -w.w;
+  }
+  return mul_f4(v, w);
+}
+
+// Line stride (complex) of a block whose lanes run over cl lines first (a power of two):
+// lines start 16 / cl complex apart modulo the 16 of one 128-byte wavefront, so
+// 16 lanes over cl lines and 16 / cl neighbouring slots meet no bank twice.
+inline int line_stride(const LineAxis& ax, int cl) {
+  const int len = ax.n1 * ax.s2, r = cl >= 8 ? 2 : 16 / cl;  // even: runs are 16-byte aligned
+  return len + ((r - len % 16) % 16 + 16) % 16;
+}
+// threads of a block with `tasks` tasks per step: as few rounds as the variant's
+// largest block allows, no larger than they need
+inline int line_threads(int tasks, int nt_max) {
+  const int rounds = (tasks + nt_max - 1) / nt_max;
+  const int t = ((tasks + rounds - 1) / rounds + 31) / 32 * 32;
+  return t < 32 ? 32 : t;
+}
+// tasks per line of the step with the larger radix (the other step has more, smaller ones):
+// a block takes as many lines as these need to fill it
+inline int line_tasks(const LineAxis& ax) { return ax.n1 < ax.n2 ? ax.n1 : ax.n2; }
+
+// Factors of the chirp convolutions: each length at most 1.33 times the one before.  F(n1, n2)
+#define ASG_CHIRP_SIZES(F)                                                               \
+  F(4, 8) F(4, 12) F(8, 8) F(8, 12) F(8, 16) F(8, 20) F(12, 16) F(16, 16) F(16, 20)     \
+  F(16, 24) F(16, 32) F(24, 24) F(20, 32) F(24, 32) F(32, 32) F(32, 40) F(32, 48) F(32, 64)

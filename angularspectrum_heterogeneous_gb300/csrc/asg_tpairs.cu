@@ -3,15 +3,15 @@
 // accumulators) and the forward real FFT along t.  Two neighbouring columns
 // c, c+1 travel as one complex line u_c + i u_{c+1}: their spectra separate by
 // symmetry, so a pair costs one complex transform of length nT each way
-// (asg_lines.cuh: direct for the four-step sizes, a chirp convolution for every
-// other length).  Planes are in natural bin order.
+// (asg_lines.cuh: direct where the length splits into two radices, a chirp
+// convolution for every other length).  Planes are in natural bin order.
 //
 // A block of 4 warps holds P pairs (a power of two up to 8).  Bounded by the
 // register DFTs and their exchanges through shared memory.  Per pass, against
 // mixed-radix Stockham lines with direct sums over the prime factors:
-// 257 x 257 x 601 27-30 -> 0.89-0.94 ms (its HBM traffic alone: 0.05 ms),
-// 51 x 51 x 401 620-640 -> 31-38 us, 200 x 180 x 400 780-930 -> 240-330 us,
-// 81 x 81 x 101 100 -> 20-24 us, 5 x 5 x 1001 120 -> 45 us.
+// 257 x 257 x 601 27-30 -> 0.9 ms (its HBM traffic alone: 0.05 ms),
+// 51 x 51 x 401 620-640 -> 38-45 us, 200 x 180 x 400 780-930 -> 100-175 us,
+// 81 x 81 x 101 100 -> 23-29 us, 5 x 5 x 1001 120 -> 46 us.
 //
 // Also here: the Burgers step alone on real columns (no transforms).
 //
@@ -20,31 +20,30 @@
 #include "asg_column.cuh"
 #include "asg_lines.cuh"
 
-ASG_DEFINE_ROOT_UPLOADER_HL(asg_roots_upload_tp)
+ASG_DEFINE_LINE_ROOT_UPLOADER(asg_roots_upload_tp)
 
 namespace {
 
 // real samples of one column of a pair: the real or imaginary parts of a padded
 // line in natural order
-template <int N2>
+template <class PL>
 struct PairColumn {
   float* base;  // the line's floats + 0 (column c) or 1 (column c + 1)
-  ASG_DEV int idx(int t) const { return 2 * (t + 2 * (t / N2)); }
-  ASG_DEV float get(int t) const { return base[idx(t)]; }
-  ASG_DEV void set(int t, float v) const { base[idx(t)] = v; }
+  const LineAxis& ax;
+  ASG_DEV float get(int t) const { return base[2 * line_pos<PL>(ax, t)]; }
+  ASG_DEV void set(int t, float v) const { base[2 * line_pos<PL>(ax, t)] = v; }
 };
 
 // the largest |u| of a block's columns into max_next (NaN if one is not finite)
-template <int NW>
 ASG_DEV void block_max_next(float am, unsigned* max_next) {
-  __shared__ float red_max[NW];
+  __shared__ float red_max[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (lane == 0) red_max[warp] = am;
   __syncthreads();
   if (tid == 0) {
     float m = 0.f;
     bool bad = false;
-    for (int w = 0; w < NW; ++w) {
+    for (int w = 0; w < (int)blockDim.x / 32; ++w) {
       const float v = red_max[w];
       bad |= (v != v);
       m = fmaxf(m, v);
@@ -54,21 +53,13 @@ ASG_DEV void block_max_next(float am, unsigned* max_next) {
   }
 }
 
-// Blocks of 128 threads per SM: the registers of the longest in-register DFT (a
-// 32-point one with the chirp's spectrum spills at four blocks).
-template <int M, bool DIRECT>
-constexpr int pair_min_blocks() {
-  return FastPlan<M>::N2 >= 64 ? 2 : FastPlan<M>::N2 >= (DIRECT ? 48 : 32) ? 3 : 4;
-}
-
-template <int M, bool DIRECT>
-__global__ void __launch_bounds__(128, pair_min_blocks<M, DIRECT>())
+template <class PL>
+__global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB)
     tk_pairs(TParams p, LineAxis ax, int lp, int LS) {
   if (*p.status != 0) return;
-  using PL = FastPlan<M>;
-  constexpr int N1 = PL::N1, N2 = PL::N2, NT = 128, NW = NT / 32;
-  constexpr int NA = DIRECT ? N1 : N1 / 2;  // step A inputs that can be non-zero
-  const int n = DIRECT ? M : ax.n;
+  constexpr bool DIRECT = PL::DIRECT;
+  constexpr int S2 = PL::S2;
+  const int n = ax.n, n1 = PL::n1(ax), n2 = PL::n2(ax), NT = blockDim.x, NW = NT / 32;
   const int P = 1 << lp;
   const int F = n / 2 + 1;
   extern __shared__ float4 smraw[];
@@ -76,147 +67,155 @@ __global__ void __launch_bounds__(128, pair_min_blocks<M, DIRECT>())
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ncols = p.ncols;
   const int c0 = blockIdx.x * 2 * P;
-  // position of bin k of a line's spectrum (direct plans: four-step slot order)
-  auto posk = [](int k) { return DIRECT ? PL::pos(PL::slot_of_freq(k)) : PL::pos(k); };
-
-  if (p.in_real) {
-    for (int cc = warp; cc < 2 * P; cc += NW) {
-      PairColumn<N2> col{reinterpret_cast<float*>(lines + (cc >> 1) * LS) + (cc & 1)};
-      const int c = c0 + cc;
-      const float* src = p.real_in + (size_t)c * n;
-      for (int t = lane; t < n; t += 32) col.set(t, c < ncols ? src[t] : 0.f);
-    }
-    __syncthreads();
-  } else {
-    // Z = S_c + i S_{c+1} on all bins from the halves f <= n/2 of both columns
-    // (imaginary parts of bins 0 and n/2 dropped, as irfft does)
-#pragma unroll 4
-    for (int it = tid; it < F * P; it += NT) {
-      const int q = it & (P - 1), f = it >> lp;
-      const int c = c0 + 2 * q;
-      const float2* s = p.spec + (size_t)f * ncols + c;
-      const float2 a = c < ncols ? s[0] : make_float2(0.f, 0.f);
-      const float2 b = c + 1 < ncols ? s[1] : make_float2(0.f, 0.f);
-      float2* line = lines + q * LS;
-      if (f == 0 || 2 * f == n) {
-        line[posk(f)] = make_float2(a.x, b.x);
-      } else {
-        line[posk(f)] = make_float2(a.x - b.y, a.y + b.x);
-        line[posk(n - f)] = make_float2(a.x + b.y, b.x - a.y);
-      }
-    }
-    __syncthreads();
-    if constexpr (!DIRECT) {
-      for (int it = tid; it < P * N2; it += NT) {
-        const int q = it & (P - 1), b = it >> lp;
-        float2* line = lines + q * LS;
-        float2 v[N1];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          const int k = b + N2 * a;
-          v[a] = k < n ? mulc_f4(line[PL::pos(k)], __ldg(ax.ch + k)) : make_float2(0.f, 0.f);
-        }
-        chirp_stepA<PL>(line, b, v, ax.tw);
-      }
-      __syncthreads();
-      for (int it = tid; it < P * N1; it += NT) {
-        const int q = it / N1, ka = it - q * N1;
-        chirp_stepB<PL, true>(lines + q * LS, ka, ax.bt);
-      }
-      __syncthreads();
-      for (int it = tid; it < P * N2; it += NT) {
-        const int q = it & (P - 1), b = it >> lp;
-        float2* line = lines + q * LS;
-        float2 v[N1];
-        chirp_stepA_inv<PL>(line, b, v, ax.tw);
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          const int t = b + N2 * a;
-          if (t < n) line[PL::pos(t)] = scale_hl(mulc_f4(v[a], __ldg(ax.ch + t)), ax.inv_hi, ax.inv_lo);
-        }
-      }
-    } else {
-      for (int it = tid; it < P * N1; it += NT) {
-        const int q = it / N1, ka = it - q * N1;
-        float2* line = lines + q * LS;
-        float2 v[N2];
-        run_load<PL>(line, ka, v);
-        dft<N2, true, true>(v);
-        run_store<PL>(line, ka, v);
-      }
-      __syncthreads();
-      for (int it = tid; it < P * N2; it += NT) {
-        const int q = it & (P - 1), b = it >> lp;
-        float2* line = lines + q * LS;
-        float2 v[N1];
-        chirp_stepA_inv<PL>(line, b, v, ax.tw);
-#pragma unroll
-        for (int a = 0; a < N1; ++a) line[PL::pos(b + N2 * a)] = scale_hl(v[a], ax.inv_hi, ax.inv_lo);
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- column work: a warp per column ----
+  // position of bin k of a line's spectrum: direct plans keep bin ka + n1 kb at slot
+  // kb + S2 ka
+  auto posk = [&](int k) {
+    if (!DIRECT) return line_pos<PL>(ax, k);
+    const int kb = PL::div1(ax, k);
+    return kb + S2 * (k - kb * n1);
+  };
   float am = 0.f;
-#pragma unroll 1
-  for (int cc = warp; cc < 2 * P; cc += NW) {
-    const int c = c0 + cc;
-    if (c >= ncols) continue;
-    PairColumn<N2> col{reinterpret_cast<float*>(lines + (cc >> 1) * LS) + (cc & 1)};
-    const float a = column_phase<0>(col, c, n, p.op, p.stats != 0);
-    am = (a != a || am != am) ? __uint_as_float(0x7fc00000u) : fmaxf(am, a);
-    if (p.write_real) {
-      float* dst = p.real_out + (size_t)c * n;
-      for (int t = lane; t < n; t += 32) dst[t] = col.get(t);
-    }
-  }
-  if (p.stats) block_max_next<NW>(am, p.op.max_next);
-  if (!p.do_r2c) return;
-  __syncthreads();
 
-  // ---- forward transform of the pairs, split into the two columns' bins ----
-  for (int it = tid; it < P * N2; it += NT) {
-    const int q = it & (P - 1), b = it >> lp;
-    float2* line = lines + q * LS;
-    float2 v[N1];
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-      const int t = b + N2 * a;
-      if constexpr (DIRECT) v[a] = line[PL::pos(t)];
-      else v[a] = t < n ? mul_f4(line[PL::pos(t)], __ldg(ax.ch + t)) : make_float2(0.f, 0.f);
-    }
-    if constexpr (DIRECT) direct_stepA<PL>(line, b, v, ax.tw);
-    else chirp_stepA<PL>(line, b, v, ax.tw);
-  }
-  __syncthreads();
-  for (int it = tid; it < P * N1; it += NT) {
-    const int q = it / N1, ka = it - q * N1;
-    float2* line = lines + q * LS;
-    if constexpr (DIRECT) {
-      float2 v[N2];
-      run_load<PL>(line, ka, v);
-      dft<N2, false, true>(v);
-      run_store<PL>(line, ka, v);
-    } else {
-      chirp_stepB<PL, false>(line, ka, ax.bt);
-    }
-  }
-  __syncthreads();
-  if constexpr (!DIRECT) {
-    for (int it = tid; it < P * N2; it += NT) {
-      const int q = it & (P - 1), b = it >> lp;
-      float2* line = lines + q * LS;
-      float2 v[N1];
-      chirp_stepA_inv<PL>(line, b, v, ax.tw);
-#pragma unroll
-      for (int a = 0; a < NA; ++a) {
-        const int k = b + N2 * a;
-        if (k < n) line[PL::pos(k)] = mul_f4(v[a], __ldg(ax.ch + k));
+  // dir 0: spectrum -> samples and the column work; dir 1: samples -> spectrum
+#pragma unroll 1
+  for (int dir = p.in_real ? 1 : 0; dir < 2; ++dir) {
+    if (dir == 0) {
+      // Z = S_c + i S_{c+1} on all bins from the halves f <= n/2 of both columns
+      // (imaginary parts of bins 0 and n/2 dropped, as irfft does)
+#pragma unroll 4
+      for (int it = tid; it < F * P; it += NT) {
+        const int q = it & (P - 1), f = it >> lp;
+        const int c = c0 + 2 * q;
+        const float2* s = p.spec + (size_t)f * ncols + c;
+        const float2 a = c < ncols ? s[0] : make_float2(0.f, 0.f);
+        const float2 b = c + 1 < ncols ? s[1] : make_float2(0.f, 0.f);
+        float2* line = lines + q * LS;
+        if (f == 0 || 2 * f == n) {
+          line[posk(f)] = make_float2(a.x, b.x);
+        } else {
+          line[posk(f)] = make_float2(a.x - b.y, a.y + b.x);
+          line[posk(n - f)] = make_float2(a.x + b.y, b.x - a.y);
+        }
       }
+      __syncthreads();
+    } else if (p.in_real) {
+      for (int cc = warp; cc < 2 * P; cc += NW) {
+        PairColumn<PL> col{reinterpret_cast<float*>(lines + (cc >> 1) * LS) + (cc & 1), ax};
+        const int c = c0 + cc;
+        const float* src = p.real_in + (size_t)c * n;
+        for (int t = lane; t < n; t += 32) col.set(t, c < ncols ? src[t] : 0.f);
+      }
+      __syncthreads();
+    }
+    if (dir == 1) {
+      // ---- column work: a warp per column ----
+#pragma unroll 1
+      for (int cc = warp; cc < 2 * P; cc += NW) {
+        const int c = c0 + cc;
+        if (c >= ncols) continue;
+        PairColumn<PL> col{reinterpret_cast<float*>(lines + (cc >> 1) * LS) + (cc & 1), ax};
+        const float a = column_phase<0>(col, c, n, p.op, p.stats != 0);
+        am = (a != a || am != am) ? __uint_as_float(0x7fc00000u) : fmaxf(am, a);
+        if (p.write_real) {
+          float* dst = p.real_out + (size_t)c * n;
+          for (int t = lane; t < n; t += 32) dst[t] = col.get(t);
+        }
+      }
+      if (p.stats) block_max_next(am, p.op.max_next);
+      if (!p.do_r2c) return;
+      __syncthreads();
+    }
+    const bool inv = dir == 0;
+    if constexpr (!DIRECT) {
+      PL::with_n1(ax, [&](auto R) {
+        constexpr int N1 = decltype(R)::v;
+        for (int it = tid; it < P * n2; it += NT) {
+          const int q = it & (P - 1), b = it >> lp;
+          float2* line = lines + q * LS;
+          float2 v[N1];
+#pragma unroll
+          for (int a = 0; a < N1 / 2; ++a) {
+            const int k = b + n2 * a;
+            v[a] = k < n ? chirp_mul(line[b + S2 * a], ax.ch + k, inv) : make_float2(0.f, 0.f);
+          }
+          line_stepA<PL, N1>(line, b, v, ax);
+        }
+      });
+      __syncthreads();
+      PL::with_n2(ax, [&](auto R) {
+        for (int it = tid; it < P * n1; it += NT) {
+          const int q = PL::div1(ax, it), ka = it - q * n1;
+          chirp_stepB<PL, decltype(R)::v>(lines + q * LS + ka * S2, ka, ax, inv);
+        }
+      });
+      __syncthreads();
+      const float sh = inv ? ax.inv_hi : 1.f, sl = inv ? ax.inv_lo : 0.f;
+      PL::with_n1(ax, [&](auto R) {
+        constexpr int N1 = decltype(R)::v;
+        for (int it = tid; it < P * n2; it += NT) {
+          const int q = it & (P - 1), b = it >> lp;
+          float2* line = lines + q * LS;
+          float2 v[N1];
+          line_stepA_inv<PL, N1>(line, b, v, ax);
+#pragma unroll
+          for (int a = 0; a < N1 / 2; ++a) {
+            const int k = b + n2 * a;
+            if (k < n) line[b + S2 * a] = scale_hl(chirp_mul(v[a], ax.ch + k, inv), sh, sl);
+          }
+        }
+      });
+    } else if (inv) {
+      PL::with_n2(ax, [&](auto R) {
+        constexpr int N2 = decltype(R)::v;
+        for (int it = tid; it < P * n1; it += NT) {
+          const int q = PL::div1(ax, it), ka = it - q * n1;
+          float2* run = lines + q * LS + ka * S2;
+          float2 v[N2];
+          run_load<N2>(run, v);
+          ldft<N2, true>(v);
+          run_store<N2>(run, v);
+        }
+      });
+      __syncthreads();
+      PL::with_n1(ax, [&](auto R) {
+        constexpr int N1 = decltype(R)::v;
+        for (int it = tid; it < P * n2; it += NT) {
+          const int q = it & (P - 1), b = it >> lp;
+          float2* line = lines + q * LS;
+          float2 v[N1];
+          line_stepA_inv<PL, N1>(line, b, v, ax);
+#pragma unroll
+          for (int a = 0; a < N1; ++a) line[b + S2 * a] = scale_hl(v[a], ax.inv_hi, ax.inv_lo);
+        }
+      });
+    } else {
+      PL::with_n1(ax, [&](auto R) {
+        constexpr int N1 = decltype(R)::v;
+        for (int it = tid; it < P * n2; it += NT) {
+          const int q = it & (P - 1), b = it >> lp;
+          float2* line = lines + q * LS;
+          float2 v[N1];
+#pragma unroll
+          for (int a = 0; a < N1; ++a) v[a] = line[b + S2 * a];
+          line_stepA<PL, N1>(line, b, v, ax);
+        }
+      });
+      __syncthreads();
+      PL::with_n2(ax, [&](auto R) {
+        constexpr int N2 = decltype(R)::v;
+        for (int it = tid; it < P * n1; it += NT) {
+          const int q = PL::div1(ax, it), ka = it - q * n1;
+          float2* run = lines + q * LS + ka * S2;
+          float2 v[N2];
+          run_load<N2>(run, v);
+          ldft<N2, false>(v);
+          run_store<N2>(run, v);
+        }
+      });
     }
     __syncthreads();
   }
+
   float2* so = p.spec_out ? p.spec_out : p.spec;
 #pragma unroll 4
   for (int it = tid; it < F * P; it += NT) {
@@ -250,27 +249,32 @@ __global__ void __launch_bounds__(256) k_flux_columns(TParams p) {
   for (int t = lane; t < nT; t += 32) dst[t] = col.get(t);
 }
 
-template <int M, bool DIRECT>
+template <class PL>
 int launch_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
-  using PL = FastPlan<M>;
-  // pairs per block: as many as 72 KB hold, fewer while the grid leaves the GPU
-  // idle (two blocks for each of its 152 SMs)
-  const int npairs = (p.ncols + 1) / 2;
-  int lp = 3;
-  while (lp > 0 && ((size_t)line_stride(PL::PADDED, 1 << lp) * sizeof(float2) << lp) > 72 * 1024)
-    --lp;
-  while (lp > 0 && (npairs >> lp) < 2 * 152) --lp;
-  const int P = 1 << lp, LS = line_stride(PL::PADDED, P);
+  // pairs per block: what fills it, at least 4 (64-byte runs in HBM), while 72 KB
+  // hold them and the grid does not leave the GPU idle (two blocks for each of its
+  // 152 SMs)
+  const int npairs = (p.ncols + 1) / 2, tasks = line_tasks(ax);
+  int lp = 0;
+  while (lp < 5 && (lp < 2 || (tasks << lp) < LineBlock<PL::BIG>::NT)) {
+    const int k = lp + 1;
+    if (((size_t)line_stride(ax, 1 << k) * sizeof(float2) << k) > 72 * 1024) break;
+    if ((npairs >> k) < 2 * 152) break;
+    lp = k;
+  }
+  const int P = 1 << lp, LS = line_stride(ax, P);
   const size_t smem = (size_t)P * LS * sizeof(float2);
+  // (four warps even where the steps have fewer tasks: the column work, the loads)
+  const int nt = LineBlock<PL::BIG>::NT;
   static bool attr_done[ASG_MAX_DEVICES] = {};
   const int dev = asg_device_slot();
   if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(tk_pairs<M, DIRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(tk_pairs<PL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              72 * 1024) != cudaSuccess)
       return ASG_ERR_CUDA;
     attr_done[dev] = true;
   }
-  tk_pairs<M, DIRECT><<<(npairs + P - 1) / P, 128, smem, st>>>(p, ax, lp, LS);
+  tk_pairs<PL><<<(npairs + P - 1) / P, nt, smem, st>>>(p, ax, lp, LS);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
 }
 
@@ -278,41 +282,17 @@ int launch_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
 
 int asg_launch_t_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
   if (ax.n != p.nT) return ASG_ERR_SHAPE;
-  if (ax.direct) {
-    switch (ax.m) {
-      case 32: return launch_pairs<32, true>(p, ax, st);
-      case 64: return launch_pairs<64, true>(p, ax, st);
-      case 96: return launch_pairs<96, true>(p, ax, st);
-      case 128: return launch_pairs<128, true>(p, ax, st);
-      case 192: return launch_pairs<192, true>(p, ax, st);
-      case 256: return launch_pairs<256, true>(p, ax, st);
-      case 384: return launch_pairs<384, true>(p, ax, st);
-      case 512: return launch_pairs<512, true>(p, ax, st);
-      case 576: return launch_pairs<576, true>(p, ax, st);
-      case 768: return launch_pairs<768, true>(p, ax, st);
-      case 1024: return launch_pairs<1024, true>(p, ax, st);
-      case 1536: return launch_pairs<1536, true>(p, ax, st);
-      case 2048: return launch_pairs<2048, true>(p, ax, st);
-      default: return ASG_ERR_SHAPE;
-    }
-  }
-  switch (ax.m) {
-    case 32: return launch_pairs<32, false>(p, ax, st);
-    case 64: return launch_pairs<64, false>(p, ax, st);
-    case 96: return launch_pairs<96, false>(p, ax, st);
-    case 128: return launch_pairs<128, false>(p, ax, st);
-    case 192: return launch_pairs<192, false>(p, ax, st);
-    case 256: return launch_pairs<256, false>(p, ax, st);
-    case 384: return launch_pairs<384, false>(p, ax, st);
-    case 512: return launch_pairs<512, false>(p, ax, st);
-    case 576: return launch_pairs<576, false>(p, ax, st);
-    case 768: return launch_pairs<768, false>(p, ax, st);
-    case 1024: return launch_pairs<1024, false>(p, ax, st);
-    case 1536: return launch_pairs<1536, false>(p, ax, st);
-    case 2048: return launch_pairs<2048, false>(p, ax, st);
-    case 4096: return launch_pairs<4096, false>(p, ax, st);
-    default: return ASG_ERR_SHAPE;
-  }
+  if (ax.direct)
+    return ax.rm == 16 ? launch_pairs<DirectPlan<16>>(p, ax, st)
+         : ax.rm == 24 ? launch_pairs<DirectPlan<24>>(p, ax, st)
+         : ax.rm == 32 ? launch_pairs<DirectPlan<32>>(p, ax, st)
+                       : launch_pairs<DirectPlan<64>>(p, ax, st);
+#define F(a, b) \
+  if (ax.n1 == a && ax.n2 == b) return launch_pairs<ChirpPlan<a, b>>(p, ax, st);
+  ASG_CHIRP_SIZES(F)
+  F(64, 64)
+#undef F
+  return ASG_ERR_SHAPE;
 }
 
 int asg_launch_flux_columns(const TParams& p, cudaStream_t st) {

@@ -23,3 +23,28 @@ ASG_DEV bool xy_should_skip(const XYParams& p) {
 }
 
 ASG_DEV bool is_dc_or_nyq(int f, int nT) { return f == 0 || 2 * f == nT; }
+
+// Engquist-Majda correction of `cur` at edge coordinate i of n (weight w)
+ASG_DEV float2 edge_correct(float2 prev, float2 cur, float2 next, int i, int n, float w, float cf,
+                            float st, float inv2d, float invd) {
+  float2 d;
+  if (i == 0) d = cscale(csub(next, cur), invd);
+  else if (i == n - 1) d = cscale(csub(cur, prev), invd);
+  else d = cscale(csub(next, prev), inv2d);
+  const float2 cd = make_float2(cf * d.y, -cf * d.x);
+  const float2 P = (i < n / 2) ? make_float2(0.5f * (cur.x + cd.x), 0.5f * (cur.y + cd.y))
+                               : make_float2(0.5f * (cur.x - cd.x), 0.5f * (cur.y - cd.y));
+  return make_float2(cur.x - st * w * P.x, cur.y - st * w * P.y);
+}
+
+constexpr size_t LINE_SMEM = 72 * 1024;  // shared memory of a block at most
+
+template <class K>
+inline int line_smem_attr(K kern, bool* done) {
+  if (*done) return ASG_OK;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LINE_SMEM) !=
+      cudaSuccess)
+    return ASG_ERR_CUDA;
+  *done = true;
+  return ASG_OK;
+}
