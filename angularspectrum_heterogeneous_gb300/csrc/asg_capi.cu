@@ -440,7 +440,7 @@ struct asg_plan {
   SourceEvent* d_src = nullptr;    // per-step list (max 64)
   // state
   int* d_step = nullptr;
-  unsigned *d_max_cur = nullptr, *d_max_next = nullptr, *d_status = nullptr;
+  unsigned *d_max_cur = nullptr, *d_max_next = nullptr, *d_status = nullptr, *d_done = nullptr;
   int* d_status_step = nullptr;
   double* d_iprev = nullptr;
   unsigned* d_hist = nullptr;
@@ -539,7 +539,7 @@ extern "C" int asg_plan_destroy(asg_plan* p) {
                   p->abl_xy_full, p->abl_t_full, p->fw_lx, p->fw_ly, p->fw_exp, p->sa_wx,
                   p->sa_wy, p->sa_coef, p->screen_fscale, p->obl_tab, p->power_acc,
                   p->d_screens, p->d_src, p->d_step, p->d_max_cur, p->d_max_next,
-                  p->d_status, p->d_status_step, p->d_iprev, p->d_hist, p->d_clamp};
+                  p->d_status, p->d_status_step, p->d_iprev, p->d_hist, p->d_clamp, p->d_done};
   for (void* q : ptrs) cudaFree(q);
   free_axis(p->ax_t);
   free_axis(p->ax_x);
@@ -756,6 +756,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   CKS(dalloc(&p->d_step, 1));
   CKS(dalloc(&p->d_max_cur, 1));
   CKS(dalloc(&p->d_max_next, 1));
+  CKS(dalloc(&p->d_done, 1));
   CKS(dalloc(&p->d_status, 1));
   CKS(dalloc(&p->d_status_step, 1));
   CKS(dalloc(&p->d_iprev, p->ncols));
@@ -1034,6 +1035,20 @@ extern "C" int asg_add_source_compact(asg_plan* p, double z, const int* cols, in
 // ---------------------------------------------------------------------------
 // kernel parameter helpers
 // ---------------------------------------------------------------------------
+// Programmatic dependent launches along the plan's stream; not inside a batch, whose
+// graph joins the streams of several plans, nor between timing events.
+static int use_pdl(const asg_plan* p) { return p->batch_refs == 0 && !p->prof; }
+
+// Whether the statistics pass closes the step itself (stats_block_done) or a one-thread
+// launch does: 2 M samples and fewer (81 x 81 x 101 3 us per step less; at 128 x 128 x 256
+// both cost the same, at 512 x 512 x 1024 the fused end takes 28 us, the launch 3).
+static bool step_end_fused(const asg_plan* p) { return (size_t)p->ncols * p->T <= (1u << 21); }
+static int close_step(asg_plan* p) {
+  if (step_end_fused(p)) return ASG_OK;
+  KScope k(p, ASG_K_OTHER);
+  return asg_launch_advance(p->d_step, p->d_max_cur, p->d_max_next, use_pdl(p), p->st);
+}
+
 static TParams tparams(asg_plan* p) {
   TParams t;
   memset(&t, 0, sizeof(t));
@@ -1054,6 +1069,9 @@ static TParams tparams(asg_plan* p) {
   t.op.ncols = p->ncols;
   t.op.iprev = p->d_iprev;
   t.op.max_next = p->d_max_next;
+  t.op.max_cur = p->d_max_cur;
+  t.op.done = step_end_fused(p) ? p->d_done : nullptr;
+  t.pdl = use_pdl(p);
   t.op.pnp = p->o_pnp;
   t.op.ppp = p->o_ppp;
   t.op.pI = p->o_pI;
@@ -1087,6 +1105,7 @@ static XYParams xyparams(asg_plan* p, const float2* table, bool zero_dc_nyq) {
   XYParams x;
   memset(&x, 0, sizeof(x));
   x.spec = p->spec;
+  x.pdl = use_pdl(p);
   x.X = p->X;
   x.Y = p->Y;
   x.G = p->G;
@@ -1404,8 +1423,7 @@ static int march_step(asg_plan* p, const Slot& s, double dzs, double btvd, int n
   t.real_out = p->real;
   t.do_r2c = last ? 0 : 1;
   CKS(run_t(p, t, ASG_K_T_END));
-  KScope k(p, ASG_K_OTHER);
-  return asg_launch_advance(p->d_step, p->d_max_cur, p->d_max_next, p->st);
+  return close_step(p);
 }
 
 // A regular step replays the captured graph of one march step.  The first
@@ -1504,6 +1522,7 @@ static int prepare_run(asg_plan* p, const float* init, double prop_dist, double 
   CK(cudaMemsetAsync(p->d_max_cur, 0, sizeof(unsigned), p->st));
   CK(cudaMemsetAsync(p->d_max_next, 0, sizeof(unsigned), p->st));
   CK(cudaMemsetAsync(p->d_status_step, 0, sizeof(int), p->st));
+  CK(cudaMemsetAsync(p->d_done, 0, sizeof(unsigned), p->st));
   CK(cudaMemsetAsync(p->d_clamp, 0, 2 * sizeof(unsigned), p->st));
   CKS(copy_host(p->real, init, (size_t)p->ncols * p->T * sizeof(float), cudaMemcpyHostToDevice,
                 p->st));
@@ -1517,7 +1536,7 @@ static int prepare_run(asg_plan* p, const float* init, double prop_dist, double 
     t.do_r2c = 1;
     CKS(run_t(p, t));
     // max_cur <- max_next, step stays 0
-    CKS(asg_launch_advance(p->d_step, p->d_max_cur, p->d_max_next, p->st));
+    CKS(close_step(p));
     CK(cudaMemsetAsync(p->d_step, 0, sizeof(int), p->st));
   }
   p->zaxis.clear();

@@ -48,13 +48,15 @@ struct ColumnOps {
   const SourceEvent* src;
   // accumulators (step end); step index read from *step
   int accumulate;
-  const int* step;
+  int* step;
   float *pnp, *ppp, *pI, *pIloss;  // [step][ncols]
   float* pax;                       // [step][nT]
   int pax_col;
   int ncols;
   double* iprev;                    // [ncols]
   unsigned* max_next;               // stability max of the field entering the next step
+  unsigned* max_cur;                // the same of the step under way
+  unsigned* done;                   // blocks of the statistics pass that have finished, or null
   unsigned* subcycle_hist;          // optional [64] histogram of per-column sub-cycles
   unsigned* subcycle_clamp;         // optional [2]: columns whose sub-cycle count was capped at
                                     // max_subcycles, and the largest count one of them needed
@@ -84,6 +86,22 @@ struct PlainColumn {
   static constexpr bool kVecRun = false;
   ASG_DEV float4* run4(int t0) const { return reinterpret_cast<float4*>(base + t0); }
 };
+// End of a block of the statistics pass, one thread, after the block's columns: its
+// largest |u| (NaN if not finite) into max_next.  With op.done the grid's last block
+// also closes the step (step counter, stability maxima) in place of a launch; the fence
+// and the count cost each block about a microsecond, so this is for small grids.
+ASG_DEV void stats_block_done(const ColumnOps& op, float m, unsigned nblocks) {
+  atomicMax(op.max_next, float_as_ordered(m));
+  if (op.done == nullptr) return;
+  __threadfence();
+  if (atomicAdd(op.done, 1u) == nblocks - 1) {
+    __threadfence();
+    *op.max_cur = atomicExch(op.max_next, 0u);
+    *op.step += 1;
+    *op.done = 0u;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // flux primitives (float32, same formulas and order as the reference)
 // ---------------------------------------------------------------------------

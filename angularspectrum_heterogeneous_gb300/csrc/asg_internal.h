@@ -11,6 +11,31 @@ struct SourceEvent;
 struct GenPlan;
 struct LineAxis;  // asg_lines.cuh
 
+// Programmatic dependent launch: the next kernel of the stream is set up while the
+// previous one runs and waits for its results (pdl_wait) after its own reads of
+// constant tables; a no-op in a launch without the attribute.  A march step is 5-13
+// short launches on small grids: 81 x 81 x 101 130 -> 125 us per step, 96 x 96 x 192
+// 140 -> 137 us.  No kernel triggers its dependents early: blocks of the next kernel
+// that sit waiting on the SMs cost more than they save (139 and 161 us).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// launch of a kernel that calls pdl_wait() before it touches what earlier kernels write
+template <class... P, class... A>
+inline int asg_launch_pdl(bool pdl, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...) == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+}
+
 // ---- t-column pass ---------------------------------------------------------
 #include "asg_column.cuh"
 
@@ -31,6 +56,7 @@ struct TParams {
   const float2* tw;      // W_nT^k, k < nT
   const float2* twM;     // W_M^k,  k < M (fast kernels)
   const unsigned* status;
+  int pdl;               // programmatic dependent launch
   int cols_per_block;    // fast kernels: 8 or 16 columns per block, 0 = default
   int prefetch;          // fast kernels: 1 = each block prefetches into L2 the spectrum of the
                          // tile that starts about one block lifetime later (set by the launcher)
@@ -60,6 +86,7 @@ enum EpiFlags : int {
 
 struct XYParams {
   float2* spec;          // [planes][X][Y]
+  int pdl;               // programmatic dependent launch (not with coop)
   int X, Y, G;           // G CTAs per (sub-)plane (thread-block cluster)
   int nsub;              // sub-planes per plane along x (1, or 2 when the column pass
                          // applies the first radix-2 stage of the x transform)
@@ -140,6 +167,9 @@ int asg_launch_xy_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaS
 int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPlan& ply,
                   cudaStream_t st);
 
+// device-side bookkeeping between steps
+int asg_launch_advance(int* step, unsigned* max_cur, unsigned* max_next, int pdl, cudaStream_t st);
+
 // ---- set-up kernels (FP64) -------------------------------------------------
 struct TableParams {
   int nplanes, ncx, ncy;
@@ -164,8 +194,6 @@ struct TableParams {
 int asg_launch_table(const TableParams& p, cudaStream_t st);
 int asg_launch_obl_table(const TableParams& p, float* out, cudaStream_t st);
 
-// device-side bookkeeping between steps
-int asg_launch_advance(int* step, unsigned* max_cur, unsigned* max_next, cudaStream_t st);
 // (x,y,nZ) <- [nZ][x*y] transposes for the outputs
 int asg_launch_transpose(const float* in, float* out, int nz, int ncols, cudaStream_t st);
 

@@ -161,14 +161,14 @@ int asg_launch_obl_table(const TableParams& p, float* out, cudaStream_t st) {
 
 // one thread: advance the step counter and rotate the stability maxima
 __global__ void k_advance(int* step, unsigned* max_cur, unsigned* max_next) {
+  pdl_wait();
   *step += 1;
   *max_cur = *max_next;
   *max_next = 0u;
 }
 
-int asg_launch_advance(int* step, unsigned* max_cur, unsigned* max_next, cudaStream_t st) {
-  k_advance<<<1, 1, 0, st>>>(step, max_cur, max_next);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+int asg_launch_advance(int* step, unsigned* max_cur, unsigned* max_next, int pdl, cudaStream_t st) {
+  return asg_launch_pdl(pdl != 0, k_advance, dim3(1), dim3(1), 0, st, step, max_cur, max_next);
 }
 
 // out[c*nz + z] = in[z*ncols + c]

@@ -39,7 +39,6 @@ enum TMode : int { TM_PLAIN = 0, TM_FLUX = 1, TM_STATS = 2 };
 template <class PL, int MODE, int C>
 __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
     tk_fast(TParams p) {
-  if (*p.status != 0) return;
   static_assert(C == 8 || C == 16, "8 or 16 columns per block");
   constexpr int CPW = C / 8;   // columns per warp
   constexpr int CY = C / 2;    // consecutive y per row
@@ -67,6 +66,10 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
   // tile -> (x, y0); column cc: row x + (cc >= CY)*X/2, y = y0 + cc % CY
   const int tile = blockIdx.x;
   const int xq = tile / (Y / CY), y0 = CY * (tile - xq * (Y / CY));
+  for (int i = tid; i < M; i += nthr) twM[i] = p.twM[i];
+  const float2 wx = p.twX[xq];  // W_X^x of this tile's column pair
+  pdl_wait();
+  if (*p.status != 0) return;
   if (p.prefetch_ahead > 0 && !p.in_real) {
     // blocks start in about index order: the tile of block b + (resident
     // blocks) starts about when this one ends, so its spectrum goes to L2 now
@@ -82,8 +85,6 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
       }
     }
   }
-  for (int i = tid; i < M; i += nthr) twM[i] = p.twM[i];
-  const float2 wx = p.twX[xq];  // W_X^x of this tile's column pair
   auto col_of = [&](int cc) {
     return (xq + (cc >= CY ? X2 : 0)) * Y + y0 + (cc & (CY - 1));
   };
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
         m = fmaxf(m, v);
       }
       if (bad) m = __uint_as_float(0x7fc00000u);
-      atomicMax(p.op.max_next, float_as_ordered(m));
+      stats_block_done(p.op, m, gridDim.x);
     }
   }
   if (!p.do_r2c) return;
@@ -332,8 +333,7 @@ static int launch_fast_t_mode(const TParams& p, cudaStream_t st) {
   const int grid = (p.X / 2) * (p.Y / (C / 2));
   TParams q = p;
   q.prefetch_ahead = p.prefetch ? resident[dev] : 0;
-  tk_fast<PL, MODE, C><<<grid, 256, smem, st>>>(q);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, tk_fast<PL, MODE, C>, dim3(grid), dim3(256), smem, st, q);
 }
 
 // 16 columns per block exist up to 1024-sample columns (three blocks of 256

@@ -35,7 +35,7 @@ struct PairColumn {
 };
 
 // the largest |u| of a block's columns into max_next (NaN if one is not finite)
-ASG_DEV void block_max_next(float am, unsigned* max_next) {
+ASG_DEV void block_max_next(float am, const ColumnOps& op) {
   __shared__ float red_max[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (lane == 0) red_max[warp] = am;
@@ -49,13 +49,14 @@ ASG_DEV void block_max_next(float am, unsigned* max_next) {
       m = fmaxf(m, v);
     }
     if (bad) m = __uint_as_float(0x7fc00000u);
-    atomicMax(max_next, float_as_ordered(m));
+    stats_block_done(op, m, gridDim.x);
   }
 }
 
 template <class PL>
 __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB)
     tk_pairs(TParams p, LineAxis ax, int lp, int LS) {
+  pdl_wait();
   if (*p.status != 0) return;
   constexpr bool DIRECT = PL::DIRECT;
   constexpr int S2 = PL::S2;
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
           for (int t = lane; t < n; t += 32) dst[t] = col.get(t);
         }
       }
-      if (p.stats) block_max_next(am, p.op.max_next);
+      if (p.stats) block_max_next(am, p.op);
       if (!p.do_r2c) return;
       __syncthreads();
     }
@@ -274,8 +275,8 @@ int launch_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
       return ASG_ERR_CUDA;
     attr_done[dev] = true;
   }
-  tk_pairs<PL><<<(npairs + P - 1) / P, nt, smem, st>>>(p, ax, lp, LS);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, tk_pairs<PL>, dim3((npairs + P - 1) / P), dim3(nt), smem, st, p,
+                        ax, lp, LS);
 }
 
 }  // namespace

@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT,
                                       ? 3  // both convolutions' code: 168 registers
                                       : LineBlock<PL::BIG>::MB)
     xy_cols(XYParams p, LineAxis ax, float2* buf, int lc, int LS) {
+  pdl_wait();
   if (xy_should_skip(p)) return;
   extern __shared__ float4 smraw[];
   float2* lines = reinterpret_cast<float2*>(smraw);
@@ -201,9 +202,9 @@ int launch_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaStream_t
   static bool done[ASG_MAX_DEVICES] = {};
   const int s = line_smem_attr(xy_cols<PL>, &done[asg_device_slot()]);
   if (s != ASG_OK) return s;
-  xy_cols<PL><<<dim3((p.Y + C - 1) / C, p.nplanes), line_threads(C * tasks, LineBlock<PL::BIG>::NT),
-                        smem, st>>>(p, ax, buf, lc, LS);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, xy_cols<PL>, dim3((p.Y + C - 1) / C, p.nplanes),
+                        dim3(line_threads(C * tasks, LineBlock<PL::BIG>::NT)), smem, st, p, ax, buf,
+                        lc, LS);
 }
 
 }  // namespace

@@ -292,7 +292,6 @@ __global__ void __launch_bounds__(NT, (NT == 256 ? 2 : 1)) xy_fast(XYParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nq = p.nplanes * nsub;
 
-  if (xy_should_skip(p)) return;
   for (int i = tid; i < Y; i += NT) {
     twY[i] = p.twY[i];
     clsy[i] = p.cls_y[i];
@@ -303,6 +302,8 @@ __global__ void __launch_bounds__(NT, (NT == 256 ? 2 : 1)) xy_fast(XYParams p) {
     const int h = i / R, j = i - (i / R) * R;
     clsx[i] = p.cls_x[h * Xs + rank * R + j];
   }
+  pdl_wait();
+  if (xy_should_skip(p)) return;
   auto zero_plane = [&](int q) {
     return p.zero_dc_nyq && is_dc_or_nyq(p.f_of_plane[q / nsub], p.nT);
   };
@@ -511,6 +512,7 @@ __global__ void __launch_bounds__(256) xy_generic(XYParams p, GenPlan plx, GenPl
   __shared__ float red[2][8];
   const int plane = blockIdx.y;
   const int tid = threadIdx.x, nthr = blockDim.x;
+  pdl_wait();
   if (xy_should_skip(p)) return;
   const int f = p.f_of_plane[plane];
   float2* gplane = p.spec + (size_t)plane * X * Y;
@@ -591,6 +593,7 @@ __global__ void __launch_bounds__(256) xy_epilogue_pass(XYParams p, const float2
                                                         float2* __restrict__ dst, int split) {
   __shared__ float2 S[EPT + 2][EPT + 3];
   __shared__ float2 XS[EPT][EPT + 3];
+  pdl_wait();
   if (*((volatile const unsigned*)p.status) != 0u) return;
   const int X = p.X, Y = p.Y, X2 = p.X / 2;
   const int ty = (Y + EPT - 1) / EPT;
@@ -694,8 +697,8 @@ __global__ void __launch_bounds__(256) xy_epilogue_pass(XYParams p, const float2
 int asg_launch_epilogue_pass(const XYParams& p, const float2* src, float2* dst, int split,
                              cudaStream_t st) {
   const int tiles = ((p.X + EPT - 1) / EPT) * ((p.Y + EPT - 1) / EPT);
-  xy_epilogue_pass<<<dim3(tiles, p.nplanes, 1), 256, 0, st>>>(p, src, dst, split);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, xy_epilogue_pass, dim3(tiles, p.nplanes, 1), dim3(256), 0, st, p,
+                        src, dst, split);
 }
 
 // ---------------------------------------------------------------------------
@@ -749,7 +752,7 @@ static int launch_fast_xy(const XYParams& p, cudaStream_t st) {
   }
   auto kern = xy_fast<PY, R, NT>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = p.G;
   attr[0].val.clusterDim.y = 1;
@@ -770,6 +773,9 @@ static int launch_fast_xy(const XYParams& p, cudaStream_t st) {
     max_clusters = n;
     cached_G = p.G;
   }
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = p.pdl ? 2 : 1;
   const int nq = p.nplanes * p.nsub;
   const int ncl = max_clusters < nq ? max_clusters : nq;
   cfg.gridDim = dim3(p.G * ncl, 1, 1);
@@ -809,6 +815,6 @@ int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPla
   if (cudaFuncSetAttribute(xy_generic, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return ASG_ERR_CUDA;
-  xy_generic<<<dim3(1, p.nplanes, 1), 256, smem, st>>>(p, plx, ply);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, xy_generic, dim3(1, p.nplanes, 1), dim3(256), smem, st, p, plx,
+                        ply);
 }

@@ -245,7 +245,6 @@ __global__ void __launch_bounds__(NT, L2Shape<PY, NT>::kMinBlocks) xy_l2(XYParam
   };
   const int nsub = p.nsub;
   const int nq = p.nplanes * nsub;
-  if (l2_should_skip(p)) return;
   if (lane == 0) {
     mbar_init(&row_mbar[warp], 1);
     mbar_init_fence();
@@ -263,6 +262,8 @@ __global__ void __launch_bounds__(NT, L2Shape<PY, NT>::kMinBlocks) xy_l2(XYParam
     for (int i = tid; i < Xs; i += NT) tw_x_s[i] = p.twX[i * nsub];  // W_Xs^i
     for (int i = tid; i < nsub * Xs; i += NT) clsx_s[i] = p.l2_cls_x[i];
   }
+  pdl_wait();
+  if (l2_should_skip(p)) return;
   const int nsub_l = nsub;
   auto tw_x = [&](int i) { return TS_SMEM ? tw_x_s[i] : __ldg(p.twX + i * nsub_l); };
   float2* scratch0 = p.l2_scratch + (size_t)cid * 2 * Xs * Y;
@@ -641,7 +642,6 @@ __global__ void __launch_bounds__(NT, L2Shape<PY, NT>::kMinBlocks) xy_l2c(XYPara
   const int rank = coop ? (int)(blockIdx.x % G) : (G > 1) ? (int)cl.block_rank() : 0;
   const int cid = blockIdx.x / G, ncl = gridDim.x / G;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (*((volatile const unsigned*)p.status) != 0u) return;
   __shared__ int sync_ok;
   __shared__ uint64_t row_mbar[NW];  // bulk row loads of each warp
   if (lane == 0) {
@@ -683,6 +683,8 @@ __global__ void __launch_bounds__(NT, L2Shape<PY, NT>::kMinBlocks) xy_l2c(XYPara
   }
   const bool fw = (p.epi & EPI_FREQW) != 0, sa = (p.epi & EPI_SUPERABS) != 0;
   const float st = p.sa_strength;
+  pdl_wait();
+  if (*((volatile const unsigned*)p.status) != 0u) return;
 
   // loads of my warp's rows of half-plane h of `plane`: bulk copies (bulk_rows
   // 2), or 16-byte cp.async
@@ -1040,14 +1042,20 @@ static int launch_groups(K kern, const XYParams& p, cudaLaunchConfig_t cfg, int 
   int ng = resident < units ? resident : units;
   if (ng > p.l2_max_clusters) ng = p.l2_max_clusters;
   if (ng < 1) return ASG_ERR_SHAPE;
-  cudaLaunchAttribute coop[1];
+  cudaLaunchAttribute coop[1], cluster[2];
+  if (!p.coop && p.pdl) {
+    cluster[0] = cfg.attrs[0];
+    cluster[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    cluster[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = cluster;
+    cfg.numAttrs = 2;
+  }
   if (p.coop) {
     if (p.grp_cnt == nullptr) return ASG_ERR_ARG;
     // every CTA of the grid is resident, so the counter barriers of a group
     // always complete
-    if (cudaMemsetAsync(p.grp_cnt, 0, (size_t)ng * sizeof(unsigned), st) != cudaSuccess ||
-        cudaMemsetAsync(p.grp_cnt + p.l2_max_clusters, 0, (size_t)ng * sizeof(unsigned), st) !=
-            cudaSuccess)
+    if (cudaMemsetAsync(p.grp_cnt, 0, (size_t)(p.l2_max_clusters + ng) * sizeof(unsigned), st) !=
+        cudaSuccess)
       return ASG_ERR_CUDA;
     coop[0].id = cudaLaunchAttributeCooperative;
     coop[0].val.cooperative = 1;

@@ -36,6 +36,7 @@ namespace {
 template <class PL, bool INV>
 __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB)
     xy_rows(XYParams p, LineAxis ax, float2* dst, int L, int LS) {
+  pdl_wait();
   if (xy_should_skip(p)) return;
   extern __shared__ float4 smraw[];
   float2* lines = reinterpret_cast<float2*>(smraw);
@@ -202,9 +203,8 @@ int launch_rows(const XYParams& p, const LineAxis& ax, float2* dst, bool inverse
                         : line_smem_attr(xy_rows<PL, false>, &done[0][dev]);
   if (s != ASG_OK) return s;
   const int grid = (total + L - 1) / L, nt = line_threads(L * tasks, LineBlock<PL::BIG>::NT);
-  if (inverse) xy_rows<PL, true><<<grid, nt, smem, st>>>(p, ax, dst, L, LS);
-  else xy_rows<PL, false><<<grid, nt, smem, st>>>(p, ax, dst, L, LS);
-  return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+  return asg_launch_pdl(p.pdl != 0, inverse ? xy_rows<PL, true> : xy_rows<PL, false>, dim3(grid),
+                        dim3(nt), smem, st, p, ax, dst, L, LS);
 }
 
 }  // namespace
