@@ -147,7 +147,13 @@ static float4 two_floats(double re, double im) {
   return make_float4(x, y, (float)(re - (double)x), (float)(im - (double)y));
 }
 
+// Resident CTA groups of the L2 plane kernels: the tuning knobs cap them at 1..64 (64: no
+// cap).  The scratch holds 64 from 256-wide planes up, where fewer are resident, and
+// 256 below: 114 groups of the 128-wide planes fit the GPU, and 128 x 128 x 256's
+// 258 half-planes took 5 rounds of 64 groups, 41 -> 33 us per stage (192 x 192 x 512
+// 125 -> 111, 64 x 128 x 256 33 -> 22).
 static constexpr int L2_MAX_CLUSTERS = 64;
+static int l2_group_cap(int Y) { return Y >= 256 ? L2_MAX_CLUSTERS : 256; }
 
 // four-step slot order of a fast line of length n (n = n1*n2)
 static void fast_factors(int n, int* n1, int* n2) {
@@ -385,7 +391,7 @@ struct asg_plan {
   int xy_sync = 0;            // group barrier of the L2 plane kernels: 0 default,
                               // 1 thread-block cluster, 2 counters in a cooperative launch
   int batch_refs = 0;         // batches holding the plan (they use cluster barriers)
-  unsigned* grp_cnt = nullptr;  // [L2_MAX_CLUSTERS] counters of the cooperative launch
+  unsigned* grp_cnt = nullptr;  // [2][groups] counters of the cooperative launch
   unsigned barrier_skew = 0;    // test hook: added to the group-barrier targets
   // CUDA graph of a regular march step (slot 0, no screen, source, callback,
   // profiling or output write); rebuilt when `gen` moves on
@@ -589,8 +595,12 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   int Gs = 0, Gl = 0;
   p->l2 = p->tfast && asg_xy_l2_supported(X, Y, 2, &Gl);
   p->xy_bulk = default_bulk(p);
-  p->split = p->l2 || (p->tfast && asg_xy_split_supported(X, Y, &Gs));
-  p->xyfast = p->split || asg_xy_fast_supported(X, Y, &p->G);
+  // planes much longer along x than along y leave a cluster's CTAs little work between
+  // their exchanges of all x: 256 x 128 x 256 107 us per stage against 80 us for the row
+  // and column passes, 512 x 128 x 256 280 against 184 (384 x 256: 254 and 250)
+  const bool tall = !p->l2 && X >= 256 && X >= 2 * Y;
+  p->split = p->l2 || (!tall && p->tfast && asg_xy_split_supported(X, Y, &Gs));
+  p->xyfast = p->split || (!tall && asg_xy_fast_supported(X, Y, &p->G));
   p->nsub = 1;
   if (p->split) {
     p->G = p->l2 ? Gl : Gs;
@@ -697,9 +707,9 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     if (2 * p->h_f_of_plane[q] == T) p->nyq_plane = q;
   if ((p->l2 || p->lines) && p->nyq_plane >= 0) CKS(dalloc(&p->nyq_tmp, (size_t)X * Y));
   if (p->l2) {
-    // scratch for up to L2_MAX_CLUSTERS clusters, two half-planes each
+    // scratch: two half-planes for each resident group
     const int Xs = X / 2;
-    CKS(dalloc(&p->l2_scratch, (size_t)L2_MAX_CLUSTERS * 2 * Xs * Y));
+    CKS(dalloc(&p->l2_scratch, (size_t)l2_group_cap(Y) * 2 * Xs * Y));
     int n1, n2;
     fast_factors(Xs, &n1, &n2);
     std::vector<int> cl(2 * Xs);
@@ -713,7 +723,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
       }
     CKS(dalloc(&p->l2_cls_x, 2 * Xs));
     CKS(h2d(p->l2_cls_x, cl.data(), 2 * Xs, p->st));
-    CKS(dalloc(&p->grp_cnt, 2 * L2_MAX_CLUSTERS));
+    CKS(dalloc(&p->grp_cnt, 2 * l2_group_cap(Y)));
   }
   CKS(dalloc(&p->real, (size_t)p->ncols * T));
   std::vector<float2> w;
@@ -1142,7 +1152,7 @@ static XYParams xyparams(asg_plan* p, const float2* table, bool zero_dc_nyq) {
   x.l2_scratch = p->l2_scratch;
   x.l2_cls_x = p->l2_cls_x;
   x.l2_max_clusters = (p->xy_clusters > 0 && p->xy_clusters < L2_MAX_CLUSTERS)
-                          ? p->xy_clusters : L2_MAX_CLUSTERS;
+                          ? p->xy_clusters : l2_group_cap(p->Y);
   x.coop = xy_sync_of(p) >= 2 ? 1 : 0;
   x.pipe = xy_sync_of(p) == 3 ? 1 : 0;
   x.bulk_rows = p->xy_bulk;
@@ -1344,7 +1354,7 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
     x.screens = p->d_screens;
     x.skip_plane = p->nyq_plane;
     x.l2_max_clusters = (p->xy_clusters_c > 0 && p->xy_clusters_c < L2_MAX_CLUSTERS)
-                            ? p->xy_clusters_c : L2_MAX_CLUSTERS;
+                            ? p->xy_clusters_c : l2_group_cap(p->Y);
     {
       KScope k(p, kind);
       CKS(asg_launch_xy_l2_closing(x, p->st));
