@@ -518,147 +518,255 @@ __global__ void __launch_bounds__(128) k_conv_out(const bf16_t* __restrict__ X,
 // ---------------------------------------------------------------------------
 // Weight gradient of a 64 -> 64 layer:
 //   dW[o][i][j] += sum_pos D[pos][o] X[pos + j - 2][i]
-// GEMM with M = o (64), N = (j, i) (320, split in 4 slabs of 80 over
-// blockIdx.y), K = positions (64 per chunk).  Tiles are staged
-// channel-major so that A fragments pair consecutive positions.
+// GEMM with M = o (64), N = (j, i) (320), K = positions, all of M x N in one block of 8
+// warps (2 x 4 of 32 x 80 each), the positions split over persistent blocks in chunks of
+// 64.  The position-major tiles arrive by cp.async, double-buffered; ldmatrix.trans
+// turns them into fragments, a tap's shift being a row offset.  1 M positions: 1210 ->
+// @@ us (scalar loads and stores of a channel-major copy before; 256 MB of HBM reads
+// take 40 us).
 // ---------------------------------------------------------------------------
-constexpr int WG_SLAB = 80;
-constexpr int DT_S = TP + 8;       // stride of the staged D^T tile [64][TP]
-constexpr int XT_S = TP + 4 + 4;   // stride of the staged X^T tile [64][TP + 4]
-constexpr size_t WGRAD_SMEM = (size_t)(NCH * DT_S + NCH * XT_S) * sizeof(bf16_t);
+constexpr int WGX = TP + 4;  // staged rows of X: pos0 - 2 .. pos0 + TP + 1
+constexpr size_t WGRAD_SMEM = (size_t)2 * (TP + WGX) * XS * sizeof(bf16_t);
 
-__global__ void __launch_bounds__(128) k_conv64_wgrad(const bf16_t* __restrict__ D,
-                                                      const bf16_t* __restrict__ X,
-                                                      float* __restrict__ dW, int npos, int nT) {
-  extern __shared__ uint4 smem_u4[];
-  bf16_t* Dt = reinterpret_cast<bf16_t*>(smem_u4);
-  bf16_t* Xt = Dt + NCH * DT_S;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gid = lane >> 2, tig = lane & 3;
-  const int slab = blockIdx.y;      // n-range [slab*80, +80)
-  const int m0 = warp * 16;         // output channels of this warp
-  float acc[10][4];
-#pragma unroll
-  for (int n = 0; n < 10; ++n)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
-  const int nchunks = npos / TP;
-  for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {
-    const int pos0 = ch * TP;
-    const int cbeg = (pos0 / nT) * nT, cend = cbeg + nT;
-    __syncthreads();
-    for (int i = tid; i < TP * NCH; i += blockDim.x) {
-      const int p = i / NCH, o = i - p * NCH;
-      Dt[o * DT_S + p] = D[(size_t)(pos0 + p) * NCH + o];
-    }
-    for (int i = tid; i < (TP + 4) * NCH; i += blockDim.x) {
-      const int r = i / NCH, c = i - r * NCH;
-      const int pos = pos0 - 2 + r;
-      Xt[c * XT_S + r] = (pos >= cbeg && pos < cend) ? X[(size_t)pos * NCH + c] : (bf16_t)0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ks = 0; ks < TP / 16; ++ks) {
-      const int p0 = ks * 16;
-      const bf16_t* ar = Dt + (m0 + gid) * DT_S + p0 + tig * 2;
-      const unsigned a0 = *reinterpret_cast<const unsigned*>(ar);
-      const unsigned a1 = *reinterpret_cast<const unsigned*>(ar + 8 * DT_S);
-      const unsigned a2 = *reinterpret_cast<const unsigned*>(ar + 8);
-      const unsigned a3 = *reinterpret_cast<const unsigned*>(ar + 8 * DT_S + 8);
-#pragma unroll
-      for (int n = 0; n < 10; ++n) {
-        const int kk = slab * WG_SLAB + n * 8 + gid;  // column (j, i) of this lane's B values
-        const int j = kk / NCH, i = kk - j * NCH;
-        // B[k = position][n = (j, i)] = X[p + j - 2][i] = Xt[i][p + j]
-        const bf16_t* xr = Xt + i * XT_S + p0 + tig * 2 + j;
-        const unsigned b0 = (unsigned)xr[0] | ((unsigned)xr[1] << 16);
-        const unsigned b1 = (unsigned)xr[8] | ((unsigned)xr[9] << 16);
-        mma_bf16(acc[n], a0, a1, a2, a3, b0, b1);
-      }
-    }
-  }
-  // acc[n][q]: o = m0 + gid (+8 for q >= 2), k = slab*80 + n*8 + tig*2 (+1 for odd q)
-#pragma unroll
-  for (int n = 0; n < 10; ++n)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int o = m0 + gid + (q >= 2 ? 8 : 0);
-      const int kk = slab * WG_SLAB + n * 8 + tig * 2 + (q & 1);
-      const int j = kk / NCH, i = kk - j * NCH;
-      atomicAdd(dW + (size_t)o * KDIM + i * KT5 + j, acc[n][q]);
-    }
+__device__ __forceinline__ void ldsm_x4_t(unsigned (&r)[4], const void* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(src) : "memory");
 }
 
-// bias gradient: db[o] += sum_pos D[pos][o]
-__global__ void k_bias_grad(const bf16_t* __restrict__ D, float* __restrict__ db, int npos) {
-  __shared__ float part[256];
-  const int o = threadIdx.x & 63, lane4 = threadIdx.x >> 6;  // 4 position lanes x 64 channels
-  float s = 0.f;
-  for (int p = blockIdx.x * 4 + lane4; p < npos; p += gridDim.x * 4) s += bf2f(D[(size_t)p * NCH + o]);
-  part[threadIdx.x] = s;
+__global__ void __launch_bounds__(256, 2) k_conv64_wgrad(const bf16_t* __restrict__ D,
+                                                         const bf16_t* __restrict__ X,
+                                                         float* __restrict__ dW, int npos, int nT) {
+  extern __shared__ uint4 smem_u4[];
+  bf16_t* base = reinterpret_cast<bf16_t*>(smem_u4);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gid = lane >> 2, tig = lane & 3;
+  const int lm = lane >> 3, lr = lane & 7;  // ldmatrix: matrix and row this lane addresses
+  const int m0 = (warp >> 2) * 32, t0 = (warp & 3) * 10;  // output channels; 8-column tiles
+  float acc[2][10][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 10; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[m][n][q] = 0.f;
+  const int nchunks = npos / TP;
+  auto load = [&](int ch, int buf) {
+    bf16_t* Ds = base + buf * (TP + WGX) * XS;
+    bf16_t* Xs = Ds + TP * XS;
+    const int pos0 = ch * TP;
+    const int cbeg = (pos0 / nT) * nT, cend = cbeg + nT;
+    for (int i = tid; i < TP * 8; i += 256)
+      cp16(Ds + (i >> 3) * XS + (i & 7) * 8, D + (size_t)(pos0 + (i >> 3)) * NCH + (i & 7) * 8);
+    for (int i = tid; i < WGX * 8; i += 256) {
+      const int pos = pos0 - 2 + (i >> 3);
+      bf16_t* d = Xs + (i >> 3) * XS + (i & 7) * 8;
+      if (pos >= cbeg && pos < cend) cp16(d, X + (size_t)pos * NCH + (i & 7) * 8);
+      else *reinterpret_cast<uint4*>(d) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int buf = 0;
+  if ((int)blockIdx.x < nchunks) load(blockIdx.x, 0);
+  for (int ch = blockIdx.x; ch < nchunks; ch += gridDim.x, buf ^= 1) {
+    if (ch + (int)gridDim.x < nchunks) {
+      load(ch + gridDim.x, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const bf16_t* Ds = base + buf * (TP + WGX) * XS;
+    const bf16_t* Xs = Ds + TP * XS;
+#pragma unroll
+    for (int ks = 0; ks < TP / 16; ++ks) {
+      unsigned a[2][4];
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        ldsm_x4_t(a[m], Ds + (ks * 16 + (lm >> 1) * 8 + lr) * XS + m0 + m * 16 + (lm & 1) * 8);
+#pragma unroll
+      for (int n = 0; n < 10; n += 2) {
+        const int t = t0 + n;  // tiles t, t + 1: columns (j, i0 .. i0 + 15), t is even
+        unsigned b[4];
+        ldsm_x4_t(b, Xs + (ks * 16 + (t >> 3) + (lm & 1) * 8 + lr) * XS + (t & 7) * 8 +
+                         (lm >> 1) * 8);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          mma_bf16(acc[m][n], a[m][0], a[m][1], a[m][2], a[m][3], b[0], b[1]);
+          mma_bf16(acc[m][n + 1], a[m][0], a[m][1], a[m][2], a[m][3], b[2], b[3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // acc[m][n][q]: o = m0 + m*16 + gid (+8 for q >= 2), column tig*2 (+1 for odd q) of tile t0 + n
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 10; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = m0 + m * 16 + gid + (q >= 2 ? 8 : 0);
+        const int t = t0 + n, j = t >> 3, i = (t & 7) * 8 + tig * 2 + (q & 1);
+        atomicAdd(dW + (size_t)o * KDIM + i * KT5 + j, acc[m][n][q]);
+      }
+}
+
+// bias gradient: db[o] += sum_pos D[pos][o] (16-byte loads of 8 channels per thread)
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16_t* __restrict__ D,
+                                                   float* __restrict__ db, int npos) {
+  __shared__ float part[32][NCH];
+  const int c = threadIdx.x & 7, pl = threadIdx.x >> 3;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int p = blockIdx.x * 32 + pl; p < npos; p += gridDim.x * 32) {
+    const uint4 q = *reinterpret_cast<const uint4*>(D + (size_t)p * NCH + c * 8);
+    const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      s[2 * e] += bf2f((bf16_t)(w[e] & 0xffffu));
+      s[2 * e + 1] += bf2f((bf16_t)(w[e] >> 16));
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) part[pl][c * 8 + e] = s[e];
   __syncthreads();
-  if (threadIdx.x < 64) atomicAdd(db + o, part[o] + part[o + 64] + part[o + 128] + part[o + 192]);
+  if (threadIdx.x < NCH) {
+    float t = 0.f;
+    for (int k = 0; k < 32; ++k) t += part[k][threadIdx.x];
+    atomicAdd(db + threadIdx.x, t);
+  }
+}
+
+// sum of the mask (the loss is a mean over the masked samples)
+__global__ void __launch_bounds__(256) k_mask_sum(const float* __restrict__ mask,
+                                                  double* __restrict__ out, int npos) {
+  __shared__ double red[8];
+  double s = 0.0;
+#pragma unroll 4
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < npos; i += gridDim.x * 256) s += (double)mask[i];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[w];
+    atomicAdd(out, t);
+  }
 }
 
 // ---------------------------------------------------------------------------
 // first layer (1 -> 64) and its weight gradient, last layer (64 -> 1) with the
 // loss, and its backward: CUDA cores
 // ---------------------------------------------------------------------------
-__global__ void k_layer1_fwd(const float* __restrict__ x, const float* __restrict__ th,
-                             float* __restrict__ Z, bf16_t* __restrict__ H, int npos, int nT) {
-  const size_t n = (size_t)npos * NCH;
-  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n;
-       idx += (size_t)gridDim.x * blockDim.x) {
-    const int pos = (int)(idx / NCH), o = (int)(idx - (size_t)pos * NCH);
-    const int t = pos % nT;
-    float z = th[OFF_B1 + o];
+// In the 1-channel layers a warp walks runs of RUN consecutive positions of a column, lane
+// l holding channels 2l, 2l + 1 and a sliding window of the five neighbouring rows or
+// samples, so each row is read once.  1 M positions: first layer 274 -> @@ us, its
+// gradient 483 -> @@, backward of the last layer 1148 -> @@.
+constexpr int RUN = 64;  // divides nT (a multiple of 128)
+
+__device__ __forceinline__ float2 bf2x2(unsigned w) {
+  return make_float2(bf2f((bf16_t)(w & 0xffffu)), bf2f((bf16_t)(w >> 16)));
+}
+__device__ __forceinline__ unsigned f2bf2(float a, float b) {
+  return (unsigned)f2bf(a) | ((unsigned)f2bf(b) << 16);
+}
+
+__global__ void __launch_bounds__(256) k_layer1_fwd(const float* __restrict__ x,
+                                                    const float* __restrict__ th,
+                                                    float* __restrict__ Z, bf16_t* __restrict__ H,
+                                                    int npos, int nT) {
+  const int lane = threadIdx.x & 31, o = 2 * lane;
+  float wa[KT5], wb[KT5];
 #pragma unroll
-    for (int j = 0; j < KT5; ++j) {
-      const int tt = t + j - 2;
-      if (tt >= 0 && tt < nT) z = fmaf(th[OFF_W1 + o * KT5 + j], x[pos + j - 2], z);
+  for (int j = 0; j < KT5; ++j) {
+    wa[j] = th[OFF_W1 + o * KT5 + j];
+    wb[j] = th[OFF_W1 + (o + 1) * KT5 + j];
+  }
+  const float ba = th[OFF_B1 + o], bb = th[OFF_B1 + o + 1];
+  const int nrun = npos / RUN, nw = gridDim.x * 8;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrun; r += nw) {
+    const int p0 = r * RUN, t0 = p0 % nT;
+    // (a sample outside the column adds fmaf(w, 0, z) = z)
+    auto xs = [&](int k) { return (t0 + k >= 0 && t0 + k < nT) ? x[p0 + k] : 0.f; };
+    float w0 = xs(-2), w1 = xs(-1), w2 = xs(0), w3 = xs(1);
+#pragma unroll 8
+    for (int k = 0; k < RUN; ++k) {
+      const float w4 = xs(k + 2);
+      const float win[KT5] = {w0, w1, w2, w3, w4};
+      float za = ba, zb = bb;
+#pragma unroll
+      for (int j = 0; j < KT5; ++j) {
+        za = fmaf(wa[j], win[j], za);
+        zb = fmaf(wb[j], win[j], zb);
+      }
+      const size_t idx = (size_t)(p0 + k) * NCH + o;
+      if (Z) *reinterpret_cast<float2*>(Z + idx) = make_float2(za, zb);
+      *reinterpret_cast<unsigned*>(H + idx) = f2bf2(gelu_f(za), gelu_f(zb));
+      w0 = w1; w1 = w2; w2 = w3; w3 = w4;
     }
-    if (Z) Z[idx] = z;
-    H[idx] = f2bf(gelu_f(z));
   }
 }
 
 // y = b4 + sum_{j,i} W4[i][j] h3[pos + j - 2][i]; with a target: the masked
-// squared error goes to loss_acc[0] (sum) and dy = 2 (y - target) mask / nmask
-__global__ void k_layer4_fwd(const bf16_t* __restrict__ H3, const float* __restrict__ th,
-                             float* __restrict__ y, const float* __restrict__ target,
-                             const float* __restrict__ mask, float inv_nmask,
-                             float* __restrict__ dy, double* __restrict__ loss_acc, int npos,
-                             int nT) {
-  __shared__ float w4[NCH * KT5];
+// squared error goes to loss_acc[0] (sum) and dy = 2 (y - target) mask / nmask with the
+// mask's sum nmask in loss_acc[1]
+// A warp owns 32 consecutive positions: lane l adds the products of channels 2l, 2l + 1 of
+// each of the 36 rows to the five positions it serves, then the lanes' partial sums
+// are transposed and added in 31 shuffles, which leaves position l in lane l.
+__global__ void __launch_bounds__(256) k_layer4_fwd(
+    const bf16_t* __restrict__ H3, const float* __restrict__ th, float* __restrict__ y,
+    const float* __restrict__ target, const float* __restrict__ mask, float* __restrict__ dy,
+    double* __restrict__ loss_acc, int npos, int nT) {
   __shared__ double red[8];
-  for (int i = threadIdx.x; i < NCH * KT5; i += blockDim.x) w4[i] = th[OFF_W4 + i];
-  __syncthreads();
+  const int lane = threadIdx.x & 31, i0 = 2 * lane;
+  float wa[KT5], wb[KT5];
+#pragma unroll
+  for (int j = 0; j < KT5; ++j) {
+    wa[j] = th[OFF_W4 + i0 * KT5 + j];
+    wb[j] = th[OFF_W4 + (i0 + 1) * KT5 + j];
+  }
+  const float b4 = th[OFF_B4];
+  const double ms = target ? loss_acc[1] : 0.0;  // mask sum
+  const float inv_nmask = 1.f / (float)(ms > 0.0 ? ms : 1.0);
   double lsum = 0.0;
-  for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < npos; pos += gridDim.x * blockDim.x) {
-    const int t = pos % nT;
-    float v = th[OFF_B4];
+  const int nrun = npos / 32, nw = gridDim.x * 8;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrun; r += nw) {
+    const int p0 = r * 32, t0 = p0 % nT;
+    float v[32];
 #pragma unroll
-    for (int j = 0; j < KT5; ++j) {
-      const int tt = t + j - 2;
-      if (tt < 0 || tt >= nT) continue;
-      const uint4* hr = reinterpret_cast<const uint4*>(H3 + (size_t)(pos + j - 2) * NCH);
+    for (int k = 0; k < 32; ++k) v[k] = 0.f;
 #pragma unroll
-      for (int c = 0; c < NCH / 8; ++c) {
-        const uint4 q = hr[c];
-        const unsigned w[4] = {q.x, q.y, q.z, q.w};
+    for (int q = -2; q < 34; ++q) {
+      if (t0 + q < 0 || t0 + q >= nT) continue;
+      const float2 h = bf2x2(*reinterpret_cast<const unsigned*>(H3 + (size_t)(p0 + q) * NCH + i0));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = c * 8 + e * 2;
-          v = fmaf(w4[i * KT5 + j], bf2f((bf16_t)(w[e] & 0xffffu)), v);
-          v = fmaf(w4[(i + 1) * KT5 + j], bf2f((bf16_t)(w[e] >> 16)), v);
-        }
+      for (int j = 0; j < KT5; ++j) {
+        const int k = q + 2 - j;
+        if (k >= 0 && k < 32) v[k] = fmaf(wb[j], h.y, fmaf(wa[j], h.x, v[k]));
       }
     }
-    y[pos] = v;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+      const bool up = (lane & s) != 0;
+#pragma unroll
+      for (int i = 0; i < s; ++i) {
+        const float give = up ? v[i] : v[i + s], keep = up ? v[i + s] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+      }
+    }
+    const int pos = p0 + lane;
+    const float o = v[0] + b4;
+    y[pos] = o;
     if (target) {
-      const float r = (v - target[pos]) * mask[pos];
-      lsum += (double)r * (double)r;
-      dy[pos] = 2.f * r * inv_nmask;
+      const float e = (o - target[pos]) * mask[pos];
+      lsum += (double)e * (double)e;
+      dy[pos] = 2.f * e * inv_nmask;
     }
   }
   if (target) {
@@ -675,58 +783,111 @@ __global__ void k_layer4_fwd(const bf16_t* __restrict__ H3, const float* __restr
 
 // backward of the last layer: dz3[pos][i] = (sum_j W4[i][j] dy[pos - j + 2]) GELU'(z3),
 // dW4[i][j] += sum_pos dy[pos] h3[pos + j - 2][i], db4 += sum dy
-__global__ void k_layer4_bwd(const float* __restrict__ dy, const bf16_t* __restrict__ H3,
-                             const float* __restrict__ Z3, const float* __restrict__ th,
-                             bf16_t* __restrict__ DZ3, float* __restrict__ g, int npos, int nT) {
+__global__ void __launch_bounds__(256) k_layer4_bwd(const float* __restrict__ dy,
+                                                    const bf16_t* __restrict__ H3,
+                                                    const float* __restrict__ Z3,
+                                                    const float* __restrict__ th,
+                                                    bf16_t* __restrict__ DZ3,
+                                                    float* __restrict__ g, int npos, int nT) {
   __shared__ float gw[NCH * KT5];
   __shared__ float gb;
   for (int i = threadIdx.x; i < NCH * KT5; i += blockDim.x) gw[i] = 0.f;
   if (threadIdx.x == 0) gb = 0.f;
   __syncthreads();
-  const int i = threadIdx.x & 63, pl = threadIdx.x >> 6, npl = blockDim.x >> 6;
-  float accw[KT5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  float accb = 0.f;
-  for (int pos = blockIdx.x * npl + pl; pos < npos; pos += gridDim.x * npl) {
-    const int t = pos % nT;
-    float d = 0.f;
+  const int lane = threadIdx.x & 31, i0 = 2 * lane;
+  float wa[KT5], wb[KT5], ga[KT5], gc[KT5], accb = 0.f;
 #pragma unroll
-    for (int j = 0; j < KT5; ++j) {
-      const int tt = t - j + 2;
-      if (tt >= 0 && tt < nT) d = fmaf(th[OFF_W4 + i * KT5 + j], dy[pos - j + 2], d);
-      const int ts = t + j - 2;
-      if (ts >= 0 && ts < nT) accw[j] = fmaf(dy[pos], bf2f(H3[(size_t)(pos + j - 2) * NCH + i]), accw[j]);
+  for (int j = 0; j < KT5; ++j) {
+    wa[j] = th[OFF_W4 + i0 * KT5 + j];
+    wb[j] = th[OFF_W4 + (i0 + 1) * KT5 + j];
+    ga[j] = gc[j] = 0.f;
+  }
+  const int nrun = npos / RUN, nw = gridDim.x * 8;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrun; r += nw) {
+    const int p0 = r * RUN, t0 = p0 % nT;
+    auto in = [&](int k) { return t0 + k >= 0 && t0 + k < nT; };
+    auto hs = [&](int k) {
+      return in(k) ? bf2x2(*reinterpret_cast<const unsigned*>(H3 + (size_t)(p0 + k) * NCH + i0))
+                   : make_float2(0.f, 0.f);
+    };
+    auto ds = [&](int k) { return in(k) ? dy[p0 + k] : 0.f; };
+    float2 h0 = hs(-2), h1 = hs(-1), h2 = hs(0), h3 = hs(1);
+    float d0 = ds(-2), d1 = ds(-1), d2 = ds(0), d3 = ds(1);
+#pragma unroll 8
+    for (int k = 0; k < RUN; ++k) {
+      const float2 h4 = hs(k + 2);
+      const float d4 = ds(k + 2);
+      const size_t idx = (size_t)(p0 + k) * NCH + i0;
+      const float2 z = *reinterpret_cast<const float2*>(Z3 + idx);
+      const float2 hw[KT5] = {h0, h1, h2, h3, h4};
+      const float dw[KT5] = {d4, d3, d2, d1, d0};  // dy[pos - j + 2]
+      float a = 0.f, b = 0.f;
+#pragma unroll
+      for (int j = 0; j < KT5; ++j) {
+        a = fmaf(wa[j], dw[j], a);
+        b = fmaf(wb[j], dw[j], b);
+        ga[j] = fmaf(d2, hw[j].x, ga[j]);
+        gc[j] = fmaf(d2, hw[j].y, gc[j]);
+      }
+      *reinterpret_cast<unsigned*>(DZ3 + idx) = f2bf2(a * gelu_grad_f(z.x), b * gelu_grad_f(z.y));
+      if (lane == 0) accb += d2;
+      h0 = h1; h1 = h2; h2 = h3; h3 = h4;
+      d0 = d1; d1 = d2; d2 = d3; d3 = d4;
     }
-    const size_t idx = (size_t)pos * NCH + i;
-    DZ3[idx] = f2bf(d * gelu_grad_f(Z3[idx]));
-    if (i == 0) accb += dy[pos];
   }
 #pragma unroll
-  for (int j = 0; j < KT5; ++j) atomicAdd(&gw[i * KT5 + j], accw[j]);
-  if (i == 0) atomicAdd(&gb, accb);
+  for (int j = 0; j < KT5; ++j) {
+    atomicAdd(&gw[i0 * KT5 + j], ga[j]);
+    atomicAdd(&gw[(i0 + 1) * KT5 + j], gc[j]);
+  }
+  if (lane == 0) atomicAdd(&gb, accb);
   __syncthreads();
   for (int k = threadIdx.x; k < NCH * KT5; k += blockDim.x) atomicAdd(g + OFF_W4 + k, gw[k]);
   if (threadIdx.x == 0) atomicAdd(g + OFF_B4, gb);
 }
 
 // first-layer weight gradient: dW1[o][j] += sum_pos dz1[pos][o] x[pos + j - 2]; db1[o]
-__global__ void k_layer1_bwd(const bf16_t* __restrict__ DZ1, const float* __restrict__ x,
-                             float* __restrict__ g, int npos, int nT) {
-  const int o = threadIdx.x & 63, pl = threadIdx.x >> 6, npl = blockDim.x >> 6;
-  float accw[KT5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-  float accb = 0.f;
-  for (int pos = blockIdx.x * npl + pl; pos < npos; pos += gridDim.x * npl) {
-    const int t = pos % nT;
-    const float d = bf2f(DZ1[(size_t)pos * NCH + o]);
-    accb += d;
+__global__ void __launch_bounds__(256) k_layer1_bwd(const bf16_t* __restrict__ DZ1,
+                                                    const float* __restrict__ x,
+                                                    float* __restrict__ g, int npos, int nT) {
+  __shared__ float gw[NCH * (KT5 + 1)];
+  for (int i = threadIdx.x; i < NCH * (KT5 + 1); i += blockDim.x) gw[i] = 0.f;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, o = 2 * lane;
+  float ga[KT5 + 1], gc[KT5 + 1];
 #pragma unroll
-    for (int j = 0; j < KT5; ++j) {
-      const int tt = t + j - 2;
-      if (tt >= 0 && tt < nT) accw[j] = fmaf(d, x[pos + j - 2], accw[j]);
+  for (int j = 0; j <= KT5; ++j) ga[j] = gc[j] = 0.f;
+  const int nrun = npos / RUN, nw = gridDim.x * 8;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrun; r += nw) {
+    const int p0 = r * RUN, t0 = p0 % nT;
+    auto xs = [&](int k) { return (t0 + k >= 0 && t0 + k < nT) ? x[p0 + k] : 0.f; };
+    float w0 = xs(-2), w1 = xs(-1), w2 = xs(0), w3 = xs(1);
+#pragma unroll 8
+    for (int k = 0; k < RUN; ++k) {
+      const float w4 = xs(k + 2);
+      const float win[KT5] = {w0, w1, w2, w3, w4};
+      const float2 d =
+          bf2x2(*reinterpret_cast<const unsigned*>(DZ1 + (size_t)(p0 + k) * NCH + o));
+#pragma unroll
+      for (int j = 0; j < KT5; ++j) {
+        ga[j] = fmaf(d.x, win[j], ga[j]);
+        gc[j] = fmaf(d.y, win[j], gc[j]);
+      }
+      ga[KT5] += d.x;
+      gc[KT5] += d.y;
+      w0 = w1; w1 = w2; w2 = w3; w3 = w4;
     }
   }
 #pragma unroll
-  for (int j = 0; j < KT5; ++j) atomicAdd(g + OFF_W1 + o * KT5 + j, accw[j]);
-  atomicAdd(g + OFF_B1 + o, accb);
+  for (int j = 0; j <= KT5; ++j) {
+    atomicAdd(&gw[o * (KT5 + 1) + j], ga[j]);
+    atomicAdd(&gw[(o + 1) * (KT5 + 1) + j], gc[j]);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < NCH * (KT5 + 1); k += blockDim.x) {
+    const int c = k / (KT5 + 1), j = k - c * (KT5 + 1);
+    atomicAdd(g + (j < KT5 ? OFF_W1 + c * KT5 + j : OFF_B1 + c), gw[k]);
+  }
 }
 
 // theta -> BF16 GEMM operands: Wg[o][j*64+i] = W[o][i][j],
@@ -888,8 +1049,7 @@ static int conv_smem_attr() {
 
 // forward of the whole network: x [npos] -> y [npos] (z's kept when keep_z)
 static int net_forward(asg_net* n, const float* x, float* y, const float* target,
-                       const float* mask, float inv_nmask, int npos, int nT, bool keep_z,
-                       cudaStream_t st) {
+                       const float* mask, int npos, int nT, bool keep_z, cudaStream_t st) {
   CKS_NET(conv_smem_attr());
   const int tiles = npos / TPC;
   const int gconv = tiles < 2 * n->nsm ? tiles : 2 * n->nsm;
@@ -898,28 +1058,29 @@ static int net_forward(asg_net* n, const float* x, float* y, const float* target
                                              keep_z ? n->z2 : nullptr, n->h2, npos, nT);
   k_conv64<0><<<gconv, 128, CONV_SMEM, st>>>(n->h2, n->wg3, n->theta + OFF_B3, nullptr,
                                              keep_z ? n->z3 : nullptr, n->h3, npos, nT);
-  k_layer4_fwd<<<4 * n->nsm, 256, 0, st>>>(n->h3, n->theta, y, target, mask, inv_nmask, n->dy,
-                                           n->loss, npos, nT);
+  k_layer4_fwd<<<4 * n->nsm, 256, 0, st>>>(n->h3, n->theta, y, target, mask, n->dy, n->loss, npos,
+                                           nT);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : net_fail(ASG_ERR_CUDA, "forward launch");
 }
 
 static int net_backward(asg_net* n, const float* x, int npos, int nT, cudaStream_t st) {
   const int tiles = npos / TPC;
   const int gconv = tiles < 2 * n->nsm ? tiles : 2 * n->nsm;
-  const int chunks = npos / TP;
-  const int gw = chunks < n->nsm ? chunks : n->nsm;
+  const int chunks = npos / TP, runs = (npos / RUN + 7) / 8;
+  const int gw = chunks < 2 * n->nsm ? chunks : 2 * n->nsm;
+  const int gr = runs < 4 * n->nsm ? runs : 4 * n->nsm;
   // last layer: dW4, db4, dz3 -> d2
-  k_layer4_bwd<<<2 * n->nsm, 256, 0, st>>>(n->dy, n->h3, n->z3, n->theta, n->d2, n->grad, npos, nT);
+  k_layer4_bwd<<<gr, 256, 0, st>>>(n->dy, n->h3, n->z3, n->theta, n->d2, n->grad, npos, nT);
   // layer 3: dW3 (dz3, h2), db3, dz2 = (W3^T * dz3) GELU'(z2) -> d1
-  k_conv64_wgrad<<<dim3(gw, KDIM / WG_SLAB), 128, WGRAD_SMEM, st>>>(n->d2, n->h2, n->grad + OFF_W3, npos, nT);
+  k_conv64_wgrad<<<gw, 256, WGRAD_SMEM, st>>>(n->d2, n->h2, n->grad + OFF_W3, npos, nT);
   k_bias_grad<<<2 * n->nsm, 256, 0, st>>>(n->d2, n->grad + OFF_B3, npos);
   k_conv64<1><<<gconv, 128, CONV_SMEM, st>>>(n->d2, n->wt3, nullptr, n->z2, nullptr, n->d1, npos, nT);
   // layer 2: dW2 (dz2, h1), db2, dz1 = (W2^T * dz2) GELU'(z1) -> d2
-  k_conv64_wgrad<<<dim3(gw, KDIM / WG_SLAB), 128, WGRAD_SMEM, st>>>(n->d1, n->h1, n->grad + OFF_W2, npos, nT);
+  k_conv64_wgrad<<<gw, 256, WGRAD_SMEM, st>>>(n->d1, n->h1, n->grad + OFF_W2, npos, nT);
   k_bias_grad<<<2 * n->nsm, 256, 0, st>>>(n->d1, n->grad + OFF_B2, npos);
   k_conv64<1><<<gconv, 128, CONV_SMEM, st>>>(n->d1, n->wt2, nullptr, n->z1, nullptr, n->d2, npos, nT);
   // layer 1
-  k_layer1_bwd<<<2 * n->nsm, 256, 0, st>>>(n->d2, x, n->grad, npos, nT);
+  k_layer1_bwd<<<gr, 256, 0, st>>>(n->d2, x, n->grad, npos, nT);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : net_fail(ASG_ERR_CUDA, "backward launch");
 }
 
@@ -970,7 +1131,7 @@ extern "C" int asg_net_create(asg_net** out) {
             cudaMalloc(&n->wc2, NCH * KDIM * 2) == cudaSuccess &&
             cudaMalloc(&n->wc3, NCH * KDIM * 2) == cudaSuccess &&
             cudaMalloc(&n->tc_err, sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&n->loss, sizeof(double)) == cudaSuccess;
+            cudaMalloc(&n->loss, 2 * sizeof(double)) == cudaSuccess;  // loss sum, mask sum
   if (!ok) {
     asg_net_destroy(n);
     return net_fail(ASG_ERR_NOMEM, "corrector parameters: cudaMalloc failed");
@@ -1044,21 +1205,16 @@ extern "C" int asg_net_train_step(asg_net* n, const float* d_x, const float* d_t
   const size_t npos = (size_t)ncols * nT;
   CKS_NET(net_ensure(n, npos));
   cudaStream_t st = 0;
-  // the loss is a mean over the masked samples: their count, on the host
-  std::vector<float> hm(npos);
-  if (cudaMemcpy(hm.data(), d_mask, npos * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-    return net_fail(ASG_ERR_CUDA, "mask download");
-  double ms = 0.0;
-  for (float v : hm) ms += v;
-  const float nmask = (float)(ms > 0.0 ? ms : 1.0);
   cudaMemsetAsync(n->grad, 0, NPARAM * 4, st);
-  cudaMemsetAsync(n->loss, 0, sizeof(double), st);
-  CKS_NET(net_forward(n, d_x, n->yb, d_target, d_mask, 1.f / nmask, (int)npos, nT, true, st));
+  cudaMemsetAsync(n->loss, 0, 2 * sizeof(double), st);
+  // the loss is a mean over the masked samples
+  k_mask_sum<<<n->nsm, 256, 0, st>>>(d_mask, n->loss + 1, (int)npos);
+  CKS_NET(net_forward(n, d_x, n->yb, d_target, d_mask, (int)npos, nT, true, st));
   CKS_NET(net_backward(n, d_x, (int)npos, nT, st));
-  double l = 0.0;
-  if (cudaMemcpy(&l, n->loss, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
+  double l[2] = {0.0, 0.0};
+  if (cudaMemcpy(l, n->loss, sizeof(l), cudaMemcpyDeviceToHost) != cudaSuccess)
     return net_fail(ASG_ERR_CUDA, "loss download");
-  if (loss_out) *loss_out = l / nmask;
+  if (loss_out) *loss_out = l[0] / (float)(l[1] > 0.0 ? l[1] : 1.0);
   if (h_grad && cudaMemcpy(h_grad, n->grad, NPARAM * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
     return net_fail(ASG_ERR_CUDA, "gradient download");
   if (lr > 0.f) {
