@@ -1943,10 +1943,9 @@ extern "C" int asg_kernel_stats(asg_plan* p, double* ms, long* launches, int nki
 // ---------------------------------------------------------------------------
 extern "C" int asg_get_tuning(asg_plan* p, asg_tuning* out) {
   if (!p || !out) return fail(ASG_ERR_ARG, "null argument");
-  const int flux = p->cfg.flux != 0;
   for (int i = 0; i < 3; ++i) {
     int c = p->t_cols[i];
-    if (c == 0) c = p->tfast ? asg_t_default_cols(p->T, p->Y, i == 0 ? flux : 0) : 4;
+    if (c == 0) c = p->tfast ? asg_t_default_cols(p->T, p->X, p->Y, i) : 4;
     (&out->t_cols_flux)[i] = c;
   }
   int ncl = p->xy_clusters > 0 ? p->xy_clusters : L2_MAX_CLUSTERS;
@@ -2017,7 +2016,7 @@ extern "C" int asg_autotune(asg_plan* p, const float* field, double dz, int step
       if (i == 1 && (!p->cfg.split_step || p->no_taper)) continue;  // no taper-only pass
       double best = 1e300;
       int best_c = 0;
-      for (int c : {8, 16}) {
+      for (int c : {8, 16, 32}) {
         if (!asg_t_cols_supported(p->T, p->Y, i == 0, c)) continue;
         p->t_cols[i] = c;
         double ms = 0.0;

@@ -57,13 +57,13 @@ struct TParams {
   const float2* twM;     // W_M^k,  k < M (fast kernels)
   const unsigned* status;
   int pdl;               // programmatic dependent launch
-  int cols_per_block;    // fast kernels: 8 or 16 columns per block, 0 = default
+  int cols_per_block;    // fast kernels: 8, 16 or 32 columns per block, 0 = default
   int prefetch;          // fast kernels: 1 = each block prefetches into L2 the spectrum of the
                          // tile that starts about one block lifetime later (set by the launcher)
   int prefetch_ahead;    // that distance in blocks (the launcher: resident blocks of the GPU)
 };
 
-int asg_t_default_cols(int nT, int Y, int flux);
+int asg_t_default_cols(int nT, int X, int Y, int slot);
 bool asg_t_cols_supported(int nT, int Y, int flux, int cols);
 
 bool asg_t_fast_supported(int nT);

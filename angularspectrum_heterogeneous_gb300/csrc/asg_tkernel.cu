@@ -19,7 +19,7 @@ ASG_DEFINE_ROOT_UPLOADER(asg_roots_upload_t)
 
 // ---------------------------------------------------------------------------
 // fast kernel: nT = 2M, M = N1*N2 (register-resident four-step FFT).
-// A block of 8 warps handles C columns (C = 8 or 16): CY = C/2 consecutive y
+// A block of 8 warps handles C columns (C = 8, 16 or 32): CY = C/2 consecutive y
 // at row x and the same CY y at row x+X/2.  That pairing lets the kernel
 // apply the first radix-2 stage of the x transform on the way out
 // (split_out: planes hold a = (s(x) + s(x+X/2))/2 and
@@ -33,13 +33,13 @@ ASG_DEFINE_ROOT_UPLOADER(asg_roots_upload_t)
 // ---------------------------------------------------------------------------
 enum TMode : int { TM_PLAIN = 0, TM_FLUX = 1, TM_STATS = 2 };
 
-// Register budget: 3 blocks per SM with 16 columns or from 512 samples up
-// (shared memory allows no more) and 4 otherwise, in every mode (the streamed
+// Register budget: 3 blocks per SM with 16 columns of more than 256 samples or from
+// 1024 samples up (shared memory allows no more) and 4 otherwise, in every mode (the streamed
 // KT step keeps about 25 values live).
 template <class PL, int MODE, int C>
-__global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
+__global__ void __launch_bounds__(256, ((PL::N >= 512 || (C >= 16 && PL::N > 128)) ? 3 : 4))
     tk_fast(TParams p) {
-  static_assert(C == 8 || C == 16, "8 or 16 columns per block");
+  static_assert(C == 8 || C == 16 || C == 32, "8, 16 or 32 columns per block");
   constexpr int CPW = C / 8;   // columns per warp
   constexpr int CY = C / 2;    // consecutive y per row
   constexpr int M = PL::N;
@@ -77,11 +77,12 @@ __global__ void __launch_bounds__(256, ((PL::N >= 512 || C == 16) ? 3 : 4))
     if (nt < (int)gridDim.x) {
       const int xq2 = nt / (Y / CY), y02 = CY * (nt - xq2 * (Y / CY));
       const size_t cA = (size_t)xq2 * Y + y02, cB = cA + (size_t)X2 * Y;
-      // M + 1 planes, rows x and x + X/2: runs of CY complex (32 or 64 bytes)
+      // M + 1 planes, rows x and x + X/2: runs of CY complex (32 to 128 bytes)
       for (int i = tid; i < 2 * (M + 1); i += nthr) {
         const float2* a = p.spec + (size_t)(i >> 1) * ncols + ((i & 1) ? cB : cA);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a));
-        if (CY == 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(a + 4));
+#pragma unroll
+        for (int k = 4; k < CY; k += 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(a + k));
       }
     }
   }
@@ -336,33 +337,52 @@ static int launch_fast_t_mode(const TParams& p, cudaStream_t st) {
   return asg_launch_pdl(p.pdl != 0, tk_fast<PL, MODE, C>, dim3(grid), dim3(256), smem, st, q);
 }
 
-// 16 columns per block exist up to 1024-sample columns (three blocks of 256
-// threads still fit an SM in the transform-only and statistics modes, two in
-// the flux mode).
+// 16 columns per block exist up to 1024-sample columns (three blocks of 256 threads still
+// fit an SM), 32 up to 256 samples: four columns per warp fill its lanes in the steps
+// of 8 tasks per column (nT = 128 and 256) and the runs in HBM are 128 bytes.
 bool asg_t_cols_supported(int nT, int Y, int flux, int cols) {
   (void)flux;
   if (cols == 8) return Y % 4 == 0;
   if (cols == 16) return nT <= 1024 && Y % 8 == 0;
+  if (cols == 32) return nT <= 256 && Y % 16 == 0;
   return false;
 }
 
-int asg_t_default_cols(int nT, int Y, int flux) {
-  return asg_t_cols_supported(nT, Y, flux, 16) ? 16 : 8;
+// slot: 0 Burgers step, 1 taper only, 2 statistics.  32 columns per block once they make
+// enough blocks: 256 x 256 x 256 plain 70 -> 53 us, KT 109 -> 90, statistics 87 -> 74; at
+// 128 x 128 x 256 (512 blocks) 22 -> 18, 31 -> 31 (Rusanov 37 -> 39) and 28 -> 26.  nT = 128:
+// plain 16.1 -> 14.4 us at 128 x 128, KT 42 -> 39 from 192 x 192, statistics 0-3 % slower.
+// nT = 192, whose steps have 12 and 8 tasks: only the plain pass of large grids (256 x 256:
+// 55 -> 51 us).
+int asg_t_default_cols(int nT, int X, int Y, int slot) {
+  if (asg_t_cols_supported(nT, Y, slot == 0, 32)) {
+    const int none = 1 << 30;
+    const int from = slot == 0   ? (nT == 192 ? none : 1152)
+                     : slot == 1 ? (nT == 192 ? 2048 : 512)
+                                 : (nT == 256 ? 512 : none);
+    if (X * Y / 32 >= from) return 32;
+  }
+  return asg_t_cols_supported(nT, Y, slot == 0, 16) ? 16 : 8;
 }
 
 template <int M>
 static int launch_fast_t(const TParams& p, cudaStream_t st) {
   const bool flux = p.op.flux != FLUX_NONE && !p.stats;
-  int c = p.cols_per_block ? p.cols_per_block : asg_t_default_cols(2 * M, p.Y, flux);
+  int c = p.cols_per_block
+              ? p.cols_per_block
+              : asg_t_default_cols(2 * M, p.X, p.Y, p.stats ? 2 : flux ? 0 : 1);
   if (!asg_t_cols_supported(2 * M, p.Y, flux, c)) return ASG_ERR_SHAPE;
   if (p.stats)
-    return c == 16 ? launch_fast_t_mode<M, TM_STATS, (M <= 512 ? 16 : 8)>(p, st)
-                   : launch_fast_t_mode<M, TM_STATS, 8>(p, st);
+    return c == 32   ? launch_fast_t_mode<M, TM_STATS, (M <= 128 ? 32 : 8)>(p, st)
+           : c == 16 ? launch_fast_t_mode<M, TM_STATS, (M <= 512 ? 16 : 8)>(p, st)
+                     : launch_fast_t_mode<M, TM_STATS, 8>(p, st);
   if (flux)
-    return c == 16 ? launch_fast_t_mode<M, TM_FLUX, (M <= 512 ? 16 : 8)>(p, st)
-                   : launch_fast_t_mode<M, TM_FLUX, 8>(p, st);
-  return c == 16 ? launch_fast_t_mode<M, TM_PLAIN, (M <= 512 ? 16 : 8)>(p, st)
-                 : launch_fast_t_mode<M, TM_PLAIN, 8>(p, st);
+    return c == 32   ? launch_fast_t_mode<M, TM_FLUX, (M <= 128 ? 32 : 8)>(p, st)
+           : c == 16 ? launch_fast_t_mode<M, TM_FLUX, (M <= 512 ? 16 : 8)>(p, st)
+                     : launch_fast_t_mode<M, TM_FLUX, 8>(p, st);
+  return c == 32   ? launch_fast_t_mode<M, TM_PLAIN, (M <= 128 ? 32 : 8)>(p, st)
+         : c == 16 ? launch_fast_t_mode<M, TM_PLAIN, (M <= 512 ? 16 : 8)>(p, st)
+                   : launch_fast_t_mode<M, TM_PLAIN, 8>(p, st);
 }
 
 bool asg_t_fast_supported(int nT) {

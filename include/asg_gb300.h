@@ -195,7 +195,7 @@ int asg_batch_last_run_ms(asg_batch* batch, double* ms);
 /* Launch shapes of a plan (no counterpart in the reference: its XLA program
  * has no tunable launch shapes). 0 in a field selects the built-in default. */
 typedef struct {
-  int t_cols_flux;   /* columns per block of the column pass with the Burgers step: 8, 16 */
+  int t_cols_flux;   /* columns per block of the column pass with the Burgers step: 8, 16, 32 (nT <= 256) */
   int t_cols_plain;  /* columns per block of the taper-only column pass: 8, 16 */
   int t_cols_stats;  /* columns per block of the column pass closing a step: 8, 16 */
   int xy_clusters;   /* cap on resident CTA groups (clusters) of the L2-exchange plane kernel: 0..64 */
