@@ -30,13 +30,13 @@
 #include "asg_common.cuh"
 
 // Block of a kernel variant whose largest radix is BIG: threads at most, blocks per SM (so
-// 128, 168 or 255 registers, what the register DFTs need without spills).  Small
-// blocks: their load, exchange and barrier phases overlap each other's (224-thread
-// blocks, two per SM: 257 x 257 x 601 rows 20 % slower).
+// 96, 128 or 255 registers; a few values spill in the largest).  Small blocks: their
+// load, exchange and barrier phases overlap each other's (224-thread blocks, two per
+// SM: 257 x 257 x 601 rows 20 % slower; one block less per SM: 200 x 180 x 400 10 %).
 template <int BIG>
 struct LineBlock {
   static constexpr int NT = 128;
-  static constexpr int MB = BIG <= 24 ? 4 : BIG <= 48 ? 3 : 2;
+  static constexpr int MB = BIG <= 24 ? 5 : BIG <= 48 ? 4 : 2;
 };
 // Device tables of one axis (built in FP64 on the host, see line_axis()).
 struct LineAxis {

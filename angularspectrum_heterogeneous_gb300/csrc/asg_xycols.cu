@@ -11,11 +11,17 @@ namespace {
 // ---------------------------------------------------------------------------
 // x transforms.  A block takes C = 2^lc y-columns of one plane; lanes run along the columns, then along the sublines.
 // ---------------------------------------------------------------------------
+// threads of a block at most and blocks per SM (so 112 or 168 registers up to radix 24: a
+// chirp variant holds both convolutions' code): eight columns' tasks in one round there
+// (two rounds of 96 threads: 257 x 257 x 601 610 us against 555)
 template <class PL>
-__global__ void __launch_bounds__(LineBlock<PL::BIG>::NT,
-                                  !PL::DIRECT && PL::BIG > 16 && PL::BIG <= 24
-                                      ? 3  // both convolutions' code: 168 registers
-                                      : LineBlock<PL::BIG>::MB)
+struct ColBlock {
+  static constexpr int NT = PL::BIG <= 24 ? 192 : LineBlock<PL::BIG>::NT;
+  static constexpr int MB = PL::BIG > 24 ? LineBlock<PL::BIG>::MB : PL::DIRECT || PL::BIG <= 16 ? 3 : 2;
+};
+
+template <class PL>
+__global__ void __launch_bounds__(ColBlock<PL>::NT, ColBlock<PL>::MB)
     xy_cols(XYParams p, LineAxis ax, float2* buf, int lc, int LS) {
   pdl_wait();
   if (xy_should_skip(p)) return;
@@ -203,7 +209,7 @@ int launch_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaStream_t
   const int s = line_smem_attr(xy_cols<PL>, &done[asg_device_slot()]);
   if (s != ASG_OK) return s;
   return asg_launch_pdl(p.pdl != 0, xy_cols<PL>, dim3((p.Y + C - 1) / C, p.nplanes),
-                        dim3(line_threads(C * tasks, LineBlock<PL::BIG>::NT)), smem, st, p, ax, buf,
+                        dim3(line_threads(C * tasks, ColBlock<PL>::NT)), smem, st, p, ax, buf,
                         lc, LS);
 }
 
