@@ -383,8 +383,9 @@ struct asg_plan {
   int t_cols[3] = {0, 0, 0};  // columns per block: flux, taper-only, statistics column passes
   int xy_clusters = 0;        // resident-cluster cap of the L2 plane kernel (0 = all)
   int xy_clusters_c = 0;      // the same for the closing-stage kernel
-  int xy_bulk = 1;            // HBM row loads of the L2 plane kernels (XYParams::bulk_rows);
-                              // set from default_bulk() at plan creation
+  int xy_bulk = 0;            // HBM row loads of the L2 plane kernels (XYParams::bulk_rows): by
+                              // default 16-byte cp.async, 1-5 % faster than bulk copies at every
+                              // plane size (128 x 128 x 1024 101 and 107 us per stage)
   int t_prefetch = 0;         // column passes: L2 prefetch of a later tile (TParams::prefetch)
   int xy_rows = 0;            // rows per diffraction CTA in a cooperative launch (asg_tuning
                               // xy_rows: 0 default, 1 sixteen, 2 eight)
@@ -465,12 +466,6 @@ struct asg_plan {
   std::vector<cudaEvent_t> ev_pool;
   std::vector<int> ev_kind;  // kind of event pair i (events 2i, 2i+1)
 };
-
-// Default HBM row loads of the plane kernels: 16-byte cp.async where the
-// diffraction kernel runs 8-row CTAs in a cooperative launch (from 256-wide
-// planes: 1-4 % faster than bulk copies there), bulk copies in the diffraction
-// kernel otherwise.
-static int default_bulk(const asg_plan* p) { return (p->l2 && p->Y >= 256) ? 0 : 1; }
 
 // launch accounting around one kernel launch of `kind`
 struct KScope {
@@ -594,7 +589,6 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   p->tfast = asg_t_fast_supported(T) && X % 2 == 0 && Y % 4 == 0;
   int Gs = 0, Gl = 0;
   p->l2 = p->tfast && asg_xy_l2_supported(X, Y, 2, &Gl);
-  p->xy_bulk = default_bulk(p);
   // planes much longer along x than along y leave a cluster's CTAs little work between
   // their exchanges of all x: 256 x 128 x 256 107 us per stage against 80 us for the row
   // and column passes, 512 x 128 x 256 280 against 184 (384 x 256: 254 and 250)
@@ -1982,7 +1976,7 @@ extern "C" int asg_set_tuning(asg_plan* p, const asg_tuning* t) {
   p->xy_clusters = t->xy_clusters;
   p->xy_clusters_c = t->xy_clusters_closing;
   p->xy_sync = t->xy_sync;
-  p->xy_bulk = t->xy_bulk == 0 ? default_bulk(p) : t->xy_bulk - 1;
+  p->xy_bulk = t->xy_bulk == 0 ? 0 : t->xy_bulk - 1;
   p->xy_rows = t->xy_rows;
   p->t_prefetch = t->t_prefetch == 0 ? 0 : t->t_prefetch - 1;
   p->gen++;
