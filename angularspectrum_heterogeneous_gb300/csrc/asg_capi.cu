@@ -434,6 +434,8 @@ struct asg_plan {
         *abl_t_full = nullptr;
   bool have_ops = false;
   bool no_taper = false;  // every taper factor is 1
+  // rows [0] to [1] and columns [2] to [3] that the damping factors, the edge weights leave
+  int fw_inside[4] = {0, 0, 0, 0}, sa_inside[4] = {0, 0, 0, 0};
   // epilogue data
   float *fw_lx = nullptr, *fw_ly = nullptr, *fw_exp = nullptr;
   float *sa_wx = nullptr, *sa_wy = nullptr, *sa_coef = nullptr;
@@ -843,6 +845,17 @@ static int build_tables(asg_plan* p, Slot& s, float2* out_pa, float2* out_p, flo
   return asg_launch_table(tp, p->st);
 }
 
+// [lo, hi): where all v are 0, if that is one range (else empty)
+static void untouched_range(int n, const float* v, int* range) {
+  int lo = 0, hi = n;
+  while (lo < n && v[lo] != 0.f) ++lo;
+  while (hi > lo && v[hi - 1] != 0.f) --hi;
+  for (int i = lo; i < hi; ++i)
+    if (v[i] != 0.f) hi = lo;
+  range[0] = lo;
+  range[1] = hi;
+}
+
 extern "C" int asg_set_step_operators(asg_plan* p, int slot, const asg_step_operators* o) {
   g_err.clear();
   if (!p || !o || slot < 0 || slot > 1) return fail(ASG_ERR_ARG, "bad argument");
@@ -932,6 +945,8 @@ extern "C" int asg_set_step_operators(asg_plan* p, int slot, const asg_step_oper
     CKS(h2d(p->fw_lx, lx.data(), X, p->st));
     CKS(h2d(p->fw_ly, ly.data(), Y, p->st));
     CKS(h2d(p->fw_exp, fe.data(), F, p->st));
+    untouched_range(X, lx.data(), &p->fw_inside[0]);
+    untouched_range(Y, ly.data(), &p->fw_inside[2]);
   }
   if (o->sa_wx && o->sa_wy) {
     std::vector<float> wx(X), wy(Y);
@@ -939,6 +954,8 @@ extern "C" int asg_set_step_operators(asg_plan* p, int slot, const asg_step_oper
     for (int y = 0; y < Y; ++y) wy[y] = (float)o->sa_wy[y];
     CKS(h2d(p->sa_wx, wx.data(), X, p->st));
     CKS(h2d(p->sa_wy, wy.data(), Y, p->st));
+    untouched_range(X, wx.data(), &p->sa_inside[0]);
+    untouched_range(Y, wy.data(), &p->sa_inside[2]);
   }
   if (p->cfg.nonlinear_obliquity && !p->obl_tab) {
     CKS(dalloc(&p->obl_tab, ntab));
@@ -1103,6 +1120,24 @@ static int xy_sync_of(const asg_plan* p) {
   if (p->batch_refs > 0) return 1;
   if (p->xy_sync != 0) return p->xy_sync;
   return (p->G >= 12 || p->Y >= 256) ? 3 : 1;
+}
+
+// boundary extras `epi` of a stage and what lies inside their bands
+static void set_epilogue(const asg_plan* p, XYParams* x, int epi) {
+  int in[4] = {0, p->X, 0, p->Y};
+  auto meet = [&](const int* r) {
+    for (int k = 0; k < 4; k += 2) {
+      in[k] = std::max(in[k], r[k]);
+      in[k + 1] = std::max(in[k], std::min(in[k + 1], r[k + 1]));
+    }
+  };
+  if (epi & EPI_FREQW) meet(p->fw_inside);
+  if (epi & EPI_SUPERABS) meet(p->sa_inside);
+  x->epi = epi;
+  x->ex0 = in[0];
+  x->ex1 = in[1];
+  x->ey0 = in[2];
+  x->ey1 = in[3];
 }
 
 static XYParams xyparams(asg_plan* p, const float2* table, bool zero_dc_nyq) {
@@ -1330,7 +1365,7 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
     x.stab_thr = p->cfg.stability_threshold;
   }
   if (!p->split) {
-    x.epi = epi;
+    set_epilogue(p, &x, epi);
     x.nscreens = nscr;
     x.screens = p->d_screens;
     if (p->lines) x.skip_plane = p->nyq_plane;
@@ -1343,7 +1378,7 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
     // both half-planes of a plane in one cluster, epilogue fused, whole planes
     // out in place; the Nyquist plane (Re() before the boundary corrections)
     // goes through the epilogue pass on its own
-    x.epi = epi;
+    set_epilogue(p, &x, epi);
     x.nscreens = nscr;
     x.screens = p->d_screens;
     x.skip_plane = p->nyq_plane;

@@ -171,16 +171,16 @@ __global__ void __launch_bounds__(ColBlock<PL>::NT, ColBlock<PL>::MB)
           if (l != 0.f) r = cscale(r, exp2f(e * l));
         }
         if (sa) line[b + S2 * a] = r;  // this task's own slots
-        else g[(size_t)x * Y + c] = r;
+        if (!sa || (x >= p.ex0 && x < p.ex1)) g[(size_t)x * Y + c] = r;
       }
     }
   });
   if (!sa) return;
   __syncthreads();
-  // Engquist-Majda x edges on the damped values
+  // Engquist-Majda x edges on the damped values of the bands
   const float cf = p.sa_coef[plane], st = p.sa_strength;
-  for (int i = tid; i < X * C; i += NT) {
-    const int c = i & (C - 1), x = i >> lc;
+  for (int i = tid; i < (p.ex0 + X - p.ex1) * C; i += NT) {
+    const int c = i & (C - 1), k = i >> lc, x = k < p.ex0 ? k : k - p.ex0 + p.ex1;
     if (c >= nc) continue;
     const float2* line = lines + c * LS;
     float2 r = line[line_pos<PL>(ax, x)];

@@ -47,6 +47,9 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
   const int total = p.nplanes * X;
   const int g0 = blockIdx.x * L, nr = min(L, total - g0);
   const bool epi = INV && (p.epi != 0 || p.nscreens > 0);
+  // columns that the epilogue leaves as they are go straight out (all are staged: the
+  // bands' edges need their neighbours)
+  const int ey0 = p.nscreens > 0 ? Y : p.ey0, ey1 = p.nscreens > 0 ? Y : p.ey1;
   auto zero_row = [&](int l) {
     return p.zero_dc_nyq && is_dc_or_nyq(p.f_of_plane[(g0 + l) / X], p.nT);
   };
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
         if constexpr (!DIRECT) r = chirp_mul(r, ax.ch + y, INV);
         if (zero) r = make_float2(0.f, 0.f);
         if (epi) line[b + S2 * a] = r;  // this task's own slots
-        else row[y] = r;
+        if (!epi || (y >= ey0 && y < ey1)) row[y] = r;
       }
     }
   });
@@ -157,8 +160,10 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
       const float g = fw ? p.fw_ly[j] : 0.f;  // 0 inside the boundary bands: factor 1
       return g != 0.f ? cscale(v, exp2f(e * g)) : v;
     };
+    const int nb = ey0 + Y - ey1;
 #pragma unroll 2
-    for (int y = tid & 31; y < Y; y += 32) {
+    for (int k = tid & 31; k < nb; k += 32) {
+      const int y = k < ey0 ? k : k - ey0 + ey1;
       float2 r;
       if (row_epi) {
         r = damped(y);
@@ -166,8 +171,8 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
         if (w != 0.f)
           r = edge_correct(y > 0 ? damped(y - 1) : r, r, y + 1 < Y ? damped(y + 1) : r, y, Y, w,
                            cf, p.sa_strength, p.sa_inv2dy, p.sa_invdy);
-        for (int k = 0; k < p.nscreens; ++k) {
-          const ScreenDev sc = p.screens[k];
+        for (int q = 0; q < p.nscreens; ++q) {
+          const ScreenDev sc = p.screens[q];
           const size_t g = (size_t)x * Y + y;
           float sn, cs;
           sincosf(sc.phase[g] * fs, &sn, &cs);
