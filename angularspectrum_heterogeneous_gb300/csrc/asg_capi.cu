@@ -838,6 +838,11 @@ static int build_tables(asg_plan* p, Slot& s, float2* out_pa, float2* out_p, flo
   tp.clip_negative = s.att_clip;
   // the plane kernels transform X/nsub-row (sub-)planes
   tp.norm = 1.0 / ((double)(p->X / p->nsub) * (double)p->Y);
+  // exact moduli and spread roundings for the line passes: 79 x 43 x 93, 16 Strang steps,
+  // field 1.3e-6 too large without, 2e-7 with.  The other plane kernels' transforms shrink
+  // the field a little more than FP32 moduli make it grow (128 x 128 x 384 error 5.1e-6 so,
+  // 5.3e-6 with exact moduli) and keep them.
+  tp.spread = p->lines ? 1 : 0;
   tp.out_pa = out_pa;
   tp.out_p = out_p;
   tp.out_a = out_a;

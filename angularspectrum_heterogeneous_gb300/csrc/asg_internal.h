@@ -189,6 +189,7 @@ struct TableParams {
   double kstart, kmax_t;   // cosine k-filter band
   int use_prop, use_att, obliquity, clip_negative;
   double norm;             // 1/(X*Y) folded in
+  int spread;              // entries' moduli to FP64 and their roundings spread over the modes
   float2* out_pa;          // propagator x attenuation (or null)
   float2* out_p;           // propagator alone (or null)
   float2* out_a;           // attenuation alone (or null)

@@ -31,6 +31,25 @@ __device__ __forceinline__ void sincos_reduced(double ph, float* s, float* c) {
   sincosf((float)r, s, c);
 }
 
+// The same with modulus 1 to FP64 (one Newton step for 1/sqrt near 1): FP32 sin and cos give
+// the small phases of low modes moduli above 1 more often than below, and each step repeats
+// it.
+ASG_DEV void sincos_unit(double a, bool unit, double* s, double* c) {
+  float sf, cf;
+  sincos_reduced(a, &sf, &cf);
+  const double sd = sf, cd = cf, m = unit ? 1.5 - 0.5 * fma(sd, sd, cd * cd) : 1.0;
+  *s = sd * m;
+  *c = cd * m;
+}
+
+// v as one float: nearest, or (spread, in [-1/2, 1/2)) nearest to v + spread ulp
+ASG_DEV float round_spread(double v, float spread) {
+  const float f = (float)v;
+  if (spread == 0.f) return f;
+  const float a = fabsf(f);
+  return (float)(v + (double)spread * (double)(nextafterf(a, INFINITY) - a));
+}
+
 // All multiplier tables of one step size in one pass: per mode the propagator
 // factor P and the attenuation/KK factor A are formed once and written as
 // out_pa = P A, out_p = P, out_a = A, out_sq = (P A)^2 (any output may be null).  The phases,
@@ -74,12 +93,12 @@ __global__ void k_build_table(TableParams p) {
             amp = (double)expf((float)(-p.dz_prop * sqrt(kk - k * k)));
             ph = p.dz_prop * k;
           }
-          float sn, cs;
-          sincos_reduced(ph, &sn, &cs);
+          double sn, cs;
+          sincos_unit(ph, p.spread != 0, &sn, &cs);
           // the reference's factor 2 on the kept bins is cancelled by the real
           // part it takes afterwards (Re(ifftn) = ifftn of (W(k)+conj W(-k))/2)
-          pr = mask * amp * (double)cs;
-          pi = mask * amp * (double)sn;
+          pr = mask * amp * cs;
+          pi = mask * amp * sn;
         } else {
           pr = 0.0;
           pi = 0.0;
@@ -103,11 +122,13 @@ __global__ void k_build_table(TableParams p) {
           }
         }
         if (prop) {
-          const double mag = (double)expf((float)(br * obl));
-          float sn, cs;
-          sincos_reduced(bi * obl, &sn, &cs);
-          ar = mag * (double)cs;
-          ai = mag * (double)sn;
+          // near 1, 1 + expm1: expf alone rounds a whole plane's factor alike
+          const float x = (float)(br * obl);
+          const double mag = p.spread != 0 && x > -0.25f ? 1.0 + (double)expm1f(x) : (double)expf(x);
+          double sn, cs;
+          sincos_unit(bi * obl, p.spread != 0, &sn, &cs);
+          ar = mag * cs;
+          ai = mag * sn;
         }
       }
       if (p.clip_negative && ar < 0.0) {
@@ -116,14 +137,23 @@ __global__ void k_build_table(TableParams p) {
       }
     }
     const double nrm = p.norm;
-    if (p.out_sq != nullptr) {
-      const double zr = pr * ar - pi * ai, zi = pr * ai + pi * ar;
-      p.out_sq[i] = make_float2((float)((zr * zr - zi * zi) * nrm), (float)(2.0 * zr * zi * nrm));
+    // a low-discrepancy sequence over the modes: the rounding errors of neighbouring entries
+    // cancel (attenuation is one factor per plane, and every plane holds the norm)
+    float d0 = 0.f, d1 = 0.f;
+    if (p.spread != 0) {
+      const unsigned h = cx * 3242174889u + cy * 2447445414u + pl * 1640531527u;
+      d0 = (float)(int)h * 2.3283064e-10f;
+      d1 = (float)(int)(h * 2654435769u) * 2.3283064e-10f;
     }
-    if (p.out_pa != nullptr)
-      p.out_pa[i] = make_float2((float)((pr * ar - pi * ai) * nrm), (float)((pr * ai + pi * ar) * nrm));
-    if (p.out_p != nullptr) p.out_p[i] = make_float2((float)(pr * nrm), (float)(pi * nrm));
-    if (p.out_a != nullptr) p.out_a[i] = make_float2((float)(ar * nrm), (float)(ai * nrm));
+    auto put = [&](float2* out, double re, double im) {
+      if (out != nullptr)
+        out[i] = make_float2(round_spread(re * nrm, d0), round_spread(im * nrm, d1));
+    };
+    const double zr = pr * ar - pi * ai, zi = pr * ai + pi * ar;
+    put(p.out_sq, zr * zr - zi * zi, 2.0 * zr * zi);
+    put(p.out_pa, zr, zi);
+    put(p.out_p, pr, pi);
+    put(p.out_a, ar, ai);
   }
 }
 
