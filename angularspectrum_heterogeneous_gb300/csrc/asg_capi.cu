@@ -2358,22 +2358,16 @@ extern "C" int asg_flux_columns(const float* in, float* out, int ncols, int nT, 
 // to its own pool, a real-time loop in which cudaMalloc/cudaFree (which
 // synchronise the device) are not allowed, or code that queues work on a
 // stream it must not stall. They call this entry point instead. Besides its
-// input and output the column kernel touches three small global areas: a
-// status word it reads first (it must be zero, or the kernel returns without
-// work), the sub-cycle cap counters it adds to, and a twiddle area it copies
-// into shared memory (unused here, since the columns go in and out as real
-// samples with no transform). All live in the fixed array below.
+// input and output the column kernel touches two small global areas: a status
+// word it reads first (it must be zero, or the kernel returns without work) and
+// the sub-cycle cap counters it adds to. Both live in the fixed struct below.
 // ---------------------------------------------------------------------------
-static constexpr int FLUX_SCRATCH_MAX_NT = 2048;  // longest column of the kernel
-
 struct FluxScratch {
   unsigned status;        // must read zero when the kernel starts
   unsigned clamp[2];      // columns capped at max_subcycles, largest count needed
-  unsigned pad[61];       // keeps the twiddle area on its own 256-byte line
-  float2 tw[FLUX_SCRATCH_MAX_NT];
-};  // 16,640 bytes in all
+};
 
-static __device__ __align__(256) FluxScratch g_flux_scratch;
+static __device__ FluxScratch g_flux_scratch;
 
 // Device address of the scratch in the current context.  Looked up on every
 // call (cudaGetSymbolAddress allocates nothing): an address kept from an
@@ -2393,9 +2387,8 @@ extern "C" int asg_flux_columns_device(const float* d_in, float* d_out, int ncol
                                        void* stream) {
   g_err.clear();
   if (!d_in || !d_out || ncols <= 0 || nT < 3) return fail(ASG_ERR_ARG, "bad argument");
-  if (nT > FLUX_SCRATCH_MAX_NT)
-    return fail(ASG_ERR_SHAPE, "nT=%d exceeds the %d samples the fixed scratch holds", nT,
-                FLUX_SCRATCH_MAX_NT);
+  if (nT > ASG_T_MAX)
+    return fail(ASG_ERR_SHAPE, "nT=%d exceeds the %d samples a column may have", nT, ASG_T_MAX);
   if (flux < ASG_FLUX_RUSANOV || flux > ASG_FLUX_KT_MINMOD)
     return fail(ASG_ERR_ARG, "unknown flux %d", flux);
   {
@@ -2425,7 +2418,6 @@ extern "C" int asg_flux_columns_device(const float* d_in, float* d_out, int ncol
   t.real_in = const_cast<float*>(d_in);
   t.write_real = 1;
   t.real_out = d_out;
-  t.tw = scr->tw;
   t.status = &scr->status;
   t.op.flux = flux;
   t.op.dz = (float)dz;

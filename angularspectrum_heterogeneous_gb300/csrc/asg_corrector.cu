@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(128) k_conv_out(const bf16_t* __restrict__ X,
 // warps (2 x 4 of 32 x 80 each), the positions split over persistent blocks in chunks of
 // 64.  The position-major tiles arrive by cp.async, double-buffered; ldmatrix.trans
 // turns them into fragments, a tap's shift being a row offset.  1 M positions: 1210 ->
-// @@ us (scalar loads and stores of a channel-major copy before; 256 MB of HBM reads
+// 166 us (scalar loads and stores of a channel-major copy before; 256 MB of HBM reads
 // take 40 us).
 // ---------------------------------------------------------------------------
 constexpr int WGX = TP + 4;  // staged rows of X: pos0 - 2 .. pos0 + TP + 1
@@ -666,8 +666,8 @@ __global__ void __launch_bounds__(256) k_mask_sum(const float* __restrict__ mask
 // ---------------------------------------------------------------------------
 // In the 1-channel layers a warp walks runs of RUN consecutive positions of a column, lane
 // l holding channels 2l, 2l + 1 and a sliding window of the five neighbouring rows or
-// samples, so each row is read once.  1 M positions: first layer 274 -> @@ us, its
-// gradient 483 -> @@, backward of the last layer 1148 -> @@.
+// samples, so each row is read once.  1 M positions: first layer 274 -> 68 us, its
+// gradient 483 -> 98, backward of the last layer 1148 -> 167.
 constexpr int RUN = 64;  // divides nT (a multiple of 128)
 
 __device__ __forceinline__ float2 bf2x2(unsigned w) {

@@ -10,8 +10,8 @@
 // register DFTs and their exchanges through shared memory.  Per pass, against
 // mixed-radix Stockham lines with direct sums over the prime factors:
 // 257 x 257 x 601 27-30 -> 0.9 ms (its HBM traffic alone: 0.05 ms),
-// 51 x 51 x 401 620-640 -> 38-45 us, 200 x 180 x 400 780-930 -> 100-175 us,
-// 81 x 81 x 101 100 -> 23-29 us, 5 x 5 x 1001 120 -> 46 us.
+// 51 x 51 x 401 620-640 -> 40-47 us, 200 x 180 x 400 780-930 -> 90-160 us,
+// 81 x 81 x 101 100 -> 23-31 us, 5 x 5 x 1001 120 -> 46 us.
 //
 // Also here: the Burgers step alone on real columns (no transforms).
 //

@@ -258,8 +258,8 @@ int asg_flux_columns(const float* in, float* out, int ncols, int nT, int flux, d
  * device memory (memory owned by their own pool, loops where a synchronising
  * cudaMalloc/cudaFree is not allowed).
  * It allocates nothing: its scratch (a status word and the sub-cycle cap
- * counters, which it clears on `stream` before each launch, and a twiddle area)
- * is a fixed 16,640-byte array in the library. Its device address is looked up
+ * counters, which it clears on `stream` before each launch) is a fixed struct
+ * in the library. Its device address is looked up
  * on every call; the first call on a device also loads the library's kernels
  * there, so make that first call before any stream capture. nT above 2048 is
  * rejected with ASG_ERR_SHAPE; an error left pending by earlier CUDA work is

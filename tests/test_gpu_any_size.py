@@ -31,6 +31,28 @@ def test_planes_of_any_size(n):
     P.test_step_operators(None, (6, n, 8))
 
 
+@pytest.mark.parametrize("factor", [0.01, 0.2, 0.34, 0.5])
+@pytest.mark.parametrize("shape", [(31, 44, 12), (45, 23, 9)])
+def test_boundary_bands_of_any_width(shape, factor):
+    """The closing epilogue visits the bands only: bands of one sample, bands with a few
+    samples between them, bands that meet (same FP32 transforms and tolerance as the step
+    operators)."""
+    from angularspectrum_heterogeneous_gb300 import Plan
+    nX, nY, nT = shape
+    kw, u = P._op_case(shape)
+    kw["boundaryFactor"] = factor
+    p = P.oracle_params(kw)
+    plan = Plan(shape, P.solver_params(kw))
+    plan.set_operators(0, 1e-4)
+    u64 = u.astype(np.float64)
+    fw = O.freq_weighted_mask(nX, nY, nT, p.dT, p.f0, factor, "wendland").astype(np.float64)
+    wx, wy = (O.boundary_weights(n, O.band_width(n, factor)).astype(np.float64) for n in (nX, nY))
+    assert rel(plan.apply_operator(5, u), O.freq_weighted_step(u64, fw)) < 2e-6
+    assert rel(plan.apply_operator(6, u), O.super_absorbing_step(
+        u64, wx, wy, p.dX, p.dY, p.dT, p.c0, 0.8)) < 2e-6
+    plan.close()
+
+
 @pytest.mark.parametrize("nT", [4, 5, 31, 33, 64, 127, 129, 640, 1000, 1025, 2048])
 @pytest.mark.parametrize("flux", ["kt", "ktmm"])
 def test_kt_runs_of_any_length(nT, flux):
