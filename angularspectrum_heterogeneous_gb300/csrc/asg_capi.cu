@@ -352,6 +352,7 @@ struct Slot {
   float2* tabC = nullptr;  // Strang: A(1/2)          | Lie: A(1)
   float2* tabM = nullptr;  // the whole step of a linear medium without boundary taper:
                            // Strang: (H(dz/2) A(1/2))^2 | Lie: H(dz) A(1)
+  bool whole = false;      // tabM holds this dz's table (a call with a taper leaves it as it was)
   // 1-D vectors kept for single-operator application
   double* kt_prop = nullptr;
   double* km_att = nullptr;
@@ -916,6 +917,7 @@ extern "C" int asg_set_step_operators(asg_plan* p, int slot, const asg_step_oper
   for (int t = 0; t < T; ++t) p->no_taper = p->no_taper && o->abl_t[t] == 1.0;
   if (p->no_taper && p->N == 0.0 && !s.tabM) CKS(dalloc(&s.tabM, ntab));
   float2* whole = p->no_taper && p->N == 0.0 ? s.tabM : nullptr;
+  s.whole = whole != nullptr;
   if (p->cfg.split_step) {
     // A = atten(dz/2) diff(dz/2), B = diff(dz/2), C = atten(dz/2)
     CKS(build_tables(p, s, s.tabA, s.tabB, s.tabC, dz / 2, dz * 0.5, whole));
@@ -1432,7 +1434,7 @@ static int march_step(asg_plan* p, const Slot& s, double dzs, double btvd, int n
   const float* at = strang ? p->abl_t_half : p->abl_t_full;
   const int epi = (p->cfg.freq_weighted ? EPI_FREQW : 0) | (p->cfg.super_absorbing ? EPI_SUPERABS : 0);
   const bool linear = p->no_taper && p->N == 0.0;
-  const bool whole = linear && s.tabM != nullptr && !(p->l2 && (epi != 0 || nscr > 0));
+  const bool whole = linear && s.whole && !(p->l2 && (epi != 0 || nscr > 0));
   TParams t = tparams(p);
   if (whole) {
     CKS(closing_stage(p, s.tabM, epi, nscr, ASG_K_XY_C, t, true, dzs));
