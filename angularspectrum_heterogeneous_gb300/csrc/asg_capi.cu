@@ -15,6 +15,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <complex>
 #include <mutex>
 #include <string>
@@ -1417,6 +1418,14 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
   return ASG_OK;
 }
 
+// whether a step runs as one spectral stage (see march_step)
+static bool whole_step(const asg_plan* p, const Slot& s, int epi, int nscr) {
+  return p->no_taper && p->N == 0.0 && s.whole && !(p->l2 && (epi != 0 || nscr > 0));
+}
+static int step_epilogue(const asg_plan* p) {
+  return (p->cfg.freq_weighted ? EPI_FREQW : 0) | (p->cfg.super_absorbing ? EPI_SUPERABS : 0);
+}
+
 // One march step.  Two spectral stages with nothing between them but a return
 // to real space run as one, with the product of their multipliers (each column
 // and plane pass left out is one read and one write of the spectrum):
@@ -1432,11 +1441,10 @@ static int march_step(asg_plan* p, const Slot& s, double dzs, double btvd, int n
   const bool strang = p->cfg.split_step != 0;
   const float* axy = strang ? p->abl_xy_half : p->abl_xy_full;
   const float* at = strang ? p->abl_t_half : p->abl_t_full;
-  const int epi = (p->cfg.freq_weighted ? EPI_FREQW : 0) | (p->cfg.super_absorbing ? EPI_SUPERABS : 0);
+  const int epi = step_epilogue(p);
   const bool linear = p->no_taper && p->N == 0.0;
-  const bool whole = linear && s.whole && !(p->l2 && (epi != 0 || nscr > 0));
   TParams t = tparams(p);
-  if (whole) {
+  if (whole_step(p, s, epi, nscr)) {
     CKS(closing_stage(p, s.tabM, epi, nscr, ASG_K_XY_C, t, true, dzs));
   } else {
     // stage A (+ stability test)
@@ -2026,7 +2034,8 @@ extern "C" int asg_set_tuning(asg_plan* p, const asg_tuning* t) {
 }
 
 // Times each candidate of each knob on `steps` march steps from `field` and
-// keeps the fastest (per-kind device time of the passes the knob drives).
+// keeps the fastest (per-kind device time of the passes the knob drives).  A knob whose
+// passes the march does not launch keeps its value.
 extern "C" int asg_autotune(asg_plan* p, const float* field, double dz, int steps,
                             asg_tuning* chosen) {
   g_err.clear();
@@ -2036,139 +2045,57 @@ extern "C" int asg_autotune(asg_plan* p, const float* field, double dz, int step
   p->prof = true;
   // the plain diffraction pass: B in the Strang march, A in the Lie march or
   // without taper; a whole step in one stage has the closing pass only
-  const int diff_kind = p->no_taper && p->N == 0.0 ? ASG_K_XY_C
+  const int diff_kind = whole_step(p, p->slot[0], step_epilogue(p), 0) ? ASG_K_XY_C
                         : p->cfg.split_step && !p->no_taper ? ASG_K_XY_B : ASG_K_XY_A;
-  auto trial = [&](int kind, double* ms) -> int {
-    int n = 0;
-    int s = asg_run(p, field, steps * dz, dz, nullptr, nullptr, &n);
-    if (s != ASG_OK) return s;
-    *ms = p->launches[kind] > 0 ? p->kms[kind] / p->launches[kind] : 0.0;
-    return ASG_OK;
-  };
   int status = ASG_OK;
+  auto tune = [&](int* knob, const std::vector<int>& candidates, const std::vector<int>& kinds) {
+    double best = 1e300;
+    int best_v = *knob;
+    for (int v : candidates) {
+      if (status != ASG_OK) break;
+      *knob = v;
+      int n = 0;
+      status = asg_run(p, field, steps * dz, dz, nullptr, nullptr, &n);
+      if (status != ASG_OK) break;
+      double ms = 0.0;  // one launch of each kind together
+      bool ran = false;
+      for (int k : kinds)
+        if (p->launches[k] > 0) {
+          ms += p->kms[k] / p->launches[k];
+          ran = true;
+        }
+      if (!ran) break;
+      if (ms < best) {
+        best = ms;
+        best_v = v;
+      }
+    }
+    *knob = best_v;
+  };
   if (p->tfast) {
     const int kinds[3] = {ASG_K_T_NONLIN, ASG_K_T_MID, ASG_K_T_END};
-    for (int i = 0; i < 3 && status == ASG_OK; ++i) {
-      if (i == 1 && (!p->cfg.split_step || p->no_taper)) continue;  // no taper-only pass
-      double best = 1e300;
-      int best_c = 0;
-      for (int c : {8, 16, 32}) {
-        if (!asg_t_cols_supported(p->T, p->Y, i == 0, c)) continue;
-        p->t_cols[i] = c;
-        double ms = 0.0;
-        status = trial(kinds[i], &ms);
-        if (status != ASG_OK) break;
-        if (ms < best) {
-          best = ms;
-          best_c = c;
-        }
-      }
-      p->t_cols[i] = best_c;
+    for (int i = 0; i < 3; ++i) {
+      std::vector<int> cols;
+      for (int c : {8, 16, 32})
+        if (asg_t_cols_supported(p->T, p->Y, i == 0, c)) cols.push_back(c);
+      tune(&p->t_cols[i], cols, {kinds[i]});
     }
     // L2 prefetch of later tiles: the three column passes together
-    double best = 1e300;
-    int best_f = 0;
-    for (int f : {0, 1}) {
-      if (status != ASG_OK) break;
-      p->t_prefetch = f;
-      double ms = 0.0;
-      status = trial(ASG_K_T_NONLIN, &ms);
-      if (status != ASG_OK) break;
-      for (int k : {ASG_K_T_MID, ASG_K_T_END})
-        if (p->launches[k] > 0) ms += p->kms[k] / p->launches[k];
-      if (ms < best) {
-        best = ms;
-        best_f = f;
-      }
-    }
-    p->t_prefetch = best_f;
+    tune(&p->t_prefetch, {0, 1}, {ASG_K_T_NONLIN, ASG_K_T_MID, ASG_K_T_END});
   }
-  if (p->l2 && status == ASG_OK && p->batch_refs == 0) {
+  if (p->l2) {
+    // the closing-stage kernel runs when the step has a boundary epilogue
+    const bool closing = step_epilogue(p) != 0;
+    std::vector<int> planes = {diff_kind};
+    if (closing) planes.push_back(ASG_K_XY_C);
     // group barrier: the plain diffraction pass and the closing pass together
-    const bool closing = p->cfg.freq_weighted || p->cfg.super_absorbing;
-    double best = 1e300;
-    int best_s = 0;
-    for (int sy : {1, 2, 3}) {
-      p->xy_sync = sy;
-      double ms = 0.0, ms_c = 0.0;
-      status = trial(diff_kind, &ms);
-      if (status != ASG_OK) break;
-      if (closing) {
-        ms_c = p->launches[ASG_K_XY_C] > 0 ? p->kms[ASG_K_XY_C] / p->launches[ASG_K_XY_C] : 0.0;
-      }
-      if (ms + ms_c < best) {
-        best = ms + ms_c;
-        best_s = sy;
-      }
-    }
-    p->xy_sync = best_s;
-  }
-  if (p->l2 && p->Y >= 256 && xy_sync_of(p) >= 2 && status == ASG_OK) {
+    if (p->batch_refs == 0) tune(&p->xy_sync, {1, 2, 3}, planes);
     // tile shape of the cooperative diffraction kernel: 16-row or 8-row CTAs
-    double best = 1e300;
-    int best_r = 2;
-    for (int r : {1, 2}) {
-      p->xy_rows = r;
-      double ms = 0.0;
-      status = trial(diff_kind, &ms);
-      if (status != ASG_OK) break;
-      if (ms < best) {
-        best = ms;
-        best_r = r;
-      }
-    }
-    p->xy_rows = best_r;
-  }
-  if (p->l2 && status == ASG_OK) {
-    double best = 1e300;
-    int best_n = 0;
-    for (int n : {0, 16, 12, 8}) {
-      p->xy_clusters = n;
-      double ms = 0.0;
-      status = trial(diff_kind, &ms);
-      if (status != ASG_OK) break;
-      if (ms < best) {
-        best = ms;
-        best_n = n;
-      }
-    }
-    p->xy_clusters = best_n;
-  }
-  if (p->l2 && status == ASG_OK) {
-    // HBM row loads of the plane kernels: cp.async, or bulk copies in the
-    // diffraction kernel, or in both (diffraction and closing passes together)
-    const bool closing = p->cfg.freq_weighted || p->cfg.super_absorbing;
-    double best = 1e300;
-    int best_b = 1;
-    for (int b : {0, 1, 2}) {
-      p->xy_bulk = b;
-      double ms = 0.0, ms_c = 0.0;
-      status = trial(diff_kind, &ms);
-      if (status != ASG_OK) break;
-      if (closing)
-        ms_c = p->launches[ASG_K_XY_C] > 0 ? p->kms[ASG_K_XY_C] / p->launches[ASG_K_XY_C] : 0.0;
-      if (ms + ms_c < best) {
-        best = ms + ms_c;
-        best_b = b;
-      }
-    }
-    p->xy_bulk = best_b;
-  }
-  // the closing-stage kernel runs when the step has a boundary epilogue
-  if (p->l2 && (p->cfg.freq_weighted || p->cfg.super_absorbing) && status == ASG_OK) {
-    double best = 1e300;
-    int best_n = 0;
-    for (int n : {0, 16, 12, 8}) {
-      p->xy_clusters_c = n;
-      double ms = 0.0;
-      status = trial(ASG_K_XY_C, &ms);
-      if (status != ASG_OK) break;
-      if (ms < best) {
-        best = ms;
-        best_n = n;
-      }
-    }
-    p->xy_clusters_c = best_n;
+    if (p->Y >= 256 && xy_sync_of(p) >= 2) tune(&p->xy_rows, {1, 2}, {diff_kind});
+    tune(&p->xy_clusters, {0, 16, 12, 8}, {diff_kind});
+    // HBM row loads: cp.async, or bulk copies in the diffraction kernel, or in both
+    tune(&p->xy_bulk, {0, 1, 2}, planes);
+    if (closing) tune(&p->xy_clusters_c, {0, 16, 12, 8}, {ASG_K_XY_C});
   }
   p->prof = prof;
   p->gen++;
