@@ -232,7 +232,8 @@ __global__ void __launch_bounds__(LineBlock<PL::BIG>::NT, LineBlock<PL::BIG>::MB
 }
 
 // The Burgers step alone on real columns: a warp per column, the column in
-// shared memory.
+// shared memory (CH < 0: the KT sub-steps in registers, see column_phase).
+template <int CH>
 __global__ void __launch_bounds__(256) k_flux_columns(TParams p) {
   if (*p.status != 0) return;
   extern __shared__ float smcol[];
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(256) k_flux_columns(TParams p) {
 #pragma unroll 4
   for (int t = lane; t < nT; t += 32) col.set(t, src[t]);
   __syncwarp();
-  column_phase<0>(col, c, nT, p.op, false);
+  column_phase<CH>(col, c, nT, p.op, false);
   float* dst = p.real_out + (size_t)c * nT;
 #pragma unroll 4
   for (int t = lane; t < nT; t += 32) dst[t] = col.get(t);
@@ -296,11 +297,22 @@ int asg_launch_t_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
   return ASG_ERR_SHAPE;
 }
 
-int asg_launch_flux_columns(const TParams& p, cudaStream_t st) {
+template <int CH>
+static int launch_flux(const TParams& p, cudaStream_t st) {
+  if (CH < 0 && p.nT > -32 * CH) {
+    if constexpr (CH < 0) return launch_flux<(CH > -8 ? CH - 1 : 0)>(p, st);
+  }
   // 8 columns per block while they fit the default 48 KB
   int warps = 8;
   while (warps > 1 && (size_t)warps * p.nT * sizeof(float) > 48 * 1024) warps /= 2;
-  k_flux_columns<<<(p.ncols + warps - 1) / warps, 32 * warps,
-                   (size_t)warps * p.nT * sizeof(float), st>>>(p);
+  k_flux_columns<CH><<<(p.ncols + warps - 1) / warps, 32 * warps,
+                       (size_t)warps * p.nT * sizeof(float), st>>>(p);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+}
+int asg_launch_flux_columns(const TParams& p, cudaStream_t st) {
+  // KT columns up to 256 samples in registers (8 samples per lane; beyond, the registers of a
+  // run leave too few warps per SM); Rusanov steps have none to keep (10000 x 224 12.7 us,
+  // 14.5 in that variant)
+  return p.op.flux == FLUX_KT_MC || p.op.flux == FLUX_KT_MINMOD ? launch_flux<-1>(p, st)
+                                                                : launch_flux<0>(p, st);
 }
