@@ -1265,14 +1265,29 @@ struct GateParams {
   unsigned* clamp;    // [2] fallback columns capped at max_sub, largest count needed
 };
 
+// A column of nT = 32 CH samples as 32 runs of CH (kt_step_stream), each run a float4 array.
+// Runs start an odd number of float4s apart, so the lanes' 16-byte accesses meet no bank twice.
+template <int CH>
+struct RunColumn {
+  static constexpr int PAD = CH % 8 == 0 ? 4 : 0, FLOATS = 32 * (CH + PAD);
+  float* base;
+  ASG_DEV int idx(int t) const { return t + PAD * (t / CH); }
+  ASG_DEV float get(int t) const { return base[idx(t)]; }
+  ASG_DEV void set(int t, float v) const { base[idx(t)] = v; }
+  template <int C>
+  static constexpr bool kVecRun = C == CH && CH % 4 == 0;
+  ASG_DEV float4* run4(int t0) const { return reinterpret_cast<float4*>(base + idx(t0)); }
+};
+
+template <int CH>
 __global__ void __launch_bounds__(256) k_flux_gate(GateParams p) {
-  extern __shared__ float sk_raw[];
+  extern __shared__ float4 gate_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 8 + warp;
+  const int c = blockIdx.x * (blockDim.x >> 5) + warp;
   if (c >= p.ncols) return;
-  const int nT = p.nT;
+  constexpr int nT = 32 * CH;
   const unsigned mask = 0xffffffffu;
-  PlainColumn col{sk_raw + warp * nT};
+  RunColumn<CH> col{reinterpret_cast<float*>(gate_raw) + warp * RunColumn<CH>::FLOATS};
   const float* src = p.in + (size_t)c * nT;
   float s = 0.f, steep = 0.f;
   for (int t = lane; t < nT; t += 32) {
@@ -1306,9 +1321,14 @@ __global__ void __launch_bounds__(256) k_flux_gate(GateParams p) {
   }
   const int steps = learned ? 1 : nsub;
   const float dzs = p.dz / (float)steps;
-  for (int k = 0; k < steps; ++k) {
-    if (p.mc) kt_step_run<true>(col, nT, p.ndt, dzs, mask);
-    else kt_step_run<false>(col, nT, p.ndt, dzs, mask);
+  if constexpr (CH <= 8) {
+    if (p.mc) kt_steps_short<CH, true>(col, nT, p.ndt, dzs, steps, mask);
+    else kt_steps_short<CH, false>(col, nT, p.ndt, dzs, steps, mask);
+  } else {
+    for (int k = 0; k < steps; ++k) {
+      if (p.mc) kt_step_stream<CH, true>(col, p.ndt, dzs, mask);
+      else kt_step_stream<CH, false>(col, p.ndt, dzs, mask);
+    }
   }
   float* dst = p.out + (size_t)c * nT;
   for (int t = lane; t < nT; t += 32) dst[t] = col.get(t);
@@ -1338,9 +1358,19 @@ __global__ void k_apply_correction(const float* __restrict__ y, const int* __res
     if (t >= 1 && t < nT - 1) out[(size_t)c * nT + t] += s * yr[t];
 }
 
-int launch_gate(const GateParams& p, cudaStream_t st) {
-  const size_t smem = (size_t)8 * p.nT * sizeof(float);  // nT <= 1024
-  k_flux_gate<<<(p.ncols + 7) / 8, 256, smem, st>>>(p);
+// nT = 32 CH, a multiple of 128 up to 1024: the KT step knows its run length (an any-length
+// step walks a chain of range tests: plain sub-cycled columns, 128 x 1024 80 -> 54 us,
+// 16384 x 128 104 -> 67 us).  A column per block up to four blocks per SM, then 2 to 8.
+template <int CH>
+int launch_gate(const GateParams& p, int nsm, cudaStream_t st) {
+  if (p.nT != 32 * CH) {
+    if constexpr (CH < 32) return launch_gate<CH + 4>(p, nsm, st);
+    return ASG_ERR_SHAPE;
+  }
+  int w = 1;
+  while (w < 8 && p.ncols > 4 * nsm * w) w *= 2;
+  k_flux_gate<CH><<<(p.ncols + w - 1) / w, 32 * w,
+                    (size_t)w * RunColumn<CH>::FLOATS * sizeof(float), st>>>(p);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
 }
 
@@ -1394,7 +1424,7 @@ extern "C" int asg_flux_columns_learned(asg_net* n, const float* d_in, float* d_
   g.list_s = list_s;
   g.counter = counter;
   g.clamp = reinterpret_cast<unsigned*>(counter + 1);
-  const int s = launch_gate(g, st);
+  const int s = launch_gate<4>(g, n->nsm, st);
   if (s != ASG_OK) return net_fail(s, "gate launch");
   int cnt[3] = {0, 0, 0};
   if (cudaMemcpyAsync(cnt, counter, sizeof(cnt), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
