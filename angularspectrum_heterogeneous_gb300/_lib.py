@@ -31,7 +31,7 @@ EXPORTED = [
     "asg_net_param_count", "asg_net_create", "asg_net_destroy", "asg_net_set_params",
     "asg_net_get_params", "asg_net_forward", "asg_net_train_step", "asg_flux_columns_learned",
     "asg_net_set_output_scale", "asg_add_source_compact", "asg_debug_set_barrier_skew",
-    "asg_flux_columns_device_clamped", "asg_set_learned", "asg_learned_stats",
+    "asg_debug_line_plan", "asg_flux_columns_device_clamped", "asg_set_learned", "asg_learned_stats",
 ]
 KERNEL_KINDS = ["xy_A", "t_nonlin", "xy_B", "t_mid", "xy_C", "t_end", "other"]
 
@@ -131,6 +131,7 @@ def load(require_device: bool = True):
     lib.asg_get_tuning.argtypes = [P, C.POINTER(Tuning)]
     lib.asg_set_tuning.argtypes = [P, C.POINTER(Tuning)]
     lib.asg_debug_set_barrier_skew.argtypes = [P, C.c_int]
+    lib.asg_debug_line_plan.argtypes = [C.c_int] + 4 * [C.POINTER(C.c_int)]
     lib.asg_autotune.argtypes = [P, F, C.c_double, C.c_int, C.POINTER(Tuning)]
     lib.asg_set_graphs.argtypes = [P, C.c_int]
     lib.asg_net_param_count.argtypes = []

@@ -202,45 +202,6 @@ static void free_axis(LineAxis& a) {
   a = LineAxis{};
 }
 
-// Operations per value of a register DFT of r points, roughly: a direct sum over a
-// prime, a radix-4 split as two stages of 2.
-static int radix_cost(int r) {
-  int c = 0;
-  while (r % 4 == 0) { c += 4; r /= 4; }
-  for (int q = 2; r > 1; ++q)
-    while (r % q == 0) { c += q; r /= q; }
-  return c;
-}
-
-// Factors (n1, n2) of a direct line among the radices of the kernel variants
-// (with_radix), the cheapest pair; false if there is none.
-static bool direct_factors(int n, int* n1, int* n2) {
-  auto ok32 = [](int r) {
-    return (r >= 1 && r <= 18) || r == 20 || r == 21 || r == 24 || r == 25 || r == 27 || r == 28 ||
-           r == 30 || r == 32;
-  };
-  auto ok64 = [](int r) {
-    return r == 27 || r == 28 || r == 30 || r == 32 || r == 36 || r == 40 || r == 48 || r == 64;
-  };
-  int best = 1 << 30;
-  for (int a = 1; a <= 64; ++a) {
-    if (n % a) continue;
-    const int b = n / a;
-    // the larger variants hold fewer warps per SM; an exchange costs about as much as a
-    // radix-4 stage
-    int c = radix_cost(a) + radix_cost(b) + (a > 1 ? 3 : 0) + abs(a - b) / 4;
-    if (n <= 1024 && ok32(a) && ok32(b)) c += a > 16 || b > 16 ? 4 : 0;
-    else if (n > 1024 && ok64(a) && ok64(b)) c += 8;
-    else continue;
-    if (c < best) {
-      best = c;
-      *n1 = a;
-      *n2 = b;
-    }
-  }
-  return best < (1 << 30);
-}
-
 // Factors of the convolution of a chirp line of n samples (n <= 2048): the shortest
 // length >= 2 n - 1 of the compiled ones.
 static bool chirp_factors(int n, int* n1, int* n2) {
@@ -260,22 +221,36 @@ static bool chirp_factors(int n, int* n1, int* n2) {
   return best < (1 << 30);
 }
 
+// How a line of n samples is transformed: n1, n2, m, direct, and the variant of a direct line.
+static bool line_factors(int n, LineAxis* a) {
+  if (n < 1 || n > LINE_DIRECT_MAX) return false;
+  a->direct = LINE_DIRECT.n1[n] != 0;
+  a->n1 = LINE_DIRECT.n1[n];
+  a->n2 = LINE_DIRECT.n2[n];
+  a->rm = LINE_DIRECT.rm[n];
+  if (!a->direct && !chirp_factors(n, &a->n1, &a->n2)) return false;
+  a->m = a->n1 * a->n2;
+  return true;
+}
+extern "C" int asg_debug_line_plan(int n, int* direct, int* variant, int* n1, int* n2) {
+  g_err.clear();
+  LineAxis a = {};
+  if (!direct || !variant || !n1 || !n2) return fail(ASG_ERR_ARG, "null argument");
+  if (!line_factors(n, &a)) return fail(ASG_ERR_SHAPE, "no transform of %d samples", n);
+  *direct = a.direct;
+  *variant = a.rm;
+  *n1 = a.n1;
+  *n2 = a.n2;
+  return ASG_OK;
+}
+
 // Factors and tables of a line of n samples.
 static int line_axis(int n, LineAxis* a, cudaStream_t st) {
   a->n = n;
   a->inv_hi = (float)(1.0 / n);
   a->inv_lo = (float)(1.0 / n - (double)a->inv_hi);
-  int n1 = 0, n2 = 0;
-  a->direct = direct_factors(n, &n1, &n2) ? 1 : 0;
-  if (!a->direct && !chirp_factors(n, &n1, &n2))
-    return fail(ASG_ERR_SHAPE, "line of %d samples too long", n);
-  const int m = n1 * n2;
-  a->m = m;
-  a->n1 = n1;
-  a->n2 = n2;
-  const int big = n1 > n2 ? n1 : n2;
-  // lengths above 1024 have their own direct radices
-  a->rm = n > 1024 ? 64 : big <= 16 ? 16 : big <= 24 ? 24 : 32;
+  if (!line_factors(n, a)) return fail(ASG_ERR_SHAPE, "line of %d samples too long", n);
+  const int n1 = a->n1, n2 = a->n2, m = a->m;
   const int tws = a->direct ? a->rm : n2;  // DirectPlan / ChirpPlan strides
   a->s2 = tws + 2;
   a->mg1 = ((1u << 20) + n1 - 1) / n1;

@@ -265,8 +265,55 @@ struct ChirpPlan {
   ASG_DEV static void with_n2(const LineAxis&, F f) { f(Radix<N2>{}); }
 };
 
-#define ASG_RADIX(R) \
-  case R: f(Radix<R>{}); break;
+// Radices of the direct variant RM: all up to 18 and the 7-smooth ones up to RM, 32 at
+// most; the variant for lengths above 1024 (RM = 64) has some from 27 to 64.
+constexpr bool line_radix(int rm, int r) {
+  if (rm == 64)
+    return r == 27 || r == 28 || r == 30 || r == 32 || r == 36 || r == 40 || r == 48 || r == 64;
+  return r >= 1 && r <= rm &&
+         (r <= 18 || r == 20 || r == 21 || r == 24 || r == 25 || r == 27 || r == 28 || r == 30 ||
+          r == 32);
+}
+// Operations per value of a register DFT of r points, roughly: a direct sum over a
+// prime, a radix-4 split as two stages of 2.
+constexpr int radix_cost(int r) {
+  int c = 0;
+  while (r % 4 == 0) { c += 4; r /= 4; }
+  for (int q = 2; r > 1; ++q)
+    while (r % q == 0) { c += q; r /= q; }
+  return c;
+}
+// Direct lines: for each length the cheapest pair n1 <= n2 of radices (0: none), its
+// variant, and which radices a variant meets as n1 or as n2.  The kernels hold the code
+// of those only.
+constexpr int LINE_DIRECT_MAX = 2048;
+struct LineDirect {
+  unsigned char n1[LINE_DIRECT_MAX + 1], n2[LINE_DIRECT_MAX + 1], rm[LINE_DIRECT_MAX + 1];
+  bool used[2][65][65];  // [n1, n2][variant][radix]
+};
+constexpr LineDirect make_line_direct() {
+  LineDirect d{};
+  int best[LINE_DIRECT_MAX + 1] = {};
+  for (int a = 1; a <= 64; ++a)
+    for (int b = a; b <= 64 && a * b <= LINE_DIRECT_MAX; ++b) {
+      const int n = a * b;
+      if (!line_radix(n > 1024 ? 64 : 32, a) || !line_radix(n > 1024 ? 64 : 32, b)) continue;
+      // the larger variants hold fewer warps per SM; an exchange costs about as much as a
+      // radix-4 stage
+      const int c = radix_cost(a) + radix_cost(b) + (a > 1 ? 3 : 0) + (b - a) / 4 +
+                    (n > 1024 ? 8 : b > 16 ? 4 : 0);
+      if (best[n] != 0 && c >= best[n]) continue;
+      best[n] = c;
+      d.n1[n] = (unsigned char)a;
+      d.n2[n] = (unsigned char)b;
+      d.rm[n] = (unsigned char)(n > 1024 ? 64 : b <= 16 ? 16 : b <= 24 ? 24 : 32);
+    }
+  for (int n = 1; n <= LINE_DIRECT_MAX; ++n)
+    if (d.n1[n] != 0) d.used[0][d.rm[n]][d.n1[n]] = d.used[1][d.rm[n]][d.n2[n]] = true;
+  return d;
+}
+constexpr LineDirect LINE_DIRECT = make_line_direct();
+
 template <int RM>
 struct DirectPlan {
   static constexpr bool DIRECT = true;
@@ -275,42 +322,24 @@ struct DirectPlan {
   ASG_DEV static int n2(const LineAxis& ax) { return ax.n2; }
   ASG_DEV static int div1(const LineAxis& ax, int i) { return div_magic(i, ax.mg1); }
   ASG_DEV static int div2(const LineAxis& ax, int i) { return div_magic(i, ax.mg2); }
-  // radices: all up to 18, the 7-smooth ones up to 32; for lengths above 1024 some
-  // up to 64
-  template <class F>
+  // f(Radix<R>) of the radix R that a line has as n1 (POS 0) or n2 (POS 1)
+  template <int POS, class F>
   ASG_DEV static void with_radix(int r, F f) {
-    if constexpr (RM == 16) {
-      switch (r) {
-        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
-        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
-        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) default: break;
-      }
-    } else if constexpr (RM == 24) {
-      switch (r) {
-        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
-        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
-        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) ASG_RADIX(17) ASG_RADIX(18)
-        ASG_RADIX(20) ASG_RADIX(21) ASG_RADIX(24) default: break;
-      }
-    } else if constexpr (RM == 32) {
-      switch (r) {
-        ASG_RADIX(1) ASG_RADIX(2) ASG_RADIX(3) ASG_RADIX(4) ASG_RADIX(5) ASG_RADIX(6)
-        ASG_RADIX(7) ASG_RADIX(8) ASG_RADIX(9) ASG_RADIX(10) ASG_RADIX(11) ASG_RADIX(12)
-        ASG_RADIX(13) ASG_RADIX(14) ASG_RADIX(15) ASG_RADIX(16) ASG_RADIX(17) ASG_RADIX(18)
-        ASG_RADIX(20) ASG_RADIX(21) ASG_RADIX(24) ASG_RADIX(25) ASG_RADIX(27) ASG_RADIX(28)
-        ASG_RADIX(30) ASG_RADIX(32) default: break;
-      }
-    } else {
-      switch (r) {
-        ASG_RADIX(27) ASG_RADIX(28) ASG_RADIX(30) ASG_RADIX(32) ASG_RADIX(36) ASG_RADIX(40)
-        ASG_RADIX(48) ASG_RADIX(64) default: break;
-      }
+#define R_(R) \
+  case R:     \
+    if constexpr (LINE_DIRECT.used[POS][RM][R]) f(Radix<R>{}); \
+    break;
+    switch (r) {
+      R_(1) R_(2) R_(3) R_(4) R_(5) R_(6) R_(7) R_(8) R_(9) R_(10) R_(11) R_(12) R_(13) R_(14)
+      R_(15) R_(16) R_(17) R_(18) R_(20) R_(21) R_(24) R_(25) R_(27) R_(28) R_(30) R_(32)
+      R_(36) R_(40) R_(48) R_(64) default: break;
     }
+#undef R_
   }
   template <class F>
-  ASG_DEV static void with_n1(const LineAxis& ax, F f) { with_radix(ax.n1, f); }
+  ASG_DEV static void with_n1(const LineAxis& ax, F f) { with_radix<0>(ax.n1, f); }
   template <class F>
-  ASG_DEV static void with_n2(const LineAxis& ax, F f) { with_radix(ax.n2, f); }
+  ASG_DEV static void with_n2(const LineAxis& ax, F f) { with_radix<1>(ax.n2, f); }
 };
 
 // position of natural index j in a line
@@ -406,7 +435,8 @@ inline int line_threads(int tasks, int nt_max) {
 // a block takes as many lines as these need to fill it
 inline int line_tasks(const LineAxis& ax) { return ax.n1 < ax.n2 ? ax.n1 : ax.n2; }
 
-// Factors of the chirp convolutions: each length at most 1.33 times the one before.  F(n1, n2)
+// Factors of the chirp convolutions: each length at most 1.5 times the one before, from
+// 128 on 1.33 times.  F(n1, n2)
 #define ASG_CHIRP_SIZES(F)                                                               \
-  F(4, 8) F(4, 12) F(8, 8) F(8, 12) F(8, 16) F(8, 20) F(12, 16) F(16, 16) F(16, 20)     \
+  F(4, 12) F(8, 8) F(8, 12) F(8, 16) F(8, 20) F(12, 16) F(16, 16) F(16, 20)     \
   F(16, 24) F(16, 32) F(24, 24) F(20, 32) F(24, 32) F(32, 32) F(32, 40) F(32, 48) F(32, 64)

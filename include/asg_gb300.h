@@ -225,6 +225,11 @@ typedef struct {
  * ASG_ERR_TIMEOUT; 0 restores normal operation. */
 int asg_debug_set_barrier_skew(asg_plan* plan, int skew);
 
+/* Test hook (no counterpart in the reference, needs no device): how an axis of n samples
+ * (1 to 2048) is transformed where no fast kernel takes it.  direct = 1: n = n1 n2 by the
+ * kernel variant `variant`; 0: as a convolution of n1 n2 points. */
+int asg_debug_line_plan(int n, int* direct, int* variant, int* n1, int* n2);
+
 /* Effective launch shapes (defaults resolved). */
 int asg_get_tuning(asg_plan* plan, asg_tuning* out);
 
