@@ -289,6 +289,73 @@ static int line_axis(int n, LineAxis* a, cudaStream_t st) {
   return ASG_OK;
 }
 
+// Passes of an axis of a small plane: the factors of its line transform, those above 9 split
+// again, primes up to 19 as they are; empty if there are none.
+static std::vector<int> plane_radices(int n) {
+  std::vector<int> r;
+  LineAxis a = {};
+  if (n < 1 || !line_factors(n, &a)) return r;
+  std::vector<int> todo = {n};
+  if (a.direct) todo = {a.n2, a.n1};
+  while (!todo.empty()) {
+    const int f = todo.back(), p = radix_split(f);
+    todo.pop_back();
+    if (f == 1) continue;
+    if (f <= 9 || (p == f && f <= 19)) {
+      r.push_back(f);
+    } else if (p == f) {
+      return {};
+    } else {
+      todo.push_back(f / p);
+      todo.push_back(p);
+    }
+  }
+  return r.size() <= 8 ? r : std::vector<int>();
+}
+// Whether a plane runs in one block: its axes have passes (19 samples only beside an axis of
+// other factors: 17 x 19 82 us per step, 88 in three launches; 19 x 19 and 23 x 16 gain
+// nothing) and
+//   * up to 8 samples along an axis, whatever fits: short rows, or columns that fill a part
+//     of the column pass's lanes (1024 x 2 55 -> 21 us per stage, 4 x 512 30 -> 18);
+//   * otherwise up to 10500 samples times passes, where the passes over all samples begin to
+//     cost as much as the two further launches (us per step of 128 samples in three
+//     launches and in one block: 16 x 16 70 and 43, 48 x 48 66 and 63, 60 x 60 78 and 90,
+//     24 x 100 66 and 76).
+static bool small_plane(int X, int Y) {
+  const int px = (int)plane_radices(X).size(), py = (int)plane_radices(Y).size();
+  if (px == 0 || py == 0 || (LINE_DIRECT.n1[X] == 0 && LINE_DIRECT.n1[Y] == 0)) return false;
+  if ((size_t)X * (Y | 1) * sizeof(float2) > ASG_PLANE_MAX_SMEM) return false;
+  return std::min(X, Y) <= 8 || X * Y * (px + py) <= 10500;
+}
+// bin in slot s of a transformed line
+static int plane_bin(const std::vector<int>& r, int n, int s) {
+  int bin = 0, w = 1;
+  for (int f : r) {
+    n /= f;
+    bin += w * (s / n);
+    s %= n;
+    w *= f;
+  }
+  return bin;
+}
+static int plane_axis(int n, PlaneAxis* a, cudaStream_t st) {
+  a->n = n;
+  a->radices = 0;
+  int i = 0;
+  for (int f : plane_radices(n)) a->radices |= (unsigned long long)f << (8 * i++);
+  std::vector<float4> tw(n);
+  for (int j = 0; j < n; ++j) {
+    const double ang = -2.0 * M_PI * (double)j / (double)n;
+    tw[j] = two_floats(cos(ang), sin(ang));
+  }
+  float4* d = nullptr;
+  CKS(dalloc(&d, n));
+  a->tw = d;
+  CKS(h2d(d, tw.data(), n, st));
+  CK(cudaStreamSynchronize(st));  // the host vector goes out of scope
+  return ASG_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Python's built-in sum() over a list of floats (CPython >= 3.12): the first
 // item enters exactly (0 + x0), later items with Neumaier compensation, and
@@ -385,6 +452,8 @@ struct asg_plan {
   GenPlan gp_x, gp_y;
   LineAxis ax_t = {};         // any-length column transforms (not tfast)
   bool lines = false;         // plane passes as any-length row and column passes
+  bool small = false;         // plane passes of one block per plane
+  PlaneAxis pl_x = {}, pl_y = {};
   LineAxis ax_x = {}, ax_y = {};
   cudaStream_t st;
   cudaEvent_t ev0, ev1;
@@ -524,6 +593,8 @@ extern "C" int asg_plan_destroy(asg_plan* p) {
   free_axis(p->ax_t);
   free_axis(p->ax_x);
   free_axis(p->ax_y);
+  cudaFree(const_cast<float4*>(p->pl_x.tw));
+  cudaFree(const_cast<float4*>(p->pl_y.tw));
   free_outputs(p);
   cudaEventDestroy(p->ev0);
   cudaEventDestroy(p->ev1);
@@ -548,7 +619,8 @@ static int upload_roots() {
       asg_roots_upload_xy(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_l2(w192.data(), w64.data()) != 0 ||
       asg_roots_upload_tp(lr.data()) != 0 ||
-      asg_roots_upload_xyrows(lr.data()) != 0 || asg_roots_upload_xycols(lr.data()) != 0)
+      asg_roots_upload_xyrows(lr.data()) != 0 || asg_roots_upload_xycols(lr.data()) != 0 ||
+      asg_roots_upload_xyplane(lr.data()) != 0)
     return fail(ASG_ERR_CUDA, "upload of the constant root tables failed");
   g_roots_done[dev] = true;
   return ASG_OK;
@@ -583,8 +655,9 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     p->G = 1;
     // the row and column passes take lines up to 1024; a plane with more rows
     // runs in one CTA's shared memory if it fits
-    p->lines = X <= ASG_LINES_MAX;
-    if (!p->lines && asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM)
+    p->small = small_plane(X, Y);
+    p->lines = !p->small && X <= ASG_LINES_MAX;
+    if (!p->small && !p->lines && asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM)
       return fail(ASG_ERR_SHAPE, "grid %dx%d: nX > 1024 without a fast plane transform", X, Y);
   }
   if (!p->tfast && T > ASG_T_MAX)
@@ -602,6 +675,10 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     CKS(line_axis(X, &p->ax_x, p->st));
     CKS(line_axis(Y, &p->ax_y, p->st));
   }
+  if (p->small) {
+    CKS(plane_axis(X, &p->pl_x, p->st));
+    CKS(plane_axis(Y, &p->pl_y, p->st));
+  }
 
   // ---- planes ----
   p->h_f_of_plane.resize(p->F);
@@ -617,6 +694,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   // natural bin held by each x slot (row order of the plane kernels) and by
   // each y slot (the fast kernels keep y in four-step slot order)
   std::vector<int> binx(X), biny(Y);
+  const std::vector<int> rx = plane_radices(X);
   for (int s = 0; s < X; ++s) {
     if (p->split) {
       const int Xs = X / 2, R = 16, h = s / Xs, sg = s % Xs;
@@ -624,6 +702,8 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     } else if (p->xyfast) {
       const int R = 32;
       binx[s] = (s / R) + p->G * (s % R);
+    } else if (p->small) {
+      binx[s] = plane_bin(rx, X, s);
     } else {
       binx[s] = s;
     }
@@ -671,6 +751,12 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     for (int s = 0; s < n; ++s) cls[s] = id[raw[s]];
   };
   classes(Y, biny, p->h_cls_y, p->ncy, p->h_rep_y);
+  if (p->small) {
+    // classes numbered in natural order (the tables' roundings are spread along it), slots
+    // in that of the passes
+    const std::vector<int> nat = p->h_cls_y, ry = plane_radices(Y);
+    for (int s = 0; s < Y; ++s) p->h_cls_y[s] = nat[plane_bin(ry, Y, s)];
+  }
 
   // ---- device buffers ----
   const size_t nspec = (size_t)p->F * p->ncols;
@@ -819,7 +905,7 @@ static int build_tables(asg_plan* p, Slot& s, float2* out_pa, float2* out_p, flo
   // field 1.3e-6 too large without, 2e-7 with.  The other plane kernels' transforms shrink
   // the field a little more than FP32 moduli make it grow (128 x 128 x 384 error 5.1e-6 so,
   // 5.3e-6 with exact moduli) and keep them.
-  tp.spread = p->lines ? 1 : 0;
+  tp.spread = p->lines || p->small ? 1 : 0;
   tp.out_pa = out_pa;
   tp.out_p = out_p;
   tp.out_a = out_a;
@@ -1193,6 +1279,7 @@ static int run_t(asg_plan* p, const TParams& t, int kind = ASG_K_OTHER) {
 static int run_xy(asg_plan* p, const XYParams& x, int kind = ASG_K_OTHER) {
   KScope k(p, kind);
   if (p->l2 && x.epi == 0 && x.nscreens == 0) return asg_launch_xy_l2(x, p->st);
+  if (p->small) return asg_launch_xy_plane(x, p->pl_x, p->pl_y, p->st);
   if (p->lines) return asg_launch_xy_lines(x, p->ax_x, p->ax_y, p->st);
   return asg_launch_xy(x, p->xyfast, p->gp_x, p->gp_y, p->st);
 }

@@ -167,6 +167,16 @@ int asg_launch_xy_lines(const XYParams& p, const LineAxis& axx, const LineAxis& 
 int asg_launch_xy_rows(const XYParams& p, const LineAxis& ax, float2* dst, bool inverse,
                        cudaStream_t st);
 int asg_launch_xy_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaStream_t st);
+// small planes, one block each (asg_xyplane.cu): an axis of n samples by passes of the
+// radices, low byte first, with tw[j] = exp(-2 pi i j / n) as (hi.re, hi.im, lo.re, lo.im)
+struct PlaneAxis {
+  int n;
+  unsigned long long radices;
+  const float4* tw;
+};
+constexpr size_t ASG_PLANE_MAX_SMEM = 47 * 1024;
+int asg_launch_xy_plane(const XYParams& p, const PlaneAxis& axx, const PlaneAxis& axy,
+                        cudaStream_t st);
 int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPlan& ply,
                   cudaStream_t st);
 
@@ -207,6 +217,7 @@ int asg_roots_upload_l2(const float2* w192, const float2* w64);
 int asg_roots_upload_tp(const float4* line_roots);
 int asg_roots_upload_xyrows(const float4* line_roots);
 int asg_roots_upload_xycols(const float4* line_roots);
+int asg_roots_upload_xyplane(const float4* line_roots);
 
 // One-time launcher set-up (shared-memory attributes, occupancy queries,
 // constant tables) is per device: what is set with one device current does not
@@ -216,6 +227,17 @@ inline int asg_device_slot() {
   int d = 0;
   if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= ASG_MAX_DEVICES) d = 0;
   return d;
+}
+
+// multiprocessors of the current device
+inline int asg_sm_count() {
+  static int n[ASG_MAX_DEVICES] = {};
+  int& c = n[asg_device_slot()];
+  int d = 0;
+  if (c == 0 && (cudaGetDevice(&d) != cudaSuccess ||
+                 cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, d) != cudaSuccess))
+    return 152;
+  return c;
 }
 
 // error reporting shared by the translation units (message for asg_last_error)

@@ -14,11 +14,9 @@
 // Nyquist plane, whose Re() precedes the corrections, is left without epilogue
 // (p.skip_plane) and goes through the epilogue pass.
 //
-// Against one CTA per plane (small planes, 51 CTAs for 101 samples) or Stockham
-// lines with direct sums over prime factors, per stage: 257 x 257 x 601 12.6 ->
-// 1.03 ms, 81 x 81 x 101 94-112 -> 27-33 us, 51 x 51 x 401 72 -> 38 us,
-// 200 x 180 x 400 580-640 -> 135-218 us (5 x 5 x 1001, three launches for one:
-// 14 -> 22 us).
+// Against one CTA per plane or Stockham lines with direct sums over prime factors, per
+// stage: 257 x 257 x 601 12.6 -> 1.03 ms, 81 x 81 x 101 94-112 -> 27-33 us, 200 x 180 x 400
+// 580-640 -> 135-218 us.  Small planes run in one launch (asg_xyplane.cu).
 //
 // Reference semantics: see asg_xykernel.cu.
 #include "asg_internal.h"
