@@ -148,13 +148,11 @@ static float4 two_floats(double re, double im) {
   return make_float4(x, y, (float)(re - (double)x), (float)(im - (double)y));
 }
 
-// Resident CTA groups of the L2 plane kernels: the tuning knobs cap them at 1..64 (64: no
-// cap).  The scratch holds 64 from 256-wide planes up, where fewer are resident, and
-// 256 below: 114 groups of the 128-wide planes fit the GPU, and 128 x 128 x 256's
-// 258 half-planes took 5 rounds of 64 groups, 41 -> 33 us per stage (192 x 192 x 512
-// 125 -> 111, 64 x 128 x 256 33 -> 22).
+// Resident CTA groups of the L2 plane kernels: the tuning knobs cap them at 1..63 (64: all
+// that fit the GPU).  Planes below 256 wide use more than 64: 114 groups of the 128-wide
+// ones fit, and 128 x 128 x 256's 258 half-planes took 5 rounds of 64 groups, 41 -> 33 us per
+// stage (192 x 192 x 512 125 -> 111, 64 x 128 x 256 33 -> 22).
 static constexpr int L2_MAX_CLUSTERS = 64;
-static int l2_group_cap(int Y) { return Y >= 256 ? L2_MAX_CLUSTERS : 256; }
 
 // four-step slot order of a fast line of length n (n = n1*n2)
 static void fast_factors(int n, int* n1, int* n2) {
@@ -453,7 +451,8 @@ struct asg_plan {
   int xy_sync = 0;            // group barrier of the L2 plane kernels: 0 default,
                               // 1 thread-block cluster, 2 counters in a cooperative launch
   int batch_refs = 0;         // batches holding the plan (they use cluster barriers)
-  unsigned* grp_cnt = nullptr;  // [2][groups] counters of the cooperative launch
+  int l2_groups = 0;          // CTA groups that the scratch holds: all that can be resident
+  unsigned* grp_cnt = nullptr;  // [2][l2_groups] counters of the cooperative launch
   unsigned barrier_skew = 0;    // test hook: added to the group-barrier targets
   // CUDA graph of a regular march step (slot 0, no screen, source, callback,
   // profiling or output write); rebuilt when `gen` moves on
@@ -783,9 +782,12 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     if (2 * p->h_f_of_plane[q] == T) p->nyq_plane = q;
   if ((p->l2 || p->lines) && p->nyq_plane >= 0) CKS(dalloc(&p->nyq_tmp, (size_t)X * Y));
   if (p->l2) {
-    // scratch: two half-planes for each resident group
+    // scratch: two half-planes for each group that can be resident, no more than there are
+    // half-planes
     const int Xs = X / 2;
-    CKS(dalloc(&p->l2_scratch, (size_t)l2_group_cap(Y) * 2 * Xs * Y));
+    p->l2_groups = std::min(asg_xy_l2_max_groups(X, Y), 2 * p->F);
+    if (p->l2_groups < 1) return fail(ASG_ERR_CUDA, "occupancy query of the plane kernels failed");
+    CKS(dalloc(&p->l2_scratch, (size_t)p->l2_groups * 2 * Xs * Y));
     int n1, n2;
     fast_factors(Xs, &n1, &n2);
     std::vector<int> cl(2 * Xs);
@@ -799,7 +801,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
       }
     CKS(dalloc(&p->l2_cls_x, 2 * Xs));
     CKS(h2d(p->l2_cls_x, cl.data(), 2 * Xs, p->st));
-    CKS(dalloc(&p->grp_cnt, 2 * l2_group_cap(Y)));
+    CKS(dalloc(&p->grp_cnt, 2 * p->l2_groups));
   }
   CKS(dalloc(&p->real, (size_t)p->ncols * T));
   std::vector<float2> w;
@@ -1226,6 +1228,11 @@ static void set_epilogue(const asg_plan* p, XYParams* x, int epi) {
   x->ey1 = in[3];
 }
 
+// CTA groups of the L2 plane kernels under a tuning knob
+static int l2_groups(const asg_plan* p, int knob) {
+  return knob > 0 && knob < L2_MAX_CLUSTERS ? std::min(knob, p->l2_groups) : p->l2_groups;
+}
+
 static XYParams xyparams(asg_plan* p, const float2* table, bool zero_dc_nyq) {
   XYParams x;
   memset(&x, 0, sizeof(x));
@@ -1266,8 +1273,7 @@ static XYParams xyparams(asg_plan* p, const float2* table, bool zero_dc_nyq) {
   x.power_acc = p->power_acc;
   x.l2_scratch = p->l2_scratch;
   x.l2_cls_x = p->l2_cls_x;
-  x.l2_max_clusters = (p->xy_clusters > 0 && p->xy_clusters < L2_MAX_CLUSTERS)
-                          ? p->xy_clusters : l2_group_cap(p->Y);
+  x.l2_max_clusters = l2_groups(p, p->xy_clusters);
   x.coop = xy_sync_of(p) >= 2 ? 1 : 0;
   x.pipe = xy_sync_of(p) == 3 ? 1 : 0;
   x.bulk_rows = p->xy_bulk;
@@ -1469,8 +1475,7 @@ static int closing_stage(asg_plan* p, const float2* table, int epi, int nscr, in
     x.nscreens = nscr;
     x.screens = p->d_screens;
     x.skip_plane = p->nyq_plane;
-    x.l2_max_clusters = (p->xy_clusters_c > 0 && p->xy_clusters_c < L2_MAX_CLUSTERS)
-                            ? p->xy_clusters_c : l2_group_cap(p->Y);
+    x.l2_max_clusters = l2_groups(p, p->xy_clusters_c);
     {
       KScope k(p, kind);
       CKS(asg_launch_xy_l2_closing(x, p->st));

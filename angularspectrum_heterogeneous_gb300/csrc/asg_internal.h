@@ -151,6 +151,7 @@ struct XYParams {
 bool asg_xy_fast_supported(int X, int Y, int* G_out);
 // L2-exchange plane kernel (asg_xyl2.cu)
 bool asg_xy_l2_supported(int X, int Y, int nsub, int* G_out);
+int asg_xy_l2_max_groups(int X, int Y);
 int asg_launch_xy_l2(const XYParams& p, cudaStream_t st);
 // closing stage with the epilogue fused, whole planes out (same support as above, nsub = 2)
 int asg_launch_xy_l2_closing(const XYParams& p, cudaStream_t st);

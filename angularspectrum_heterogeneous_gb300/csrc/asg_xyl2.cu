@@ -26,6 +26,8 @@
 // (angular_spectrum_solver.py :649-655, :667-685, :630-643).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "asg_internal.h"
 
 namespace cg = cooperative_groups;
@@ -1034,22 +1036,31 @@ static int coop_max_groups(K kern, int nt, size_t smem, int G) {
   return per_sm * nsm / G;
 }
 
+static cudaLaunchAttribute cluster_attr(int G) {
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeClusterDimension;
+  a.val.clusterDim.x = G;
+  a.val.clusterDim.y = 1;
+  a.val.clusterDim.z = 1;
+  return a;
+}
+
 // Launches `units` (sub-)planes over at most `resident` groups (clusters, or
 // CTA groups of a cooperative launch) and the scratch the plan sized.
 template <class K>
-static int launch_groups(K kern, const XYParams& p, cudaLaunchConfig_t cfg, int resident,
-                         int units, cudaStream_t st) {
+static int launch_groups(K kern, const XYParams& p, int nt, size_t smem, int resident, int units,
+                         cudaStream_t st) {
   int ng = resident < units ? resident : units;
   if (ng > p.l2_max_clusters) ng = p.l2_max_clusters;
   if (ng < 1) return ASG_ERR_SHAPE;
-  cudaLaunchAttribute coop[1], cluster[2];
-  if (!p.coop && p.pdl) {
-    cluster[0] = cfg.attrs[0];
-    cluster[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    cluster[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = cluster;
-    cfg.numAttrs = 2;
-  }
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.G * ng, 1, 1);
+  cfg.blockDim = dim3(nt, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (p.coop) {
     if (p.grp_cnt == nullptr) return ASG_ERR_ARG;
     // every CTA of the grid is resident, so the counter barriers of a group
@@ -1057,73 +1068,78 @@ static int launch_groups(K kern, const XYParams& p, cudaLaunchConfig_t cfg, int 
     if (cudaMemsetAsync(p.grp_cnt, 0, (size_t)(p.l2_max_clusters + ng) * sizeof(unsigned), st) !=
         cudaSuccess)
       return ASG_ERR_CUDA;
-    coop[0].id = cudaLaunchAttributeCooperative;
-    coop[0].val.cooperative = 1;
-    cfg.attrs = coop;
-    cfg.numAttrs = 1;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  } else {
+    attr[0] = cluster_attr(p.G);
+    if (p.pdl) {
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.numAttrs = 2;
+    }
   }
-  cfg.gridDim = dim3(p.G * ng, 1, 1);
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
   return e == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
+}
+
+// Groups of G CTAs resident at once with `smem` bytes per CTA, as clusters and as groups of a
+// cooperative launch (queried once per kernel and device); sets the kernel's attributes.
+struct GroupLimits {
+  int clusters = 0, groups = 0;  // 0: not queried yet
+};
+template <class K>
+static int group_limits(K kern, int G, int nt, size_t smem, GroupLimits* cached,
+                        GroupLimits* out) {
+  GroupLimits& l = cached[asg_device_slot()];
+  if (l.clusters == 0) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return ASG_ERR_CUDA;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = cluster_attr(G);
+    cfg.gridDim = dim3(G * 1024, 1, 1);
+    cfg.blockDim = dim3(nt, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    // groups of more than 16 CTAs run only as cooperative launches
+    if (G > 16 || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = 1;
+    l.groups = coop_max_groups(kern, nt, smem, G);
+    l.clusters = n;
+  }
+  *out = l;
+  return ASG_OK;
 }
 
 // R rows per CTA and NT threads per block; the plan's group size p.G is that
 // of 16-row CTAs (the cluster shape), the launch uses Xn / R.
 template <int Yn, int Xn, int R, int NT>
-static int launch_l2(const XYParams& pin, cudaStream_t st) {
+struct L2Launch {
   using PY = FastPlan<Yn>;
-  using PX = FastPlan<Xn>;
-  XYParams p = pin;
-  if (p.G != Xn / 16) return ASG_ERR_SHAPE;
-  p.G = Xn / R;
-  const int Yc = Yn / p.G;
-  const int nbuf = (R * PY::PADDED > Xn * Yc) ? R * PY::PADDED : Xn * Yc;
-  p.l2_buf_elems = nbuf;
-  const size_t smem =
+  static constexpr int G = Xn / R, Yc = Yn / G;
+  static constexpr int nbuf = (R * PY::PADDED > Xn * Yc) ? R * PY::PADDED : Xn * Yc;
+  static constexpr size_t smem =
       L2Shape<PY, NT>::kTablesInSmem
           ? (size_t)(nbuf + Yn + Xn) * sizeof(float2) + (size_t)(Yn + 2 * Xn) * sizeof(int)
           : (size_t)nbuf * sizeof(float2);
-  auto kern = xy_l2<PY, PX, R, NT>;
-  static int max_clusters_dev[ASG_MAX_DEVICES], cached_G_dev[ASG_MAX_DEVICES];
-  static bool init_dev[ASG_MAX_DEVICES] = {};
-  const int dev = asg_device_slot();
-  int& max_clusters = max_clusters_dev[dev];
-  int& cached_G = cached_G_dev[dev];
-  if (!init_dev[dev]) {
-    max_clusters = -1;
-    cached_G = -1;
-    init_dev[dev] = true;
+  static int limits(GroupLimits* l) {
+    static GroupLimits cached[ASG_MAX_DEVICES];
+    return group_limits(xy_l2<PY, FastPlan<Xn>, R, NT>, G, NT, smem, cached, l);
   }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.G;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(NT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  static int max_groups_dev[ASG_MAX_DEVICES];
-  int& max_groups = max_groups_dev[dev];
-  if (max_clusters < 0 || cached_G != p.G) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return ASG_ERR_CUDA;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cfg.gridDim = dim3(p.G * 1024, 1, 1);
-    int n = 0;
-    // groups of more than 16 CTAs run only as cooperative launches
-    if (p.G > 16 || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0)
-      n = 1;
-    max_clusters = n;
-    max_groups = coop_max_groups(kern, NT, smem, p.G);
-    cached_G = p.G;
+  static int launch(const XYParams& pin, cudaStream_t st) {
+    XYParams p = pin;
+    if (p.G != Xn / 16) return ASG_ERR_SHAPE;
+    p.G = G;
+    p.l2_buf_elems = nbuf;
+    GroupLimits l;
+    const int s = limits(&l);
+    if (s != ASG_OK) return s;
+    return launch_groups(xy_l2<PY, FastPlan<Xn>, R, NT>, p, NT, smem,
+                         p.coop ? l.groups : l.clusters, p.nplanes * p.nsub, st);
   }
-  const int nq = p.nplanes * p.nsub;
-  return launch_groups(kern, p, cfg, p.coop ? max_groups : max_clusters, nq, st);
-}
+};
 
 // Cooperative launches of the transform (not the power sums, which keep the
 // summation order of the cluster shape) run 8-row CTAs of 4 warps from
@@ -1134,9 +1150,9 @@ static int launch_l2(const XYParams& pin, cudaStream_t st) {
 template <int Yn, int Xn>
 static int launch_l2_mode(const XYParams& p, cudaStream_t st) {
   if constexpr (Yn >= 256) {
-    if (p.coop && !p.power_only && p.rows8) return launch_l2<Yn, Xn, 8, 128>(p, st);
+    if (p.coop && !p.power_only && p.rows8) return L2Launch<Yn, Xn, 8, 128>::launch(p, st);
   }
-  return launch_l2<Yn, Xn, 16, 256>(p, st);
+  return L2Launch<Yn, Xn, 16, 256>::launch(p, st);
 }
 
 int asg_launch_xy_l2(const XYParams& p, cudaStream_t st) {
@@ -1153,62 +1169,66 @@ int asg_launch_xy_l2(const XYParams& p, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 template <int Yn, int Xn>
-static int launch_l2c(const XYParams& pin, cudaStream_t st) {
+struct L2cLaunch {
   using PY = FastPlan<Yn>;
-  using PX = FastPlan<Xn>;
-  constexpr int R = 16, NT = 256;
-  constexpr int G = Xn / R, Yc = Yn / G, YR = Yc < 16 ? Yc : 16;
-  XYParams p = pin;
-  if (p.G != G || p.nsub != 2) return ASG_ERR_SHAPE;
-  const int nbuf = (R * PY::PADDED > 2 * Xn * YR) ? R * PY::PADDED : 2 * Xn * YR;
-  p.l2_buf_elems = nbuf;
-  const size_t smem = (size_t)(nbuf + Yn + Xn) * sizeof(float2) +
-                      (size_t)(2 * (2 * Xn) + 2 * Yn) * sizeof(float) +
-                      (size_t)(Yn + 2 * Xn) * sizeof(int);
-  auto kern = xy_l2c<PY, PX, R, NT>;
-  static int max_clusters_dev[ASG_MAX_DEVICES];
-  static bool init_dev[ASG_MAX_DEVICES] = {};
-  const int dev = asg_device_slot();
-  int& max_clusters = max_clusters_dev[dev];
-  if (!init_dev[dev]) {
-    max_clusters = -1;
-    init_dev[dev] = true;
+  static constexpr int R = 16, NT = 256;
+  static constexpr int G = Xn / R, Yc = Yn / G, YR = Yc < 16 ? Yc : 16;
+  static constexpr int nbuf = (R * PY::PADDED > 2 * Xn * YR) ? R * PY::PADDED : 2 * Xn * YR;
+  static constexpr size_t smem = (size_t)(nbuf + Yn + Xn) * sizeof(float2) +
+                                 (size_t)(2 * (2 * Xn) + 2 * Yn) * sizeof(float) +
+                                 (size_t)(Yn + 2 * Xn) * sizeof(int);
+  static int limits(GroupLimits* l) {
+    static GroupLimits cached[ASG_MAX_DEVICES];
+    return group_limits(xy_l2c<PY, FastPlan<Xn>, R, NT>, G, NT, smem, cached, l);
   }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = G;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(NT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  static int max_groups_dev[ASG_MAX_DEVICES];
-  int& max_groups = max_groups_dev[dev];
-  if (max_clusters < 0) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return ASG_ERR_CUDA;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cfg.gridDim = dim3(G * 1024, 1, 1);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = 1;
-    max_clusters = n;
-    max_groups = coop_max_groups(kern, NT, smem, G);
+  static int launch(const XYParams& pin, cudaStream_t st) {
+    XYParams p = pin;
+    if (p.G != G || p.nsub != 2) return ASG_ERR_SHAPE;
+    p.l2_buf_elems = nbuf;
+    GroupLimits l;
+    const int s = limits(&l);
+    if (s != ASG_OK) return s;
+    return launch_groups(xy_l2c<PY, FastPlan<Xn>, R, NT>, p, NT, smem,
+                         p.coop ? l.groups : l.clusters, p.nplanes, st);
   }
-  return launch_groups(kern, p, cfg, p.coop ? max_groups : max_clusters, p.nplanes, st);
-}
+};
 
 int asg_launch_xy_l2_closing(const XYParams& p, cudaStream_t st) {
   const int Xs = p.X / p.nsub;
   switch (p.Y) {
-    case 128: return Xs == 32 ? launch_l2c<128, 32>(p, st) : launch_l2c<128, 64>(p, st);
-    case 192: return launch_l2c<192, 96>(p, st);
-    case 256: return launch_l2c<256, 128>(p, st);
-    case 384: return launch_l2c<384, 192>(p, st);
-    case 512: return launch_l2c<512, 256>(p, st);
+    case 128: return Xs == 32 ? L2cLaunch<128, 32>::launch(p, st) : L2cLaunch<128, 64>::launch(p, st);
+    case 192: return L2cLaunch<192, 96>::launch(p, st);
+    case 256: return L2cLaunch<256, 128>::launch(p, st);
+    case 384: return L2cLaunch<384, 192>::launch(p, st);
+    case 512: return L2cLaunch<512, 256>::launch(p, st);
     default: return ASG_ERR_SHAPE;
+  }
+}
+
+// The most groups that a launch of either kernel on X x Y planes keeps resident: what the
+// exchange scratch has to hold.  0 if the queries fail.
+template <int Yn, int Xn>
+static int l2_max_groups() {
+  int m = 0;
+  auto take = [&](int s, const GroupLimits& l) {
+    if (s != ASG_OK) return false;
+    m = std::max(m, std::max(l.clusters, l.groups));
+    return true;
+  };
+  GroupLimits a, b, c;
+  if constexpr (Yn >= 256) {
+    if (!take(L2Launch<Yn, Xn, 8, 128>::limits(&c), c)) return 0;
+  }
+  return take(L2Launch<Yn, Xn, 16, 256>::limits(&a), a) && take(L2cLaunch<Yn, Xn>::limits(&b), b)
+             ? m : 0;
+}
+int asg_xy_l2_max_groups(int X, int Y) {
+  switch (Y) {
+    case 128: return X == 64 ? l2_max_groups<128, 32>() : l2_max_groups<128, 64>();
+    case 192: return l2_max_groups<192, 96>();
+    case 256: return l2_max_groups<256, 128>();
+    case 384: return l2_max_groups<384, 192>();
+    case 512: return l2_max_groups<512, 256>();
+    default: return 0;
   }
 }

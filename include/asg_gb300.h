@@ -198,8 +198,9 @@ typedef struct {
   int t_cols_flux;   /* columns per block of the column pass with the Burgers step: 8, 16, 32 (nT <= 256) */
   int t_cols_plain;  /* columns per block of the taper-only column pass: 8, 16 */
   int t_cols_stats;  /* columns per block of the column pass closing a step: 8, 16 */
-  int xy_clusters;   /* cap on resident CTA groups (clusters) of the L2-exchange plane kernel: 0..64 */
-  int xy_clusters_closing; /* the same for the closing-stage kernel (fused epilogue): 0..64 */
+  int xy_clusters;   /* cap on resident CTA groups (clusters) of the L2-exchange plane kernel:
+                      * 1..63, 64 all that fit the GPU; 0 = default (64) */
+  int xy_clusters_closing; /* the same for the closing-stage kernel (fused epilogue) */
   int xy_sync;       /* group barrier of those kernels: 1 thread-block cluster, 2 counter
                       * barrier in a cooperative launch, 3 the same with split-phase
                       * barriers over two scratch halves in the diffraction kernel (the
