@@ -180,12 +180,12 @@ __global__ void k_build_obl(TableParams p, float* out) {
 }
 
 int asg_launch_table(const TableParams& p, cudaStream_t st) {
-  k_build_table<<<4 * 152, 256, 0, st>>>(p);
+  k_build_table<<<4 * asg_sm_count(), 256, 0, st>>>(p);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
 }
 
 int asg_launch_obl_table(const TableParams& p, float* out, cudaStream_t st) {
-  k_build_obl<<<4 * 152, 256, 0, st>>>(p, out);
+  k_build_obl<<<4 * asg_sm_count(), 256, 0, st>>>(p, out);
   return cudaPeekAtLastError() == cudaSuccess ? ASG_OK : ASG_ERR_CUDA;
 }
 

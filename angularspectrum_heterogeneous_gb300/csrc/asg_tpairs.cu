@@ -254,14 +254,13 @@ __global__ void __launch_bounds__(256) k_flux_columns(TParams p) {
 template <class PL>
 int launch_pairs(const TParams& p, const LineAxis& ax, cudaStream_t st) {
   // pairs per block: what fills it, at least 4 (64-byte runs in HBM), while 72 KB
-  // hold them and the grid does not leave the GPU idle (two blocks for each of its
-  // 152 SMs)
+  // hold them and the grid does not leave the GPU idle (two blocks for each SM)
   const int npairs = (p.ncols + 1) / 2, tasks = line_tasks(ax);
   int lp = 0;
   while (lp < 5 && (lp < 2 || (tasks << lp) < LineBlock<PL::BIG>::NT)) {
     const int k = lp + 1;
     if (((size_t)line_stride(ax, 1 << k) * sizeof(float2) << k) > 72 * 1024) break;
-    if ((npairs >> k) < 2 * 152) break;
+    if ((npairs >> k) < 2 * asg_sm_count()) break;
     lp = k;
   }
   const int P = 1 << lp, LS = line_stride(ax, P);

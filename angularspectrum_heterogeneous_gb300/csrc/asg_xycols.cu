@@ -201,7 +201,7 @@ int launch_cols(const XYParams& p, const LineAxis& ax, float2* buf, cudaStream_t
   while (lc > 0 && ((size_t)line_stride(ax, 1 << lc) * sizeof(float2) << lc) > LINE_SMEM) --lc;
   while (lc >= 3 && lc < 5 && (tasks << lc) < 128 && (1 << lc) < p.Y &&
          ((size_t)line_stride(ax, 2 << lc) * sizeof(float2) << (lc + 1)) <= LINE_SMEM &&
-         p.nplanes * ((p.Y + (2 << lc) - 1) >> (lc + 1)) >= 8 * 152)
+         p.nplanes * ((p.Y + (2 << lc) - 1) >> (lc + 1)) >= 8 * asg_sm_count())
     ++lc;
   const int C = 1 << lc, LS = line_stride(ax, C);
   const size_t smem = (size_t)C * LS * sizeof(float2);

@@ -198,7 +198,7 @@ int launch_rows(const XYParams& p, const LineAxis& ax, float2* dst, bool inverse
   if (L * tasks > LineBlock<PL::BIG>::NT && L > 1) --L;
   while (L > 1 && (size_t)L * LS * sizeof(float2) > 48 * 1024) --L;
   const int total = p.nplanes * p.X;
-  while (L > 1 && total / L < 4 * 152) --L;
+  while (L > 1 && total / L < 4 * asg_sm_count()) --L;
   const size_t smem = (size_t)L * LS * sizeof(float2);
   static bool done[2][ASG_MAX_DEVICES] = {};
   const int dev = asg_device_slot();
