@@ -60,8 +60,10 @@ static int fail(int code, const char* fmt, ...) {
 template <typename T>
 static int dalloc(T** p, size_t n) {
   if (n == 0) n = 1;
-  if (cudaMalloc((void**)p, n * sizeof(T)) != cudaSuccess)
+  if (cudaMalloc((void**)p, n * sizeof(T)) != cudaSuccess) {
+    (void)cudaGetLastError();  // reported here, not left pending
     return fail(ASG_ERR_NOMEM, "cudaMalloc of %zu bytes failed", n * sizeof(T));
+  }
   return ASG_OK;
 }
 template <typename T>
@@ -612,10 +614,12 @@ extern "C" int asg_plan_destroy(asg_plan* p) {
   cudaFree(const_cast<float4*>(p->pl_x.tw));
   cudaFree(const_cast<float4*>(p->pl_y.tw));
   free_outputs(p);
-  cudaEventDestroy(p->ev0);
-  cudaEventDestroy(p->ev1);
+  // (a plan whose creation failed early has none: destroying a null handle would leave an error
+  // pending, which the next launch would report as its own)
+  if (p->ev0) cudaEventDestroy(p->ev0);
+  if (p->ev1) cudaEventDestroy(p->ev1);
   for (auto e : p->ev_pool) cudaEventDestroy(e);
-  cudaStreamDestroy(p->st);
+  if (p->st) cudaStreamDestroy(p->st);
   delete p;
   return ASG_OK;
 }
