@@ -22,7 +22,8 @@ def test_square_planes(n):
 
 @pytest.mark.parametrize("shape", [(4, 1024, 9), (1024, 4, 8), (2, 729, 8), (625, 3, 9), (8, 400, 8),
                                    (512, 8, 9), (1536, 3, 8), (7, 680, 8), (17, 19, 9), (19, 8, 8),
-                                   (5, 48, 7), (75, 16, 8), (12, 121, 9), (20, 100, 8)])
+                                   (5, 48, 7), (75, 16, 8), (12, 121, 9), (20, 100, 8),
+                                   (3, 1000, 9), (1000, 3, 8)])
 def test_narrow_planes(shape):
     P.test_step_operators(None, shape)
 
