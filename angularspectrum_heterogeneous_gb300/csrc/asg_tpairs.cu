@@ -6,8 +6,9 @@
 // (asg_lines.cuh: direct where the length splits into two radices, a chirp
 // convolution for every other length).  Planes are in natural bin order.
 //
-// A block of 4 warps holds P pairs (a power of two up to 8).  Bounded by the
-// register DFTs and their exchanges through shared memory.  Per pass, against
+// A block of 4 warps holds P pairs (a power of two up to 32).  Bounded by instruction
+// issue and its latencies (five blocks per SM by registers, 40 to 55 % of the issue slots):
+// register DFTs, their exchanges through shared memory, instruction fetch.  Per pass, against
 // mixed-radix Stockham lines with direct sums over the prime factors:
 // 257 x 257 x 601 27-30 -> 0.9 ms (its HBM traffic alone: 0.05 ms),
 // 51 x 51 x 401 620-640 -> 40-47 us, 200 x 180 x 400 780-930 -> 90-160 us,

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(NT, (NT == 256 ? 2 : 1)) xy_fast(XYParams p) {
 
 // ---------------------------------------------------------------------------
 // one CTA per plane, whole plane in shared memory (ping-pong): planes with more
-// than 1024 rows, which the line passes (asg_xyrows.cu) do not take
+// than 1024 rows that neither the line passes (asg_xyrows.cu) nor asg_xyplane.cu take
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) xy_generic(XYParams p, GenPlan plx, GenPlan ply) {
   const int X = p.X, Y = p.Y;

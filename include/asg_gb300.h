@@ -195,9 +195,10 @@ int asg_batch_last_run_ms(asg_batch* batch, double* ms);
 /* Launch shapes of a plan (no counterpart in the reference: its XLA program
  * has no tunable launch shapes). 0 in a field selects the built-in default. */
 typedef struct {
-  int t_cols_flux;   /* columns per block of the column pass with the Burgers step: 8, 16, 32 (nT <= 256) */
-  int t_cols_plain;  /* columns per block of the taper-only column pass: 8, 16 */
-  int t_cols_stats;  /* columns per block of the column pass closing a step: 8, 16 */
+  int t_cols_flux;   /* columns per block of the column pass with the Burgers step: 8, 16
+                      * (nT <= 1024), 32 (nT <= 256) */
+  int t_cols_plain;  /* the same of the taper-only column pass */
+  int t_cols_stats;  /* the same of the column pass closing a step */
   int xy_clusters;   /* cap on resident CTA groups (clusters) of the L2-exchange plane kernel:
                       * 1..63, 64 all that fit the GPU; 0 = default (64) */
   int xy_clusters_closing; /* the same for the closing-stage kernel (fused epilogue) */
