@@ -306,9 +306,10 @@ static int line_axis(int n, LineAxis* a, cudaStream_t st) {
   return ASG_OK;
 }
 
-// Passes of an axis of a small plane: the factors of its line transform, those above 9 split
-// again, primes up to 19 as they are; empty if there are none.
-static std::vector<int> plane_radices(int n) {
+// Passes of an axis of a small plane of `lines` lines of n samples: the factors of its line
+// transform, those above 9 split again; primes up to 17 as they are, and up to 61 where a
+// block has a thread for each pair of their bins.  Empty if there are none.
+static std::vector<int> plane_radices(int n, int lines) {
   std::vector<int> r;
   LineAxis a = {};
   if (n < 1 || !line_factors(n, &a)) return r;
@@ -318,7 +319,8 @@ static std::vector<int> plane_radices(int n) {
     const int f = todo.back(), p = radix_split(f);
     todo.pop_back();
     if (f == 1) continue;
-    if (f <= 9 || (p == f && f <= 19)) {
+    if (f <= 9 || (p == f && (f <= 17 || (f <= 61 && asg_plane_spread(f, n, lines) <=
+                                                         ASG_PLANE_THREADS)))) {
       r.push_back(f);
     } else if (p == f) {
       return {};
@@ -329,18 +331,18 @@ static std::vector<int> plane_radices(int n) {
   }
   return r.size() <= 8 ? r : std::vector<int>();
 }
-// Whether a plane runs in one block: its axes have passes (19 samples only beside an axis of
-// other factors: 17 x 19 82 us per step, 88 in three launches; 19 x 19 and 23 x 16 gain
-// nothing) and
+// Whether a plane runs in one block: its axes have passes and
 //   * up to 8 samples along an axis, whatever fits: short rows, or columns that fill a part
 //     of the column pass's lanes (1024 x 2 55 -> 21 us per stage, 4 x 512 30 -> 18);
 //   * otherwise up to 10500 samples times passes, where the passes over all samples begin to
 //     cost as much as the two further launches (us per step of 128 samples in three
 //     launches and in one block: 16 x 16 70 and 43, 48 x 48 66 and 63, 60 x 60 78 and 90,
 //     24 x 100 66 and 76).
+// Larger primes are slower so than as convolutions in three launches unless spread over the
+// block (16 x 23 80 and 61, 37 x 3 72 and 60; rolled, 38 x 38 93 and 98, 23 x 23 74 and 100).
 static bool small_plane(int X, int Y) {
-  const int px = (int)plane_radices(X).size(), py = (int)plane_radices(Y).size();
-  if (px == 0 || py == 0 || (LINE_DIRECT.n1[X] == 0 && LINE_DIRECT.n1[Y] == 0)) return false;
+  const int px = (int)plane_radices(X, Y).size(), py = (int)plane_radices(Y, X).size();
+  if (px == 0 || py == 0) return false;
   if ((size_t)X * (Y | 1) * sizeof(float2) > ASG_PLANE_MAX_SMEM) return false;
   return std::min(X, Y) <= 8 || X * Y * (px + py) <= 10500;
 }
@@ -355,11 +357,11 @@ static int plane_bin(const std::vector<int>& r, int n, int s) {
   }
   return bin;
 }
-static int plane_axis(int n, PlaneAxis* a, cudaStream_t st) {
+static int plane_axis(int n, int lines, PlaneAxis* a, cudaStream_t st) {
   a->n = n;
   a->radices = 0;
   int i = 0;
-  for (int f : plane_radices(n)) a->radices |= (unsigned long long)f << (8 * i++);
+  for (int f : plane_radices(n, lines)) a->radices |= (unsigned long long)f << (8 * i++);
   std::vector<float4> tw(n);
   for (int j = 0; j < n; ++j) {
     const double ang = -2.0 * M_PI * (double)j / (double)n;
@@ -696,8 +698,8 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     CKS(line_axis(Y, &p->ax_y, p->st));
   }
   if (p->small) {
-    CKS(plane_axis(X, &p->pl_x, p->st));
-    CKS(plane_axis(Y, &p->pl_y, p->st));
+    CKS(plane_axis(X, Y, &p->pl_x, p->st));
+    CKS(plane_axis(Y, X, &p->pl_y, p->st));
   }
 
   // ---- planes ----
@@ -714,7 +716,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   // natural bin held by each x slot (row order of the plane kernels) and by
   // each y slot (the fast kernels keep y in four-step slot order)
   std::vector<int> binx(X), biny(Y);
-  const std::vector<int> rx = plane_radices(X);
+  const std::vector<int> rx = plane_radices(X, Y);
   for (int s = 0; s < X; ++s) {
     if (p->split) {
       const int Xs = X / 2, R = 16, h = s / Xs, sg = s % Xs;
@@ -774,7 +776,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   if (p->small) {
     // classes numbered in natural order (the tables' roundings are spread along it), slots
     // in that of the passes
-    const std::vector<int> nat = p->h_cls_y, ry = plane_radices(Y);
+    const std::vector<int> nat = p->h_cls_y, ry = plane_radices(Y, X);
     for (int s = 0; s < Y; ++s) p->h_cls_y[s] = nat[plane_bin(ry, Y, s)];
   }
 

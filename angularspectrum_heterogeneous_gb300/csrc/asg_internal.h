@@ -176,6 +176,11 @@ struct PlaneAxis {
   const float4* tw;
 };
 constexpr size_t ASG_PLANE_MAX_SMEM = 47 * 1024;
+constexpr int ASG_PLANE_THREADS = 256;
+// threads that a pass of the odd prime r takes on `lines` lines of n samples, one per pair of bins
+__host__ __device__ inline int asg_plane_spread(int r, int n, int lines) {
+  return lines * (n / r) * ((r + 1) / 2);
+}
 int asg_launch_xy_plane(const XYParams& p, const PlaneAxis& axx, const PlaneAxis& axy,
                         cudaStream_t st);
 int asg_launch_xy(const XYParams& p, bool fast, const GenPlan& plx, const GenPlan& ply,

@@ -7,8 +7,8 @@
 // Row, column and row pass of such a plane cost three launches, 21 to 25 us per stage
 // however small it is; one block per plane takes 10 to 14 up to 32 x 32, 18 for 48 x 48,
 // with 65 planes as with 513.  Hence small radices (a DFT of 12 or 16 points per thread
-// took 14 to 16 us), one copy of a pass's code for both axes and rolled sums over odd primes
-// (17 x 17 22 -> 18 us).
+// took 14 to 16 us), one copy of a pass's code for both axes and sums over odd primes spread
+// over the block's threads where these are enough (17 x 17 22 -> 15 us), else rolled.
 //
 // A line is transformed in its own slots: a pass of radix r on sublines of m samples takes
 // the samples b + (m / r) a to their DFT's bins ka at b + (m / r) ka, times W_m^(b ka), and
@@ -26,7 +26,7 @@ ASG_DEFINE_LINE_ROOT_UPLOADER(asg_roots_upload_xyplane)
 
 namespace {
 
-constexpr int PLANE_NT = 256;
+constexpr int PLANE_NT = ASG_PLANE_THREADS;
 
 // The lines of an axis: line l at base + l ls, its sample j es further per step.
 struct Lines {
@@ -115,6 +115,57 @@ ASG_DEV void pass_prime(const Lines& L, const PlaneAxis& ax, int m) {
   __syncthreads();
 }
 
+// The same, a thread per DFT and pair of bins k, R - k (k = 0: the plain sum), for a block with a
+// thread for each: all inputs are read before any bin is written.  A rolled sum leaves most of
+// a small plane's threads idle (17 x 17 18 -> 15 us per stage, 11 x 11 17 -> 13).
+template <bool INV>
+ASG_DEV void pass_spread(const Lines& L, const PlaneAxis& ax, int R, int m) {
+  const int H = (R - 1) / 2, mp = m / R, ts = ax.n / m, st = mp * L.es;
+  const int rs = ax.n / R;  // exp(-2 pi i e / R) at tw[e rs]
+  const int dfts = L.count * rs, k = threadIdx.x / dfts, it = threadIdx.x - k * dfts;
+  const bool on = k <= H, turn = mp > 1;
+  const int j = it / L.count, l = it - j * L.count, sub = j / mp, b = j - sub * mp;
+  float2* s = L.base + l * L.ls + (sub * m + b) * L.es;
+  float2 x, y;
+  if (on) {
+    const float2 v0 = s[0];
+    float2 r = make_float2(0.f, 0.f), q = r;
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {  // the roots' low parts first (see ldft)
+      if (part == 1 && k == 0) r = v0;
+      int e = 0;
+#pragma unroll 4
+      for (int a = 1; a <= H; ++a) {
+        float2 u = s[a * st], w = s[(R - a) * st];
+        if (INV && turn) {
+          u = mulc_f4(u, __ldg(ax.tw + ts * b * a));
+          w = mulc_f4(w, __ldg(ax.tw + ts * b * (R - a)));
+        }
+        e = e + k < R ? e + k : e + k - R;
+        const float4 f = __ldg(ax.tw + e * rs);
+        const float c = part ? f.x : f.z, sn = part ? f.y : f.w;
+        const float2 t = cadd(u, w), d = csub(u, w);
+        r = make_float2(fmaf(t.x, c, r.x), fmaf(t.y, c, r.y));
+        q = make_float2(fmaf(d.x, sn, q.x), fmaf(d.y, sn, q.y));
+      }
+    }
+    if (k > 0) r = cadd(r, v0);
+    const float2 iq = make_float2(-q.y, q.x);
+    x = INV ? csub(r, iq) : cadd(r, iq);
+    y = INV ? cadd(r, iq) : csub(r, iq);
+    if (!INV && turn && k > 0) {
+      x = mul_f4(x, __ldg(ax.tw + ts * b * k));
+      y = mul_f4(y, __ldg(ax.tw + ts * b * (R - k)));
+    }
+  }
+  __syncthreads();
+  if (on) {
+    s[k * st] = x;
+    if (k > 0) s[(R - k) * st] = y;
+  }
+  __syncthreads();
+}
+
 // All passes of an axis (not inlined: the second axis finds the code fetched).
 template <bool INV>
 __device__ __noinline__ void plane_passes(Lines L, PlaneAxis ax) {
@@ -125,7 +176,10 @@ __device__ __noinline__ void plane_passes(Lines L, PlaneAxis ax) {
   for (int i = 0; i < np; ++i) {
     const int r = (int)(ax.radices >> (8 * (INV ? np - 1 - i : i))) & 255;
     if (INV) m *= r;
-    switch (r) {
+    const int spread = r > 9 ? asg_plane_spread(r, ax.n, L.count) : 0;
+    if (spread > 0 && spread <= (int)blockDim.x) {
+      pass_spread<INV>(L, ax, r, m);
+    } else switch (r) {
       case 2: pass_small<2, INV>(L, ax, m); break;
       case 3: pass_small<3, INV>(L, ax, m); break;
       case 4: pass_small<4, INV>(L, ax, m); break;
@@ -137,7 +191,6 @@ __device__ __noinline__ void plane_passes(Lines L, PlaneAxis ax) {
       case 11: pass_prime<11, INV>(L, ax, m); break;
       case 13: pass_prime<13, INV>(L, ax, m); break;
       case 17: pass_prime<17, INV>(L, ax, m); break;
-      case 19: pass_prime<19, INV>(L, ax, m); break;
       default: break;
     }
     if (!INV) m /= r;
@@ -235,5 +288,14 @@ int asg_launch_xy_plane(const XYParams& p, const PlaneAxis& axx, const PlaneAxis
   // planes be resident
   int nt = std::min(PLANE_NT, std::max(32, (p.X * p.Y / 4 + 31) / 32 * 32));
   if (nt == PLANE_NT && p.nplanes > 3 * asg_sm_count()) nt /= 2;
+  // and the threads that passes of odd primes spread over, where a block has as many
+  auto spread = [&](const PlaneAxis& ax, int lines) {
+    for (unsigned long long r = ax.radices; r != 0; r >>= 8) {
+      const int t = (r & 255) > 9 ? asg_plane_spread((int)(r & 255), ax.n, lines) : 0;
+      if (t <= PLANE_NT) nt = std::max(nt, (t + 31) / 32 * 32);
+    }
+  };
+  spread(axx, p.Y);
+  spread(axy, p.X);
   return asg_launch_pdl(p.pdl != 0, xy_plane, dim3(p.nplanes), dim3(nt), smem, st, p, axx, axy, RS);
 }

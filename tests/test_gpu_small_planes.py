@@ -23,7 +23,12 @@ def test_square_planes(n):
 @pytest.mark.parametrize("shape", [(4, 1024, 9), (1024, 4, 8), (2, 729, 8), (625, 3, 9), (8, 400, 8),
                                    (512, 8, 9), (1536, 3, 8), (7, 680, 8), (17, 19, 9), (19, 8, 8),
                                    (5, 48, 7), (75, 16, 8), (12, 121, 9), (20, 100, 8),
-                                   (3, 1000, 9), (1000, 3, 8)])
+                                   (3, 1000, 9), (1000, 3, 8),
+                                   # sums of odd primes spread over the block: partly and
+                                   # wholly filled, beside another pass, one line too many
+                                   (37, 3, 8), (3, 41, 9), (61, 8, 8), (8, 53, 9), (16, 23, 8),
+                                   (31, 16, 9), (17, 31, 8), (46, 5, 9), (4, 58, 8), (19, 19, 9),
+                                   (23, 11, 8), (38, 6, 9), (2, 43, 8)])
 def test_narrow_planes(shape):
     P.test_step_operators(None, shape)
 
