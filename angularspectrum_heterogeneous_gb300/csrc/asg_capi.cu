@@ -306,22 +306,40 @@ static int line_axis(int n, LineAxis* a, cudaStream_t st) {
   return ASG_OK;
 }
 
+// n as the fewest factors up to 9, the most even of these (largest first), into *best.
+static void few_radices(int n, int top, std::vector<int>& cur, std::vector<int>* best) {
+  if (n == 1) {
+    if (best->empty() || cur.size() < best->size() ||
+        (cur.size() == best->size() && cur[0] < (*best)[0]))
+      *best = cur;
+    return;
+  }
+  for (int f = std::min(n, top); f >= 2; --f) {
+    if (n % f != 0) continue;
+    cur.push_back(f);
+    few_radices(n / f, f, cur, best);
+    cur.pop_back();
+  }
+}
 // Passes of an axis of a small plane of `lines` lines of n samples: the factors of its line
-// transform, those above 9 split again; primes up to 17 as they are, and up to 61 where a
-// block has a thread for each pair of their bins.  Empty if there are none.
-static std::vector<int> plane_radices(int n, int lines) {
+// transform, those above 9 split again and, where that leaves more than two, grouped anew;
+// primes up to 17 as they are, and up to 61 where a block of `threads` has one for each pair
+// of their bins.  Empty if there are none.
+static std::vector<int> plane_radices(int n, int lines, int threads) {
   std::vector<int> r;
   LineAxis a = {};
   if (n < 1 || !line_factors(n, &a)) return r;
   std::vector<int> todo = {n};
   if (a.direct) todo = {a.n2, a.n1};
+  int smooth = 1;
   while (!todo.empty()) {
     const int f = todo.back(), p = radix_split(f);
     todo.pop_back();
     if (f == 1) continue;
-    if (f <= 9 || (p == f && (f <= 17 || (f <= 61 && asg_plane_spread(f, n, lines) <=
-                                                         ASG_PLANE_THREADS)))) {
+    if (f <= 9 ||
+        (p == f && (f <= 17 || (f <= 61 && asg_plane_spread(f, n, lines) <= threads)))) {
       r.push_back(f);
+      if (f <= 9) smooth *= f;
     } else if (p == f) {
       return {};
     } else {
@@ -329,22 +347,43 @@ static std::vector<int> plane_radices(int n, int lines) {
       todo.push_back(p);
     }
   }
+  if (r.size() > 2) {
+    std::vector<int> cur, best;
+    few_radices(smooth, 9, cur, &best);
+    for (int f : r)
+      if (f > 9) best.push_back(f);
+    if (best.size() < r.size()) r = best;
+  }
   return r.size() <= 8 ? r : std::vector<int>();
 }
 // Whether a plane runs in one block: its axes have passes and
 //   * up to 8 samples along an axis, whatever fits: short rows, or columns that fill a part
 //     of the column pass's lanes (1024 x 2 55 -> 21 us per stage, 4 x 512 30 -> 18);
-//   * otherwise up to 10500 samples times passes, where the passes over all samples begin to
+//   * otherwise up to 9800 samples times passes, where the passes over all samples begin to
 //     cost as much as the two further launches (us per step of 128 samples in three
-//     launches and in one block: 16 x 16 70 and 43, 48 x 48 66 and 63, 60 x 60 78 and 90,
-//     24 x 100 66 and 76).
-// Larger primes are slower so than as convolutions in three launches unless spread over the
-// block (16 x 23 80 and 61, 37 x 3 72 and 60; rolled, 38 x 38 93 and 98, 23 x 23 74 and 100).
-static bool small_plane(int X, int Y) {
-  const int px = (int)plane_radices(X, Y).size(), py = (int)plane_radices(Y, X).size();
-  if (px == 0 || py == 0) return false;
+//     launches and in one block: 16 x 16 70 and 43, 48 x 48 66 and 63, 20 x 100 66 and 68,
+//     60 x 60 78 and 90, 24 x 100 66 and 76); 10500 if a line pass has a radix above 16, so
+//     fewer warps (51 x 51 120 and 110).
+// Direct sums over larger primes cost arithmetic, which the convolutions of the line passes save
+// once the GPU is full: up to 17, 550 k samples in all planes (44 x 44 x 512 92 and 94 us per step
+// in one and in three launches, x 768 113 and 103; 34 x 34 x 768 one block, x 1024 166 and 162);
+// above 17, 5 M samples times primes (37 x 4 x 2048 gains, 47 x 7 x 1024 128 and 121).
+static bool small_plane(int X, int Y, int nplanes) {
+  const int nt = asg_plane_threads(nplanes);
+  const std::vector<int> rx = plane_radices(X, Y, nt), ry = plane_radices(Y, X, nt);
+  if (rx.empty() || ry.empty()) return false;
   if ((size_t)X * (Y | 1) * sizeof(float2) > ASG_PLANE_MAX_SMEM) return false;
-  return std::min(X, Y) <= 8 || X * Y * (px + py) <= 10500;
+  const size_t total = (size_t)X * Y * nplanes;
+  size_t sums = 0;  // primes above 17
+  bool prime = false;
+  for (const auto* r : {&rx, &ry})
+    for (int f : *r) {
+      prime = prime || f > 9;
+      sums += f > 17 ? f : 0;
+    }
+  if ((prime && total > 550000) || total * sums > 5000000) return false;
+  const int limit = LINE_DIRECT.rm[X] > 16 || LINE_DIRECT.rm[Y] > 16 ? 10500 : 9800;
+  return std::min(X, Y) <= 8 || X * Y * (int)(rx.size() + ry.size()) <= limit;
 }
 // bin in slot s of a transformed line
 static int plane_bin(const std::vector<int>& r, int n, int s) {
@@ -357,11 +396,11 @@ static int plane_bin(const std::vector<int>& r, int n, int s) {
   }
   return bin;
 }
-static int plane_axis(int n, int lines, PlaneAxis* a, cudaStream_t st) {
+static int plane_axis(int n, const std::vector<int>& radices, PlaneAxis* a, cudaStream_t st) {
   a->n = n;
   a->radices = 0;
   int i = 0;
-  for (int f : plane_radices(n, lines)) a->radices |= (unsigned long long)f << (8 * i++);
+  for (int f : radices) a->radices |= (unsigned long long)f << (8 * i++);
   std::vector<float4> tw(n);
   for (int j = 0; j < n; ++j) {
     const double ang = -2.0 * M_PI * (double)j / (double)n;
@@ -677,7 +716,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     p->G = 1;
     // the row and column passes take lines up to 1024; a plane with more rows
     // runs in one CTA's shared memory if it fits
-    p->small = small_plane(X, Y);
+    p->small = small_plane(X, Y, p->F);
     p->lines = !p->small && X <= ASG_LINES_MAX;
     if (!p->small && !p->lines && asg_xy_generic_smem(X, Y) > ASG_XY_GENERIC_MAX_SMEM)
       return fail(ASG_ERR_SHAPE, "grid %dx%d: nX > 1024 without a fast plane transform", X, Y);
@@ -697,9 +736,11 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
     CKS(line_axis(X, &p->ax_x, p->st));
     CKS(line_axis(Y, &p->ax_y, p->st));
   }
+  const int plane_nt = asg_plane_threads(p->F);
+  const std::vector<int> rx = plane_radices(X, Y, plane_nt), ry = plane_radices(Y, X, plane_nt);
   if (p->small) {
-    CKS(plane_axis(X, Y, &p->pl_x, p->st));
-    CKS(plane_axis(Y, X, &p->pl_y, p->st));
+    CKS(plane_axis(X, rx, &p->pl_x, p->st));
+    CKS(plane_axis(Y, ry, &p->pl_y, p->st));
   }
 
   // ---- planes ----
@@ -716,7 +757,6 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   // natural bin held by each x slot (row order of the plane kernels) and by
   // each y slot (the fast kernels keep y in four-step slot order)
   std::vector<int> binx(X), biny(Y);
-  const std::vector<int> rx = plane_radices(X, Y);
   for (int s = 0; s < X; ++s) {
     if (p->split) {
       const int Xs = X / 2, R = 16, h = s / Xs, sg = s % Xs;
@@ -776,7 +816,7 @@ static int plan_create_impl(const asg_config* cfg, asg_plan* p) {
   if (p->small) {
     // classes numbered in natural order (the tables' roundings are spread along it), slots
     // in that of the passes
-    const std::vector<int> nat = p->h_cls_y, ry = plane_radices(Y, X);
+    const std::vector<int> nat = p->h_cls_y;
     for (int s = 0; s < Y; ++s) p->h_cls_y[s] = nat[plane_bin(ry, Y, s)];
   }
 

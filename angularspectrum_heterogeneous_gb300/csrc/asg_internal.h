@@ -176,7 +176,6 @@ struct PlaneAxis {
   const float4* tw;
 };
 constexpr size_t ASG_PLANE_MAX_SMEM = 47 * 1024;
-constexpr int ASG_PLANE_THREADS = 256;
 // threads that a pass of the odd prime r takes on `lines` lines of n samples, one per pair of bins
 __host__ __device__ inline int asg_plane_spread(int r, int n, int lines) {
   return lines * (n / r) * ((r + 1) / 2);
@@ -244,6 +243,14 @@ inline int asg_sm_count() {
                  cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, d) != cudaSuccess))
     return 152;
   return c;
+}
+
+// threads of a small plane's block at most: 256, less where that lets all planes be resident
+// (80 registers per thread)
+inline int asg_plane_threads(int nplanes) {
+  const int per_sm = (nplanes + asg_sm_count() - 1) / asg_sm_count();
+  const int t = 768 / per_sm / 32 * 32;
+  return t > 256 ? 256 : t < 64 ? 64 : t;
 }
 
 // error reporting shared by the translation units (message for asg_last_error)

@@ -26,7 +26,7 @@ ASG_DEFINE_LINE_ROOT_UPLOADER(asg_roots_upload_xyplane)
 
 namespace {
 
-constexpr int PLANE_NT = ASG_PLANE_THREADS;
+constexpr int PLANE_NT = 256;
 
 // The lines of an axis: line l at base + l ls, its sample j es further per step.
 struct Lines {
@@ -284,18 +284,16 @@ int asg_launch_xy_plane(const XYParams& p, const PlaneAxis& axx, const PlaneAxis
   const int RS = p.Y | 1;
   const size_t smem = (size_t)p.X * RS * sizeof(float2);
   if (axx.n != p.X || axy.n != p.Y || smem > ASG_PLANE_MAX_SMEM) return ASG_ERR_SHAPE;
-  // about four samples per thread, a DFT of radix 4; half the threads where that lets all
-  // planes be resident
-  int nt = std::min(PLANE_NT, std::max(32, (p.X * p.Y / 4 + 31) / 32 * 32));
-  if (nt == PLANE_NT && p.nplanes > 3 * asg_sm_count()) nt /= 2;
-  // and the threads that passes of odd primes spread over, where a block has as many
+  // about four samples per thread, a DFT of radix 4; passes of odd primes spread over more;
+  // no more threads than let all planes be resident
+  int nt = std::max(32, (p.X * p.Y / 4 + 31) / 32 * 32);
   auto spread = [&](const PlaneAxis& ax, int lines) {
-    for (unsigned long long r = ax.radices; r != 0; r >>= 8) {
-      const int t = (r & 255) > 9 ? asg_plane_spread((int)(r & 255), ax.n, lines) : 0;
-      if (t <= PLANE_NT) nt = std::max(nt, (t + 31) / 32 * 32);
-    }
+    for (unsigned long long r = ax.radices; r != 0; r >>= 8)
+      if ((r & 255) > 9)
+        nt = std::max(nt, (asg_plane_spread((int)(r & 255), ax.n, lines) + 31) / 32 * 32);
   };
   spread(axx, p.Y);
   spread(axy, p.X);
+  nt = std::min(nt, asg_plane_threads(p.nplanes));
   return asg_launch_pdl(p.pdl != 0, xy_plane, dim3(p.nplanes), dim3(nt), smem, st, p, axx, axy, RS);
 }
