@@ -323,7 +323,7 @@ static void few_radices(int n, int top, std::vector<int>& cur, std::vector<int>*
 }
 // Passes of an axis of a small plane of `lines` lines of n samples: the factors of its line
 // transform, those above 9 split again and, where that leaves more than two, grouped anew;
-// primes up to 17 as they are, and up to 61 where a block of `threads` has one for each pair
+// primes up to 17 as they are, and up to 79 where a block of `threads` has one for each pair
 // of their bins.  Empty if there are none.
 static std::vector<int> plane_radices(int n, int lines, int threads) {
   std::vector<int> r;
@@ -337,7 +337,7 @@ static std::vector<int> plane_radices(int n, int lines, int threads) {
     todo.pop_back();
     if (f == 1) continue;
     if (f <= 9 ||
-        (p == f && (f <= 17 || (f <= 61 && asg_plane_spread(f, n, lines) <= threads)))) {
+        (p == f && (f <= 17 || (f <= 79 && asg_plane_spread(f, n, lines) <= threads)))) {
       r.push_back(f);
       if (f <= 9) smooth *= f;
     } else if (p == f) {

@@ -28,7 +28,9 @@ def test_square_planes(n):
                                    # wholly filled, beside another pass, one line too many
                                    (37, 3, 8), (3, 41, 9), (61, 8, 8), (8, 53, 9), (16, 23, 8),
                                    (31, 16, 9), (17, 31, 8), (46, 5, 9), (4, 58, 8), (19, 19, 9),
-                                   (23, 11, 8), (38, 6, 9), (2, 43, 8)])
+                                   (23, 11, 8), (38, 6, 9), (2, 43, 8), (67, 3, 8), (4, 79, 9),
+                                   # line passes with fewer than eight columns
+                                   (381, 2, 8), (331, 3, 9), (997, 4, 8), (83, 5, 9)])
 def test_narrow_planes(shape):
     P.test_step_operators(None, shape)
 
