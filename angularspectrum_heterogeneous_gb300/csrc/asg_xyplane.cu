@@ -6,9 +6,10 @@
 // above all instruction fetch, since each pass over a plane is short and its code cold.
 // Row, column and row pass of such a plane cost three launches, 21 to 25 us per stage
 // however small it is; for 65 planes one block each takes 10 to 14 up to 32 x 32, 18 for
-// 48 x 48 (16 x 16: 12 with 65 planes, 14 with 1025).  Hence small radices (a DFT of 12 or 16 points per thread
-// took 14 to 16 us), one copy of a pass's code for both axes and sums over odd primes spread
-// over the block's threads where these are enough (17 x 17 22 -> 15 us), else rolled.
+// 48 x 48 (16 x 16: 12 with 65 planes, 14 with 1025).  Hence small radices (a DFT of 12 or
+// 16 points per thread took 14 to 16 us), one copy of a pass's code for both axes and sums
+// over odd primes spread over the block's threads where these are enough (17 x 17 22 -> 15
+// us), else rolled.
 //
 // A line is transformed in its own slots: a pass of radix r on sublines of m samples takes
 // the samples b + (m / r) a to their DFT's bins ka at b + (m / r) ka, times W_m^(b ka), and
